@@ -155,6 +155,24 @@ int check_out(const void* p, int ld, int H, int out_dtype) {
     return KB_OK;
 }
 
+// Launch with programmatic stream serialization (see pdl_wait): the launch latency and the set-up of a kernel run under the tail of
+// the one before it. `extra` = a further launch attribute (cluster size, cooperative) or null.
+template <typename... P, typename... A>
+int launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const cudaLaunchAttribute* extra, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 1;
+    if (extra) attr[cfg.numAttrs++] = *extra;
+    cfg.attrs = attr;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? KB_OK : KB_ERR_CUDA;
+}
+
 // Collects the tensors one launch of the pre-pass stages.
 struct PrepBatch {
     PrepParams pp = {};
@@ -173,48 +191,31 @@ struct PrepBatch {
 int launch_prep(DeviceState* st, const PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {
     if (pb.pp.blocks == 0) {
         // nothing to stage: the words still have to be cleared before the attention kernel starts
-        if (pb.pp.zero_n > 0 && cudaMemsetAsync(pb.pp.zero_ptr, 0, (size_t)pb.pp.zero_n * sizeof(unsigned int), stream) != cudaSuccess) return KB_ERR_CUDA;
+        if (pb.pp.zero_n > 0) return launch_dependent(zero_words_kernel, dim3(1), dim3(256), 0, stream, nullptr, pb.pp.zero_ptr, pb.pp.zero_n);
         return KB_OK;
     }
     ProfScope ps(st, KB_PROF_NORM_ROPE, stream);
     const unsigned grid = pb.pp.blocks;
-#define KB_PREP(IN, OUT) qk_prep_kernel<IN, OUT><<<grid, 256, 0, stream>>>(pb.pp)
-    if (out_dtype == KB_F32) {
-        KB_PREP(float, float);        // in-place fp32 norm / RoPE as the engine's own ops do (validated by the caller)
-    } else if (out_dtype == KB_F16) {
-        if (in_dtype == KB_F16) KB_PREP(__half, __half);
-        else if (in_dtype == KB_BF16) KB_PREP(__nv_bfloat16, __half);
-        else KB_PREP(float, __half);
-    } else {
-        if (in_dtype == KB_F16) KB_PREP(__half, __nv_bfloat16);
-        else if (in_dtype == KB_BF16) KB_PREP(__nv_bfloat16, __nv_bfloat16);
-        else KB_PREP(float, __nv_bfloat16);
-    }
+#define KB_PREP(IN, OUT) launch_dependent(qk_prep_kernel<IN, OUT>, dim3(grid), dim3(256), 0, stream, nullptr, pb.pp)
+    if (out_dtype == KB_F32) return KB_PREP(float, float);   // in-place fp32 norm / RoPE as the engine's own ops do (validated by the caller)
+    if (out_dtype == KB_F16)
+        return in_dtype == KB_F16 ? KB_PREP(__half, __half) : in_dtype == KB_BF16 ? KB_PREP(__nv_bfloat16, __half) : KB_PREP(float, __half);
+    return in_dtype == KB_F16 ? KB_PREP(__half, __nv_bfloat16) : in_dtype == KB_BF16 ? KB_PREP(__nv_bfloat16, __nv_bfloat16) : KB_PREP(float, __nv_bfloat16);
 #undef KB_PREP
-    return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_CUDA;
 }
 
 template <int MODE, typename OutT>
 int launch_attn_t(const CUtensorMap& tq, const CUtensorMap& tk0, const CUtensorMap& tv0, const CUtensorMap& tk1,
                   const CUtensorMap& tv1, const CUtensorMap& to, const AttnParams& p, int sm_count, cudaStream_t stream) {
     // persistent kernel: one CTA per SM (its shared memory and TMEM fill an SM) walks the work items
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(ATTN_THREADS, 1, 1);
-    cfg.gridDim = dim3((unsigned)((p.split || p.n_items >= sm_count) ? sm_count : p.n_items), 1, 1);
-    cfg.dynamicSmemBytes = MODE == MODE_NAG ? ATTN_SMEM_NAG : ATTN_SMEM_PAIR;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    cfg.numAttrs = 0;
-    if (MODE == MODE_NAG || p.split) {
-        // the CTAs holding the heads of one query tile (NAG) or the parts of a cut item (split) wait for each other:
-        // all CTAs must be resident at once
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attn_fwd_kernel<MODE, OutT>, tq, tk0, tv0, tk1, tv1, to, p);
-    return e == cudaSuccess ? KB_OK : KB_ERR_CUDA;
+    const unsigned grid = (unsigned)((p.split || p.n_items >= sm_count) ? sm_count : p.n_items);
+    // the CTAs holding the heads of one query tile (NAG) or the parts of a cut item (split) wait for each other:
+    // all CTAs must be resident at once
+    cudaLaunchAttribute coop;
+    coop.id = cudaLaunchAttributeCooperative;
+    coop.val.cooperative = 1;
+    return launch_dependent(attn_fwd_kernel<MODE, OutT>, dim3(grid), dim3(ATTN_THREADS), MODE == MODE_NAG ? ATTN_SMEM_NAG : ATTN_SMEM_PAIR, stream,
+                            (MODE == MODE_NAG || p.split) ? &coop : nullptr, tq, tk0, tv0, tk1, tv1, to, p);
 }
 
 template <int MODE>
@@ -586,18 +587,11 @@ int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& ma
     p.tiles_n = p.tiles_n_seg * n_seg;
     const int n_tiles = p.tiles_m * p.tiles_n, max_groups = st->sm_count / per_group;
     const int groups = n_tiles < max_groups ? n_tiles : max_groups;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(groups * per_group));
-    cfg.blockDim = dim3(G_THREADS);
-    cfg.dynamicSmemBytes = G_SMEM;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = per_group; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = per_group; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
     ProfScope ps(st, KB_PROF_LINEAR, stream);
-    return cudaLaunchKernelEx(&cfg, gemm16_kernel<EPI, PAIR>, ta, maps, p) == cudaSuccess ? KB_OK : KB_ERR_CUDA;
+    return launch_dependent(gemm16_kernel<EPI, PAIR>, dim3((unsigned)(groups * per_group)), dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
 }
 
 // CTA pairs on 256x256 tiles when that fills the device better. Measured on B200 a CTA of a pair spends about 11/8 of the
@@ -816,8 +810,8 @@ int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, cons
         const long long warps = (long long)B * H * ((Tq + 127) / 128) * 128;
         const unsigned grid = (unsigned)((warps + 7) / 8);
         // dO as the tensor cores see it (fp16), so that the rows of dS sum to zero as exactly as the products allow
-        bwd_delta_kernel<<<grid, 256, 0, stream>>>(stats, static_cast<const __half*>(gg), ldg, o16, H * 128, B, Tq, H);
-        if (cudaGetLastError() != cudaSuccess) return KB_ERR_CUDA;
+        if ((rc = launch_dependent(bwd_delta_kernel, dim3(grid), dim3(256), 0, stream, nullptr, stats, static_cast<const __half*>(gg), ldg, o16, H * 128, B, Tq, H)))
+            return rc;
     }
     CUtensorMap tq, tk, tv, tg;
     if ((rc = make_tmap(&tq, qq, Tq, H, B, ldq)) || (rc = make_tmap(&tk, kk, Tk, H, B, ldk)) || (rc = make_tmap(&tv, vv, Tk, H, B, ldv)) ||
@@ -848,14 +842,15 @@ int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, cons
     }
     const long long n_dkv = (long long)B * H * ((Tk + 127) / 128) * qsplit, n_dq = (long long)B * H * ((Tq + 127) / 128);
     if (n_dkv + n_dq > 0x7fffffffLL) return KB_ERR_SHAPE;
-    attn_bwd_kernel<<<(unsigned)(n_dkv + n_dq), BWD_THREADS, BWD_SMEM, stream>>>(tq, tk, tv, tg, tdq, tdk, tdv, p, (int)n_dkv);
-    if (cudaGetLastError() != cudaSuccess) return KB_ERR_CUDA;
+    if ((rc = launch_dependent(attn_bwd_kernel, dim3((unsigned)(n_dkv + n_dq)), dim3(BWD_THREADS), BWD_SMEM, stream, nullptr, tq, tk, tv, tg, tdq, tdk, tdv,
+                               p, (int)n_dkv)))
+        return rc;
     if (qsplit > 1) {
         const size_t n = (size_t)B * Tk * H * 32;                 // one thread per four columns
-        bwd_reduce_kernel<<<dim3((unsigned)((n + 255) / 256), 2), 256, 0, stream>>>(static_cast<float*>(dk), ld_dk, static_cast<float*>(dv), ld_dv, part_dk,
-                                                                                   part_dv, B * Tk, H * 128, qsplit);
+        return launch_dependent(bwd_reduce_kernel, dim3((unsigned)((n + 255) / 256), 2), dim3(256), 0, stream, nullptr, static_cast<float*>(dk), ld_dk,
+                                static_cast<float*>(dv), ld_dv, part_dk, part_dv, B * Tk, H * 128, qsplit);
     }
-    return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_CUDA;
+    return KB_OK;
 }
 
 int kb_cross_kv(void* k16, void* v16, int ld_out, const void* ctx, int ld_ctx, int ctx_dtype, int L, int N, int K, const void* Wk,

@@ -76,6 +76,8 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
 // (rows past Tq get 0). dO fp16 as staged for the tensor cores, O fp16 from the forward pass (its 16-bit output path: bulk
 // tensor stores instead of per-thread fp32 row stores; the rounding moves D by ~1e-4 of the dP it is subtracted from).
 __global__ void bwd_delta_kernel(float* stats, const __half* dout, int ld_do, const __half* o, int ld_o, int B, int Tq, int H) {
+    pdl_launch();
+    pdl_wait();
     const int nqb = (Tq + BM - 1) / BM;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -129,10 +131,12 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
+    pdl_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
 
     if (warp < 8) {
         setmaxnreg_inc<BWD_SOFTMAX_REGS>();
@@ -372,6 +376,8 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
 // dk / dv [B*Tk, ld] = sum over the qsplit partial results [qsplit][B*Tk][cols] in scratch, in the order of the parts
 // (bit-identical from run to run); one thread per four columns of a row, both tensors in one launch (blockIdx.y).
 __global__ void bwd_reduce_kernel(float* dk, int ld_dk, float* dv, int ld_dv, const float* part_dk, const float* part_dv, int rows, int cols, int qsplit) {
+    pdl_launch();
+    pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t per_row = (size_t)cols / 4;
     if (i >= (size_t)rows * per_row) return;

@@ -312,10 +312,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
+    pdl_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();                                                   // nothing in global memory is touched before this
 
     // 384 threads start with 168 registers each; the MMA/TMA warpgroup gives most of its share to the
     // softmax ones. Everything a softmax thread runs from here on sits inside this branch so that the

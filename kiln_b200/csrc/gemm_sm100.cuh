@@ -133,10 +133,12 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
         tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);                       // two accumulator buffers
         tmem_relinquish();
     }
+    pdl_launch();
     tc_fence_before();
     if (PAIR) { cluster_arrive(); cluster_wait(); } else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
 
     if (warp < G_EPI_WARPS) {
         setmaxnreg_inc<224>();                                            // the row buffers of the epilogue live in registers

@@ -14,6 +14,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace kb {
 
 // eight consecutive elements as fp32
@@ -114,6 +116,13 @@ struct PrepParams {
     int zero_n;                  // attention kernel launched next on the stream expects at zero)
 };
 
+// Clears the words of a call that stages nothing (a kernel and not a memset, so that the chain of dependent launches holds).
+__global__ void zero_words_kernel(unsigned int* ptr, int n) {
+    pdl_launch();
+    pdl_wait();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ptr[i] = 0u;
+}
+
 // Measured on B200: a plain one-16-byte-load-per-thread conversion runs at the speed of a device copy
 // (101 MB in 18.6 us), and unrolling for more loads in flight buys nothing; what costs bandwidth is
 // occupancy and narrow accesses. So: no loop, one pass, 16-byte accesses for 16-bit data everywhere, and a thread
@@ -127,6 +136,8 @@ constexpr int PREP_ITEMS_PER_BLOCK_ROPE = 32;   // 256 threads / 8 lanes
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(256)
 qk_prep_kernel(const __grid_constant__ PrepParams pp) {
+    pdl_launch();
+    pdl_wait();
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < pp.zero_n; i += 256) pp.zero_ptr[i] = 0u;
     int si = 0;

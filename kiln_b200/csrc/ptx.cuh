@@ -16,6 +16,16 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// ---------------------------------------------------------------- dependent launches
+// Kernels of this library are launched with programmatic stream serialization: a kernel may be placed on SMs that its predecessor on
+// the stream has left while the predecessor's last blocks still run. pdl_launch() allows that for the kernel behind this one;
+// pdl_wait() returns once every kernel in front has completed and its writes are visible. A kernel touches no global memory before
+// its pdl_wait(), and every thread that touches any executes it; only its own set-up (barriers, TMEM, tensor map prefetch) runs ahead.
+// Measured back to back on B200: 1.5-3 us per kernel boundary; self-attention of 1000 fp32 tokens (two kernels) 32.8 -> 28.8 us, the
+// gradients of a self- and a cross-attention at 1024 tokens (ten kernels) 135.5 -> 119.2 us, 4096 tokens (167 us) unchanged.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
