@@ -97,6 +97,7 @@ int init_device(DeviceState& st, int dev) {
     if ((rc = set_smem(attn_fwd_kernel<MODE_PAIR, __half>, ATTN_SMEM_PAIR))) return rc;
     if ((rc = set_smem(attn_fwd_kernel<MODE_PAIR, __nv_bfloat16>, ATTN_SMEM_PAIR))) return rc;
     if ((rc = set_smem(attn_fwd_kernel<MODE_PAIR, float>, ATTN_SMEM_PAIR))) return rc;
+    if ((rc = set_smem(attn_fwd_kernel<MODE_PAIR, RowStats>, ATTN_SMEM_PAIR))) return rc;
     if ((rc = set_smem(attn_fwd_kernel<MODE_NAG, __half>, ATTN_SMEM_NAG))) return rc;
     if ((rc = set_smem(attn_fwd_kernel<MODE_NAG, __nv_bfloat16>, ATTN_SMEM_NAG))) return rc;
     if ((rc = set_smem(attn_fwd_kernel<MODE_NAG, float>, ATTN_SMEM_NAG))) return rc;
@@ -224,6 +225,8 @@ int launch_attn(int out_dtype, const CUtensorMap& tq, const CUtensorMap& tk0, co
     // 16-bit outputs of single-GPU calls leave through TMA stores: [B][Tq][H*128] view of `out`, box = 64 columns x 128 rows
     CUtensorMap to;
     memset(&to, 0, sizeof(to));
+    if constexpr (MODE == MODE_PAIR)
+        if (p.stats) return launch_attn_t<MODE_PAIR, RowStats>(tq, tk0, tv0, tk1, tv1, to, p, sm_count, stream);
     if (out_dtype != KB_F32 && p.n_peers == 0) {
         const cuuint64_t dims[3] = {(cuuint64_t)p.H * 128, (cuuint64_t)p.Tq, (cuuint64_t)p.B};
         const cuuint64_t strides[2] = {(cuuint64_t)p.ldo * 2, (cuuint64_t)p.Tq * (cuuint64_t)p.ldo * 2};
@@ -295,11 +298,18 @@ bool split_pays(int n_items, int nb, int sm_count) {
     return balanced < whole;
 }
 
+// what the backward pass wants from the forward one instead of O (AttnParams::stats)
+struct GradSpec {
+    float* stats;
+    const __half* dout;
+    int ld_do;
+};
+
 // shared body of self- and cross-attention: q [B*Tq], k/v [B*Tk]
 int attn_pair(void* out, const void* q, const void* k, const void* v, const void* qn_w, const void* kn_w,
               const float* rope_cos, const float* rope_sin, int B, int Tq, int Tk, int npad, int H, int ld_q, int ld_k,
               int ld_v, int ld_o, int dtype, int out_dtype, float eps, void* workspace, size_t workspace_bytes,
-              cudaStream_t stream, const PeerSpec* peers = nullptr, float* stats = nullptr) {
+              cudaStream_t stream, const PeerSpec* peers = nullptr, const GradSpec* grad = nullptr) {
     if (!valid_in_dtype(dtype)) return KB_ERR_ARG;
     if (B <= 0 || Tq <= 0 || Tk <= 0 || H <= 0 || npad < 0) return KB_ERR_ARG;
     if (peers) {
@@ -317,7 +327,7 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     if (!aligned16(qn_w) || !aligned16(kn_w) || !aligned16(rope_cos) || !aligned16(rope_sin)) return KB_ERR_ALIGN;
     int rc;
     if ((rc = check_mat(q, ld_q, H, dtype)) || (rc = check_mat(k, ld_k, H, dtype)) || (rc = check_mat(v, ld_v, H, dtype)) ||
-        (rc = check_out(out, ld_o, H, out_dtype)))
+        (!grad && (rc = check_out(out, ld_o, H, out_dtype))))
         return rc;
     DeviceState* st;
     if ((rc = get_state(&st))) return rc;
@@ -340,7 +350,7 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     p.n_items = ((Tq + 2 * BM - 1) / (2 * BM)) * H * B;
     p.scale_log2 = SCALE_LOG2;
     p.status = st->status;
-    p.stats = stats;
+    if (grad) { p.stats = grad->stats; p.dout = grad->dout; p.ld_do = grad->ld_do; }
     // Balanced schedule: worth it when equal (item, key block) ranges per SM beat whole items per SM by more than the
     // cost of writing and merging the cut items' partial results (about two key blocks), and the workspace has room for
     // those partial results; otherwise every CTA takes whole items.
@@ -746,7 +756,9 @@ void bwd_qsplit(int B, int Tq, int Tk, int H, int sm_count, int* qsplit, int* q_
 }
 size_t bwd_partial_bytes(int B, int Tk, int H, int qsplit) { return qsplit > 1 ? 2 * align256((size_t)qsplit * B * Tk * H * 128 * sizeof(float)) : 0; }
 size_t bwd_fixed_bytes(int B, int Tq, int Tk, int H, int dtype) {
-    size_t n = bwd_stats_bytes(B, Tq, H) + align256((size_t)B * Tq * H * 128 * 2);                         // statistics, O (fp16)
+    // statistics; room for an fp16 O, which nothing uses since the forward pass leaves D itself: the least workspace that a call
+    // accepts stays what callers know
+    size_t n = bwd_stats_bytes(B, Tq, H) + align256((size_t)B * Tq * H * 128 * 2);
     if (dtype != KB_F16) n += 2 * align256((size_t)B * Tq * H * 128 * 2) + 2 * align256((size_t)B * Tk * H * 128 * 2);   // fp16 Q, dO, K, V
     return n;
 }
@@ -780,7 +792,7 @@ int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, cons
     if ((rc = get_state(&st))) return rc;
     Stage sg{static_cast<char*>(workspace), workspace_bytes};
     float* stats = static_cast<float*>(sg.take_bytes(bwd_stats_bytes(B, Tq, H)));
-    __half* o16 = static_cast<__half*>(sg.take_bytes((size_t)B * Tq * H * 128 * 2));
+    sg.take_bytes((size_t)B * Tq * H * 128 * 2);                  // see bwd_fixed_bytes
     int qsplit, q_per;
     bwd_qsplit(B, Tq, Tk, H, st->sm_count, &qsplit, &q_per);
     float* part_dk = nullptr;
@@ -802,17 +814,12 @@ int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, cons
     }
     if (sg.overflow) return KB_ERR_WORKSPACE;
     if ((rc = launch_prep(st, pb, dtype, KB_F16, stream))) return rc;
-    // forward on the fp16 operands: O for D, and L into the statistics
-    if ((rc = attn_pair(o16, qq, kk, vv, nullptr, nullptr, nullptr, nullptr, B, Tq, Tk, npad, H, ldq, ldk, ldv, H * 128, KB_F16, KB_F16, 0.f,
-                        sg.ws, sg.left, stream, nullptr, stats)))
+    // forward on the fp16 operands: both statistics of every row (dO as the tensor cores see it, so that the rows of dS sum to zero as
+    // exactly as the products allow)
+    const GradSpec grad{stats, static_cast<const __half*>(gg), ldg};
+    if ((rc = attn_pair(nullptr, qq, kk, vv, nullptr, nullptr, nullptr, nullptr, B, Tq, Tk, npad, H, ldq, ldk, ldv, 0, KB_F16, KB_F16, 0.f, sg.ws, sg.left,
+                        stream, nullptr, &grad)))
         return rc;
-    {
-        const long long warps = (long long)B * H * ((Tq + 127) / 128) * 128;
-        const unsigned grid = (unsigned)((warps + 7) / 8);
-        // dO as the tensor cores see it (fp16), so that the rows of dS sum to zero as exactly as the products allow
-        if ((rc = launch_dependent(bwd_delta_kernel, dim3(grid), dim3(256), 0, stream, nullptr, stats, static_cast<const __half*>(gg), ldg, o16, H * 128, B, Tq, H)))
-            return rc;
-    }
     CUtensorMap tq, tk, tv, tg;
     if ((rc = make_tmap(&tq, qq, Tq, H, B, ldq)) || (rc = make_tmap(&tk, kk, Tk, H, B, ldk)) || (rc = make_tmap(&tv, vv, Tk, H, B, ldv)) ||
         (rc = make_tmap(&tg, gg, Tq, H, B, ldg)))

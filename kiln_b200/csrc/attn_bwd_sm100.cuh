@@ -6,10 +6,10 @@
 // Here nothing of size Tq x Tk exists in memory: like the forward kernel the products are formed tile by tile on the tensor
 // cores (fp16 operands, fp32 accumulation in TMEM) and P is recomputed from a per-row statistic.
 //
-// Four launches (kb_attn_bwd): the staging pre-pass (Q, K, V, dO -> fp16), the forward kernel, which also leaves
-// L_i = log2 of the softmax denominator of row i (npad zero keys included) in the "stats" array, a small kernel for
-// D_i = sum_d dO[i, d] O[i, d] (= sum_j P_ij dP_ij, what k_dsoftmax sums), and this file's kernel, whose thread blocks
-// play one of two roles:
+// Three launches (kb_attn_bwd): the staging pre-pass (Q, K, V, dO -> fp16), the forward kernel in its RowStats form, which stores no
+// O but leaves in the "stats" array L_i = log2 of the softmax denominator of row i (npad zero keys included) and
+// D_i = sum_d dO[i, d] O[i, d] (= sum_j P_ij dP_ij, what k_dsoftmax sums; dO as the tensor cores see it, O in fp32), and this
+// file's kernel, whose thread blocks play one of two roles:
 //
 //   BWD_DKV  one thread block per (key block j, head, image), query blocks i streamed through a two-stage ring:
 //              S^T  = K_j Q_i^T            dP^T = V_j dO_i^T                      (two SS products into TMEM)
@@ -70,30 +70,6 @@ enum { BB_RES = 0, BB_XFULL = 1, BB_XEMPTY = 3, BB_TFULL = 5, BB_PFULL = 7, BB_A
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
-// D_i = sum_d dO[i, d] * O[i, d] per (row, head) into the stats array; one warp per (row, head), rows of whole query blocks
-// (rows past Tq get 0). dO fp16 as staged for the tensor cores, O fp16 from the forward pass (its 16-bit output path: bulk
-// tensor stores instead of per-thread fp32 row stores; the rounding moves D by ~1e-4 of the dP it is subtracted from).
-__global__ void bwd_delta_kernel(float* stats, const __half* dout, int ld_do, const __half* o, int ld_o, int B, int Tq, int H) {
-    pdl_launch();
-    pdl_wait();
-    const int nqb = (Tq + BM - 1) / BM;
-    const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const long long total = (long long)B * H * nqb * BM;
-    if (w >= total) return;
-    const int r = (int)(w % (nqb * BM)), h = (int)((w / (nqb * BM)) % H), b = (int)(w / ((long long)nqb * BM * H));
-    float s = 0.f;
-    if (r < Tq) {
-        const uint2 gv = *reinterpret_cast<const uint2*>(dout + ((size_t)b * Tq + r) * (size_t)ld_do + (size_t)h * HD + lane * 4);
-        const uint2 ow = *reinterpret_cast<const uint2*>(o + ((size_t)b * Tq + r) * (size_t)ld_o + (size_t)h * HD + lane * 4);
-        const float2 ga = __half22float2(*reinterpret_cast<const __half2*>(&gv.x)), gb = __half22float2(*reinterpret_cast<const __half2*>(&gv.y));
-        const float2 oa = __half22float2(*reinterpret_cast<const __half2*>(&ow.x)), ob = __half22float2(*reinterpret_cast<const __half2*>(&ow.y));
-        s = ga.x * oa.x + ga.y * oa.y + gb.x * ob.x + gb.y * ob.y;
-    }
-    for (int o2 = 16; o2 > 0; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-    if (lane == 0) stats[(((size_t)b * H + h) * nqb + r / BM) * 256 + 128 + (r % BM)] = s;
 }
 
 // One thread block's work in either role: (blk, h, b) = (key block, head, image) for BWD_DKV, (query block, head, image) for BWD_DQ.

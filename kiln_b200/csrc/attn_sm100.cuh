@@ -128,9 +128,12 @@ struct AttnParams {
     // (nag_flag_peers), so each GPU blends with the norms over all heads; the counters only grow (nag_epoch-th call).
     int nag_heads, nag_h0;
     unsigned int nag_epoch;
-    // MODE_PAIR, optional (the backward pass): [B][H][ceil(Tq/128)][2][128] floats; the first 128 of a query block receive
-    // L = log2 of each row's softmax denominator in units of scale_log2 * score (so that P = 2^(scale_log2 * s - L))
+    // MODE_PAIR with RowStats output (the backward pass): [B][H][ceil(Tq/128)][2][128] floats per query block; the first 128 receive
+    // L = log2 of each row's softmax denominator in units of scale_log2 * score (so that P = 2^(scale_log2 * s - L)), the others
+    // D = sum_d dO[row, d] O[row, d] (0 for rows past Tq)
     float* stats;
+    const __half* dout; // RowStats: dO [B*Tq, ld_do]
+    int ld_do;
     float* nag_part_peers[MAX_PEERS];
     unsigned int* nag_flag_peers[MAX_PEERS];
     int split;          // MODE_PAIR: balanced (item, key block) ranges per CTA with partial results merged
@@ -175,6 +178,11 @@ __device__ __forceinline__ void store32(OutT* dst, const float (&v)[32]) {
                                                           pack16<DT>(v[8 * i + 4], v[8 * i + 5]), pack16<DT>(v[8 * i + 6], v[8 * i + 7]));
     }
 }
+
+// "Output type" of the forward pass inside the backward one (MODE_PAIR): nothing of O is stored, only the statistics L and D of its
+// rows. A thread holds a whole row of O in its epilogue, so D costs sixteen 16-byte reads of dO there, in place of a store of O and a
+// second kernel that reads it back: 16.3 us at 4096 tokens x 16 heads, 5.4 us at 1024.
+struct RowStats { float unused; };
 
 // One work segment: which rows, head and batch element, and which 128-key blocks [jb, je[i]) each stream runs
 // (je[i] <= jb: the stream does not exist in this segment). nb = blocks of the whole item (MODE_PAIR).
@@ -671,7 +679,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                             }
                             const float inv = scale / l;
                             const float k_mine = a_mine * inv;
-                            if (p.stats)
+                            if constexpr (std::is_same<OutT, RowStats>::value)
                                 p.stats[(((size_t)it.b * p.H + it.h) * ((p.Tq + BM - 1) / BM) + (size_t)(it.q0 / BM + i)) * 256 + t] =
                                     (p.npad[0] ? fmaxf(Mf, 0.f) : Mf) + log2f(l);
                             // one 32-column chunk of the merged, normalised row
@@ -772,6 +780,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                     named_bar_sync(3 + i, 128);                  // every warp is done with the staging tile
                                     if (t < p.n_peers) atomicAdd_system(p.ctr_peers[t], 1ull);
                                 }
+                            } else if constexpr (std::is_same<OutT, RowStats>::value) {
+                                const int row = it.q0 + i * BM + t;
+                                const uint4* const g = reinterpret_cast<const uint4*>(p.dout + ((size_t)it.b * p.Tq + (size_t)min(row, p.Tq - 1)) * (size_t)p.ld_do +
+                                                                                      (size_t)it.h * HD);
+                                float D = 0.f;
+#pragma unroll
+                                for (int q = 0; q < 4; q++) {
+                                    uint4 g4[4];
+#pragma unroll
+                                    for (int cc = 0; cc < 4; cc++) g4[cc] = __ldg(g + 4 * q + cc);
+                                    float v[32];
+                                    chunk(q, v);
+#pragma unroll
+                                    for (int cc = 0; cc < 4; cc++) {
+                                        const uint32_t gw[4] = {g4[cc].x, g4[cc].y, g4[cc].z, g4[cc].w};
+#pragma unroll
+                                        for (int e = 0; e < 4; e++) {
+                                            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
+                                            D = fmaf(gf.x, v[8 * cc + 2 * e], fmaf(gf.y, v[8 * cc + 2 * e + 1], D));
+                                        }
+                                    }
+                                }
+                                p.stats[(((size_t)it.b * p.H + it.h) * ((p.Tq + BM - 1) / BM) + (size_t)(it.q0 / BM + i)) * 256 + BM + t] = row < p.Tq ? D : 0.f;
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(bar(BAR_OFREE + i));
                             } else {
                                 const int row = it.q0 + i * BM + t;
                                 OutT* dst = reinterpret_cast<OutT*>(p.out) + ((size_t)it.b * p.Tq + (size_t)row) * (size_t)p.ldo + (size_t)it.h * HD;
