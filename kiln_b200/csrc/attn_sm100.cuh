@@ -19,6 +19,10 @@
 //               norms in a small global scratch, bump a per-tile counter and wait, bounded, for the
 //               other heads. Nothing but the blended result is written as output.
 //
+//   MODE_KEYS : one 128-row query tile of one (batch, head); stream 0 runs the even 128-key blocks of its K/V sequence, stream 1
+//               the odd ones, and the epilogue merges the two (m, l, O). Twice the items of MODE_PAIR at half the length: for
+//               few query tiles (keys_cost in abi.cu has the rule and what both sides measured).
+//
 // Warp roles (384 threads): warps 0-3 / 4-7: softmax of stream 0 / 1 (warp w owns TMEM lanes 32*(w%4)..+31,
 // one query row per thread), warps 8 / 10 issue the MMAs of stream 0 / 1 (one lane each), warp 9 issues TMA loads
 // (one lane), warp 11 idle.
@@ -62,7 +66,7 @@
 
 namespace kb {
 
-constexpr int MODE_PAIR = 0, MODE_NAG = 1;
+constexpr int MODE_PAIR = 0, MODE_NAG = 1, MODE_KEYS = 2;
 constexpr int DT_F16 = 0, DT_BF16 = 1;
 
 constexpr int HD = 128;                 // head size
@@ -70,7 +74,8 @@ constexpr int BM = 128;                 // query rows per stream tile
 constexpr int BN = 128;                 // keys per block
 constexpr int TILE_BYTES = BM * HD * 2; // 32 KiB: one Q, K or V tile (two 64-column swizzled halves)
 constexpr int HALF_BYTES = TILE_BYTES / 2;
-constexpr int NSTAGE = 4;               // K/V ring depth
+constexpr int NSTAGE = 4;               // K/V ring depth of MODE_PAIR and MODE_NAG
+constexpr int NSTAGE_KEYS = 6;          // of MODE_KEYS, whose streams share no tile (four new ones per step of both streams)
 #ifndef KB_POLY_PAIRS
 #define KB_POLY_PAIRS 0
 #endif
@@ -90,10 +95,13 @@ static_assert(256 * SOFTMAX_REGS + 128 * OTHER_REGS == ATTN_THREADS * 168 && OTH
 // runs still stage in the Q tile), 1 KB of barriers and shared words. MODE_NAG: Q, two tiles holding the previous item's unblended g and Z+ as fp16 (see the
 // NAG epilogue), K/V ring, 3 KB control block (barriers, words, 2.5 KB of epilogue scratch): exactly the 227 KB a thread
 // block may have.
+// MODE_KEYS: Q (the output is staged in it: an SM has one item, so nobody waits for the space), K/V ring, NAG's control block.
 constexpr int CTRL_BYTES_PAIR = 1024, CTRL_BYTES_NAG = 3072;
 constexpr int ATTN_TILES_PAIR = 3 + NSTAGE, ATTN_TILES_NAG = 3 + NSTAGE;
 constexpr int ATTN_SMEM_PAIR = ATTN_TILES_PAIR * TILE_BYTES + CTRL_BYTES_PAIR;
 constexpr int ATTN_SMEM_NAG = ATTN_TILES_NAG * TILE_BYTES + CTRL_BYTES_NAG;
+constexpr int ATTN_SMEM_KEYS = (1 + NSTAGE_KEYS) * TILE_BYTES + CTRL_BYTES_NAG;
+constexpr int attn_smem(int mode) { return mode == MODE_PAIR ? ATTN_SMEM_PAIR : mode == MODE_NAG ? ATTN_SMEM_NAG : ATTN_SMEM_KEYS; }
 static_assert(ATTN_SMEM_NAG <= 232448, "shared memory per thread block on sm_100");
 
 // error bits written to the status word
@@ -115,8 +123,8 @@ struct AttnParams {
     unsigned long long* ctr_peers[MAX_PEERS];
     int n_peers, col0;
     int Tq, H, B;
-    int n_items;        // MODE_PAIR: ceil(Tq/256) * H * B; MODE_NAG: ceil(Tq/128) * H
-    int Tk[2];          // MODE_PAIR uses [0]; MODE_NAG: positive, negative context
+    int n_items;        // MODE_PAIR: ceil(Tq/256) * H * B; MODE_NAG: ceil(Tq/128) * H; MODE_KEYS: ceil(Tq/128) * H * B
+    int Tk[2];          // MODE_PAIR and MODE_KEYS use [0] (MODE_KEYS: more than 128 keys, so that both streams exist); MODE_NAG: positive, negative context
     int npad[2];
     float scale_log2;   // log2(e) / sqrt(128)
     float nag_s, nag_tau, nag_alpha;
@@ -128,7 +136,7 @@ struct AttnParams {
     // (nag_flag_peers), so each GPU blends with the norms over all heads; the counters only grow (nag_epoch-th call).
     int nag_heads, nag_h0;
     unsigned int nag_epoch;
-    // MODE_PAIR with RowStats output (the backward pass): [B][H][ceil(Tq/128)][2][128] floats per query block; the first 128 receive
+    // RowStats output (the backward pass): [B][H][ceil(Tq/128)][2][128] floats per query block; the first 128 receive
     // L = log2 of each row's softmax denominator in units of scale_log2 * score (so that P = 2^(scale_log2 * s - L)), the others
     // D = sum_d dO[row, d] O[row, d] (0 for rows past Tq)
     float* stats;
@@ -144,7 +152,8 @@ struct AttnParams {
 
 // barrier slots inside the control block
 enum { BAR_QFULL = 0, BAR_QEMPTY = 2, BAR_SFULL = 4, BAR_SREQ = 6, BAR_PFULL = 8, BAR_PEMPTY = 10, BAR_ODONE = 12, BAR_OFREE = 14,
-       BAR_SFREE = 16, BAR_PARKED = 17, BAR_NORMS = 18, BAR_KVFULL = 20, BAR_KVEMPTY = 20 + NSTAGE, BAR_COUNT = 20 + 2 * NSTAGE };
+       BAR_SFREE = 16, BAR_PARKED = 17, BAR_NORMS = 18, BAR_KVFULL = 20, BAR_KVEMPTY = 20 + NSTAGE_KEYS, BAR_COUNT = 20 + 2 * NSTAGE_KEYS };
+static_assert(BAR_COUNT * 8 <= 256, "the shared words of the control block start at byte 256");
 // when a stream asks for its next S: 0 = before its exponentials, 1 = after the first half of them, 2 = with P (no overlap)
 #ifndef KB_SREQ_AT
 #define KB_SREQ_AT 1
@@ -179,10 +188,25 @@ __device__ __forceinline__ void store32(OutT* dst, const float (&v)[32]) {
     }
 }
 
-// "Output type" of the forward pass inside the backward one (MODE_PAIR): nothing of O is stored, only the statistics L and D of its
+// "Output type" of the forward pass inside the backward one (MODE_PAIR, MODE_KEYS): nothing of O is stored, only the statistics L and D of its
 // rows. A thread holds a whole row of O in its epilogue, so D costs sixteen 16-byte reads of dO there, in place of a store of O and a
 // second kernel that reads it back: 16.3 us at 4096 tokens x 16 heads, 5.4 us at 1024.
 struct RowStats { float unused; };
+
+// dot product of 32 fp16 values (four 16-byte pieces) and 32 floats
+__device__ __forceinline__ float dot32(const uint4 (&g)[4], const float (&v)[32]) {
+    float s = 0.f;
+#pragma unroll
+    for (int cc = 0; cc < 4; cc++) {
+        const uint32_t gw[4] = {g[cc].x, g[cc].y, g[cc].z, g[cc].w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
+            s = fmaf(gf.x, v[8 * cc + 2 * e], fmaf(gf.y, v[8 * cc + 2 * e + 1], s));
+        }
+    }
+    return s;
+}
 
 // One work segment: which rows, head and batch element, and which 128-key blocks [jb, je[i]) each stream runs
 // (je[i] <= jb: the stream does not exist in this segment). nb = blocks of the whole item (MODE_PAIR).
@@ -234,6 +258,15 @@ struct SegIter {
             o.qt = qp;
             o.je[0] = je;
             o.je[1] = (o.q0 + BM < p.Tq) ? je : jb;
+        } else if (MODE == MODE_KEYS) {
+            const int nqt = (p.Tq + BM - 1) / BM;
+            const int hb = item / nqt;
+            o.qt = item % nqt;
+            o.h = hb % p.H;
+            o.b = hb / p.H;
+            o.q0 = o.qt * BM;
+            o.je[0] = (nb + 1) / 2;                               // blocks 0, 2, 4, ... and 1, 3, 5, ...
+            o.je[1] = nb / 2;
         } else {
             o.h = item % p.H;                                     // heads fastest: the heads of a query tile run side by side
             o.qt = item / p.H;
@@ -248,7 +281,7 @@ struct SegIter {
 
 // K/V ring bookkeeping. The loader fills ring entries in a fixed order and every consumer counts the same way:
 //   MODE_PAIR segment: K(jb), then per key block V(j), K(j+1): K(j) is entry 2(j-jb), V(j) entry 2(j-jb)+1 of the segment;
-//   MODE_NAG item: K0(0), K1(0), then per block j and stream i (0 first): V_i(j), K_i(j+1).
+//   MODE_NAG and MODE_KEYS item: K0(0), K1(0), then per block j and stream i (0 first): V_i(j), K_i(j+1).
 // nag_entry returns the entry of V_i(j) within the item (K_i(j+1), when it exists, is the next one).
 __device__ __forceinline__ int nag_entry(int i, int j, int L0, int L1) {
     int e = (L0 > 0) + (L1 > 0);
@@ -279,12 +312,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (threadIdx.x == 0) atomicOr(p.status, ST_TIMEOUT);
         return;
     }
-    constexpr int N_FRONT = MODE == MODE_NAG ? 3 : 2;             // tiles in front of the K/V ring
+    constexpr int N_FRONT = MODE == MODE_NAG ? 3 : MODE == MODE_PAIR ? 2 : 1;   // tiles in front of the K/V ring
+    constexpr int NST = MODE == MODE_KEYS ? NSTAGE_KEYS : NSTAGE;
     const uint32_t sQ = base;
-    const uint32_t sKV = base + N_FRONT * TILE_BYTES;             // NSTAGE tiles
+    const uint32_t sKV = base + N_FRONT * TILE_BYTES;             // NST tiles
     constexpr int N_BACK = MODE == MODE_PAIR ? 1 : 0;             // MODE_PAIR: the output staging tile behind the ring
-    uint8_t* const ctrl = smem + (N_FRONT + NSTAGE + N_BACK) * TILE_BYTES;
-    const uint32_t bars = sKV + (NSTAGE + N_BACK) * TILE_BYTES;   // BAR_COUNT x 8 bytes
+    uint8_t* const ctrl = smem + (N_FRONT + NST + N_BACK) * TILE_BYTES;
+    const uint32_t bars = sKV + (NST + N_BACK) * TILE_BYTES;   // BAR_COUNT x 8 bytes
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 256);
     volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(ctrl + 260);
     volatile uint32_t* const warp_ok = reinterpret_cast<volatile uint32_t*>(ctrl + 264);   // [8] per softmax warp
@@ -293,6 +327,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     volatile uint32_t* const sm_item = reinterpret_cast<volatile uint32_t*>(ctrl + 312);   // [1] NAG: query tile of the item just parked
     volatile uint32_t* const sm_store = reinterpret_cast<volatile uint32_t*>(ctrl + 316);  // [3] NAG: {a blended tile waits in the Q tile, its head, its first row}
     float* const fbuf = reinterpret_cast<float*>(ctrl + 512);     // MODE_NAG epilogue scratch: 1/l of both streams [2][128], norm totals [2][128]
+                                                                  // MODE_KEYS: m [2][128], l [2][128], partial D [128]
+    // key block j of stream i as a block of the stream's K/V sequence
+    auto key_block = [](int i, int j) { return MODE == MODE_KEYS ? 2 * j + i : j; };
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -303,8 +340,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (i >= BAR_SREQ && i < BAR_SREQ + 2) count = 4;               // one arrival per softmax warp of the stream
             if (i >= BAR_PFULL && i < BAR_PFULL + 2) count = 4;
             if (i == BAR_SFREE) count = 4;
-            if (i >= BAR_KVEMPTY && i < BAR_KVEMPTY + NSTAGE) count = MODE == MODE_PAIR ? 2 : 1;   // PAIR: both streams use every K/V tile
-            if (i >= BAR_OFREE && i < BAR_OFREE + 2) count = MODE == MODE_NAG ? 8 : 4;   // NAG: both warpgroups read both O
+            if (i == BAR_QEMPTY && MODE == MODE_KEYS) count = 2;            // both warpgroups stage in the Q tile
+            if (i >= BAR_KVEMPTY && i < BAR_KVEMPTY + NST) count = MODE == MODE_PAIR ? 2 : 1;   // PAIR: both streams use every K/V tile
+            if (i >= BAR_OFREE && i < BAR_OFREE + 2) count = MODE != MODE_PAIR ? 8 : 4;   // NAG, KEYS: both warpgroups read both O
             mbar_init(bar(i), count);
         }
         *abort_flag = 0u;
@@ -458,8 +496,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const bool two = MODE == MODE_PAIR && it.je[1] > jb;
             auto release = [&](uint32_t entry) {
                 if (t == 0) {
-                    mbar_arrive(bar(BAR_KVEMPTY + (ring0 + entry) % NSTAGE));
-                    if (MODE == MODE_PAIR && !two) mbar_arrive(bar(BAR_KVEMPTY + (ring0 + entry) % NSTAGE));   // stream 1 is absent: its share too
+                    mbar_arrive(bar(BAR_KVEMPTY + (ring0 + entry) % NST));
+                    if (MODE == MODE_PAIR && !two) mbar_arrive(bar(BAR_KVEMPTY + (ring0 + entry) % NST));   // stream 1 is absent: its share too
                 }
             };
             auto k_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) : (j == 0 ? (i == 1 && it.je[0] > 0 ? 1 : 0) : nag_entry(i, j - 1, it.je[0], it.je[1]) + 1)); };
@@ -483,8 +521,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(BAR_SFREE));
                 release(k_entry(j));                               // S_i(j) is complete: this stream is done with K(j)
-                if (j == j_last && (Tk & (BN - 1))) {              // ragged last block: keys >= Tk score -inf
-                    const int valid = Tk - j * BN;
+                if (key_block(i, j) == j_last && (Tk & (BN - 1))) {   // ragged last block: keys >= Tk score -inf
+                    const int valid = Tk - j_last * BN;
 #pragma unroll
                     for (int q = 0; q < 4; q++)
 #pragma unroll
@@ -706,7 +744,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                     // 16-bit output: the tile leaves in two rounds of 64 columns through this stream's own
                                     // [128][64] staging half (128-byte rows, 128-byte swizzle: what a bulk tensor store reads);
                                     // rows past Tq are clipped by the tensor map
-                                    uint8_t* const half_stage = smem + (2 + NSTAGE) * TILE_BYTES + i * HALF_BYTES;
+                                    uint8_t* const half_stage = smem + (2 + NST) * TILE_BYTES + i * HALF_BYTES;
 #pragma unroll
                                     for (int hh = 0; hh < 2; hh++) {
 #pragma unroll
@@ -792,15 +830,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                     for (int cc = 0; cc < 4; cc++) g4[cc] = __ldg(g + 4 * q + cc);
                                     float v[32];
                                     chunk(q, v);
-#pragma unroll
-                                    for (int cc = 0; cc < 4; cc++) {
-                                        const uint32_t gw[4] = {g4[cc].x, g4[cc].y, g4[cc].z, g4[cc].w};
-#pragma unroll
-                                        for (int e = 0; e < 4; e++) {
-                                            const float2 gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[e]));
-                                            D = fmaf(gf.x, v[8 * cc + 2 * e], fmaf(gf.y, v[8 * cc + 2 * e + 1], D));
-                                        }
-                                    }
+                                    D += dot32(g4, v);
                                 }
                                 p.stats[(((size_t)it.b * p.H + it.h) * ((p.Tq + BM - 1) / BM) + (size_t)(it.q0 / BM + i)) * 256 + BM + t] = row < p.Tq ? D : 0.f;
                                 tc_fence_before();
@@ -823,6 +853,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                             if (t == 0 && sizeof(OutT) == 2 && p.n_peers != 0) mbar_arrive(bar(BAR_QEMPTY + i));
                         }
                     }
+                }
+            } else if (MODE == MODE_KEYS) {
+                // merge the two streams: statistics through shared memory, then each warpgroup takes 64 columns of both O
+                float* const f_m = fbuf;
+                float* const f_l = fbuf + 256;
+                f_m[i * 128 + t] = row_m * c;
+                f_l[i * 128 + t] = row_l;
+                if (lane == 0) warp_ok[warp] = ok ? 1u : 0u;
+                tc_fence_before();
+                named_bar_sync(1, 256);                                       // both streams' O and statistics are final
+                ok = (warp_ok[0] & warp_ok[1] & warp_ok[2] & warp_ok[3] & warp_ok[4] & warp_ok[5] & warp_ok[6] & warp_ok[7]) != 0u;
+                if (ok) {
+                    tc_fence_after();
+                    const float m0 = f_m[t], m1 = f_m[128 + t], Mf = fmaxf(m0, m1);
+                    const float a0 = ex2(m0 - Mf), a1 = ex2(m1 - Mf);
+                    float l = f_l[t] * a0 + f_l[128 + t] * a1, scale = 1.f;
+                    if (p.npad[0]) {                                          // engine/src/tcflash.cuh:140-144
+                        const float mn = fmaxf(Mf, 0.f);
+                        scale = exp2f(Mf - mn);
+                        l = l * scale + (float)p.npad[0] * exp2f(-mn);
+                    }
+                    const float inv = scale / l, k0 = a0 * inv, k1 = a1 * inv;
+                    const uint32_t tA = tmem_base + lane_base + 256u + (uint32_t)(i * 64), tB = tA + 128u;
+                    auto chunk = [&](int q, float (&v)[32]) {                 // columns 64 i + 32 q .. + 31 of the merged, normalised row
+                        uint32_t a[32], b[32];
+                        tmem_ld32(tA + 32u * q, a);
+                        tmem_ld32(tB + 32u * q, b);
+                        tmem_wait_ld();
+                        reg_fence32(a);
+                        reg_fence32(b);
+#pragma unroll
+                        for (int e = 0; e < 32; e++) v[e] = __uint_as_float(a[e]) * k0 + __uint_as_float(b[e]) * k1;
+                    };
+                    auto o_read = [&]() {                                     // both O are read out: the next item's P*V may start
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) { mbar_arrive(bar(BAR_OFREE + 0)); mbar_arrive(bar(BAR_OFREE + 1)); }
+                    };
+                    const int row = it.q0 + t;
+                    if constexpr (sizeof(OutT) == 2) {
+                        constexpr int ODT = std::is_same<OutT, __nv_bfloat16>::value ? DT_BF16 : DT_F16;
+                        // staged as in MODE_PAIR, in the Q tile: every S product of the item has completed
+                        uint8_t* const half_stage = smem + i * HALF_BYTES;
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            float v[32];
+                            chunk(q, v);
+                            if (q == 1) o_read();
+#pragma unroll
+                            for (int cc = 0; cc < 4; cc++)
+                                *reinterpret_cast<uint4*>(half_stage + t * 128 + (((4 * q + cc) ^ (t & 7)) << 4)) =
+                                    make_uint4(pack16<ODT>(v[8 * cc + 0], v[8 * cc + 1]), pack16<ODT>(v[8 * cc + 2], v[8 * cc + 3]),
+                                               pack16<ODT>(v[8 * cc + 4], v[8 * cc + 5]), pack16<ODT>(v[8 * cc + 6], v[8 * cc + 7]));
+                        }
+                        fence_proxy_async_smem();
+                        named_bar_sync(3 + i, 128);                           // the staged half is complete
+                        if (t == 0) {
+                            tma_store_3d(&tmO, smem_u32(half_stage), it.h * HD + 64 * i, it.q0, it.b);
+                            tma_store_commit();
+                            tma_store_wait_read();
+                        }
+                    } else if constexpr (std::is_same<OutT, RowStats>::value) {
+                        const uint4* const g = reinterpret_cast<const uint4*>(p.dout + ((size_t)it.b * p.Tq + (size_t)min(row, p.Tq - 1)) * (size_t)p.ld_do +
+                                                                              (size_t)it.h * HD + i * 64);
+                        float D = 0.f;
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            uint4 g4[4];
+#pragma unroll
+                            for (int cc = 0; cc < 4; cc++) g4[cc] = __ldg(g + 4 * q + cc);
+                            float v[32];
+                            chunk(q, v);
+                            D += dot32(g4, v);
+                        }
+                        o_read();
+                        float* const f_d = fbuf + 512;
+                        if (i == 1) f_d[t] = D;
+                        named_bar_sync(5, 256);
+                        if (i == 0) {
+                            float* const st = p.stats + (((size_t)it.b * p.H + it.h) * ((p.Tq + BM - 1) / BM) + (size_t)it.qt) * 256 + t;
+                            st[0] = (p.npad[0] ? fmaxf(Mf, 0.f) : Mf) + log2f(l);
+                            st[BM] = row < p.Tq ? D + f_d[t] : 0.f;
+                        }
+                    } else {
+                        OutT* dst = reinterpret_cast<OutT*>(p.out) + ((size_t)it.b * p.Tq + (size_t)row) * (size_t)p.ldo + (size_t)it.h * HD + i * 64;
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            float v[32];
+                            chunk(q, v);
+                            if (row < p.Tq) store32<OutT>(dst + 32 * q, v);
+                        }
+                        o_read();
+                    }
+                    if (t == 0) mbar_arrive(bar(BAR_QEMPTY));                 // this warpgroup is done with the Q tile
                 }
             } else {
                 // NAG combine (engine/src/dit.cu:295-324) on Z+ = O0/l0 and Z- = O1/l1 straight from TMEM.
@@ -1010,15 +1134,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 // descriptor words: the high word is common to every tile here (stride between 8-row groups 1024 bytes, 128-byte
                 // swizzle), the low word is the tile's base plus a constant per k step
                 constexpr uint32_t DESC_HI = smem_desc_hi_sw128(1024);
-                const uint32_t q_lo = smem_desc_lo(sQ + (MODE == MODE_NAG ? 0 : i) * TILE_BYTES, 16);
+                const uint32_t q_lo = smem_desc_lo(sQ + (MODE == MODE_PAIR ? i : 0) * TILE_BYTES, 16);
                 const uint32_t tO = tmem_base + 256u + (uint32_t)(i * 128), tP = tmem_base + 128u + (uint32_t)(i * 64);
                 uint32_t ring = 0;                                            // ring slot index, counted exactly as the loader counts
                 uint32_t n_s = 0;                                             // S products issued so far by BOTH warps (they share the staging area in turn)
                 uint32_t qf_cnt = 0, pf_cnt = 0, of_cnt = 0, sr_cnt = 0;
                 bool good = true;
-                auto kv_wait = [&](uint32_t idx) { return mbar_wait(bar(BAR_KVFULL + idx % NSTAGE), (idx / NSTAGE) & 1u, abort_flag); };
-                auto kv_addr = [&](uint32_t idx) { return sKV + (idx % NSTAGE) * TILE_BYTES; };
-                auto q_wait = [&]() { const bool r = mbar_wait(bar(BAR_QFULL + (MODE == MODE_NAG ? 0 : i)), qf_cnt & 1u, abort_flag); ++qf_cnt; return r; };
+                auto kv_wait = [&](uint32_t idx) { return mbar_wait(bar(BAR_KVFULL + idx % NST), (idx / NST) & 1u, abort_flag); };
+                auto kv_addr = [&](uint32_t idx) { return sKV + (idx % NST) * TILE_BYTES; };
+                auto q_wait = [&]() { const bool r = mbar_wait(bar(BAR_QFULL + (MODE == MODE_PAIR ? i : 0)), qf_cnt & 1u, abort_flag); ++qf_cnt; return r; };
                 auto p_wait = [&]() { const bool r = mbar_wait(bar(BAR_PFULL + i), pf_cnt & 1u, abort_flag); ++pf_cnt; tc_fence_after(); return r; };
                 auto sreq_wait = [&]() { const bool r = mbar_wait(bar(BAR_SREQ + i), sr_cnt & 1u, abort_flag); ++sr_cnt; return r; };
                 // O_i (in NAG mode both O) of the previous segment has been read out; passes at once for the first one
@@ -1038,7 +1162,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     return true;
                 };
                 // O_i (+)= P_i V; P_i may be overwritten and O_i rescaled once these MMAs are done
-                auto issue_PV = [&](uint32_t v_saddr, int j, int Tk, bool first) {
+                auto issue_PV = [&](uint32_t v_saddr, int j, int Tk, bool first) {   // j: block of the K/V sequence
                     const int valid = min(BN, Tk - j * BN);
                     const int nkk = (valid + 15) >> 4;                        // 16 keys per MMA; P is 0 past `valid`
                     const uint32_t blo = smem_desc_lo(v_saddr, HALF_BYTES);
@@ -1105,7 +1229,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                     }
                                     good = kv_wait(ring) && (j > 0 || o_free_wait()) && p_wait();
                                     if (!good) break;
-                                    issue_PV(kv_addr(ring), j, p.Tk[i], j == 0);
+                                    issue_PV(kv_addr(ring), key_block(i, j), p.Tk[MODE == MODE_NAG ? i : 0], j == 0);
                                     if (!more) tc_commit(bar(BAR_ODONE + i));
                                 }
                                 ring += more ? 2u : 1u;
@@ -1150,11 +1274,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     ++q_loads[i];
                 };
                 auto load_kv = [&](const CUtensorMap* tm, int row0) {
-                    const uint32_t st = n % NSTAGE;
-                    good = mbar_wait(bar(BAR_KVEMPTY + st), ((n / NSTAGE) & 1u) ^ 1u, abort_flag);
+                    const uint32_t st = n % NST;
+                    good = mbar_wait(bar(BAR_KVEMPTY + st), ((n / NST) & 1u) ^ 1u, abort_flag);
                     if (!good) return;
                     mbar_expect_tx(bar(BAR_KVFULL + st), TILE_BYTES);
-                    load_tile(sKV + st * TILE_BYTES, tm, bar(BAR_KVFULL + st), row0, MODE == MODE_NAG ? 0 : it.b);
+                    load_tile(sKV + st * TILE_BYTES, tm, bar(BAR_KVFULL + st), row0, it.b);
                     ++n;
                 };
                 SegIter<MODE> iter(p);
@@ -1178,12 +1302,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                             if (good && j + 1 < je) load_kv(&tmK0, (j + 1) * BN);
                         }
                     } else {
+                        if (MODE == MODE_KEYS) {
+                            load_kv(&tmK0, 0);
+                            if (good) load_kv(&tmK0, BN);
+                        }
                         const int nmax = max(it.je[0], it.je[1]);
                         for (int j = 0; j < nmax && good; ++j) {
                             for (int i = 0; i < 2 && good; i++) {
                                 if (j >= it.je[i]) continue;
-                                load_kv(i ? &tmV1 : &tmV0, j * BN);
-                                if (good && j + 1 < it.je[i]) load_kv(i ? &tmK1 : &tmK0, (j + 1) * BN);
+                                load_kv(MODE == MODE_NAG && i ? &tmV1 : &tmV0, key_block(i, j) * BN);
+                                if (good && j + 1 < it.je[i]) load_kv(MODE == MODE_NAG && i ? &tmK1 : &tmK0, key_block(i, j + 1) * BN);
                             }
                         }
                     }
@@ -1201,7 +1329,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 // on failure, let the copies already requested land before the CTA's shared memory goes away: a bounded wait on
                 // the FULL barrier of every ring slot and Q tile that still has a request outstanding
                 if (!good || *abort_flag) {
-                    for (uint32_t k = n > (uint32_t)NSTAGE ? n - NSTAGE : 0u; k < n; ++k) drain_wait(bar(BAR_KVFULL + k % NSTAGE), (k / NSTAGE) & 1u);
+                    for (uint32_t k = n > (uint32_t)NST ? n - NST : 0u; k < n; ++k) drain_wait(bar(BAR_KVFULL + k % NST), (k / NST) & 1u);
                     for (int i = 0; i < 2; i++)
                         if (q_loads[i]) drain_wait(bar(BAR_QFULL + i), (q_loads[i] - 1u) & 1u);
                 }

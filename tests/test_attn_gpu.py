@@ -106,6 +106,27 @@ def test_self_batch_and_strides(kb):
         assert_close(a[sl].float().cpu().numpy(), ref, f"batched self b={b}")
 
 
+@pytest.mark.parametrize("Tq,Tk,npad,B,out_kind", [(1, 129, 383, 1, "f16"), (129, 256, 0, 1, "f32"), (128, 257, 255, 1, "bf16"), (300, 384, 0, 2, "f16"),
+                                                   (1152, 512, 0, 1, "f32"), (1025, 1153, 0, 1, "f16")])
+def test_few_query_tiles_with_the_keys_split_over_both_streams(kb, Tq, Tk, npad, B, out_kind):
+    """At most one 128-row query tile per SM and more than 128 keys: even and odd key blocks run as two streams that the epilogue
+    merges. Uneven block counts, ragged last block in either stream, one valid key in it, padding, images, every output type."""
+    H, kind = 2, "bf16" if out_kind == "bf16" else "f16"
+    q, k, v = seeded(21, B * Tq, H * 128, kind), seeded(22, B * Tk, H * 128, kind), seeded(23, B * Tk, H * 128, kind)
+    for b in range(B):
+        k[b * Tk + Tk - 1] *= 2                                # the last key, alone in its block or not, weighs more (times a power of
+                                                               # two: still exact in 16 bits, so that oracle and kernel see the same keys)
+    if B == 1:
+        out = _cross(kb, q, k, v, Tq, Tk, npad, H, kind, out_kind)
+    else:
+        Tk, k, v = Tq, k[:B * Tq], v[:B * Tq]
+        out = _self(kb, q, k, v, B, Tq, H, kind, out_kind)
+    for b in range(B):
+        qs, ks = slice(b * Tq, (b + 1) * Tq), slice(b * Tk, (b + 1) * Tk)
+        ref = oracle.attention(q[qs], k[ks], v[ks], H, npad)
+        (assert_close_bf16_storage if out_kind == "bf16" else assert_close)(out[qs], ref, f"{Tq}x{Tk} npad {npad} image {b} {out_kind}")
+
+
 def test_fp32_inputs_as_the_engine_holds_them(kb):
     """Q, K, V in fp32 (engine/src/dit.cu:429-430) with fp16 output: the attention16() contract."""
     T, Tk, H = 300, 77, 4
