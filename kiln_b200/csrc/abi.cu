@@ -309,6 +309,18 @@ bool split_pays(int n_items, int nb, int sm_count) {
 // 20.7 -> 14.9, 1152 22.5 -> 15.6; beyond one round 1280 25.1 -> 28.4, 2048 35.3 -> 42.0, 3456 90.0 (balanced) -> 91.4.
 bool keys_pay(int items_keys, int nb, int sm_count) { return nb >= 2 && items_keys <= sm_count; }
 
+// A 16-bit Q that needs no rotation is normalised and converted by the attention kernel itself, in shared memory, and the pre-pass
+// leaves it out: it would read and write all of Q (T x 2048 x 2 bytes each way) and, for fp16 activations with K and V in fp16, it
+// would be a launch for nothing else. Measured on B200, 16 heads: cross 1536 x 26 fp16 15.2 -> 13.2 us back to back (device time
+// 13.7 -> 10.5), NAG 1536 x (378, 168) fp16 34.9 -> 33.1, NAG 4096 x (512, 512) bf16 75.5 -> 71.7. (With RoPE a thread would read 512 bytes of tables per row, one line per lane: slower than the
+// pre-pass. An fp32 tile does not fit into the 32 KB of a Q tile.)
+bool prepares_q(int dtype, const float* rope_cos) { return dtype != KB_F32 && !rope_cos; }
+void set_raw_q(AttnParams& p, int dtype, const void* qn_w, float eps) {
+    p.q_raw = dtype == KB_BF16 ? 2 : 1;
+    p.qn_w = static_cast<const __nv_bfloat16*>(qn_w);
+    p.eps = eps;
+}
+
 // what the backward pass wants from the forward one instead of O (AttnParams::stats)
 struct GradSpec {
     float* stats;
@@ -351,7 +363,12 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     pb.pp.H = H; pb.pp.eps = eps;
     const void *qq = q, *kk = k, *vv = v;
     int ldq = ld_q, ldk = ld_k, ldv = ld_v;
-    if (stage_q) { void* d = sg.take((size_t)B * Tq, H); if (d) pb.add(d, H * 128, q, ld_q, B * Tq, Tq, qn_w, rope_cos, rope_sin); qq = d; ldq = H * 128; }
+    // The space for a staged Q is part of the workspace that a call asks for, used or not.
+    const bool q_in_kernel = stage_q && prepares_q(dtype, rope_cos);
+    if (stage_q) {
+        void* d = sg.take((size_t)B * Tq, H);
+        if (!q_in_kernel) { if (d) pb.add(d, H * 128, q, ld_q, B * Tq, Tq, qn_w, rope_cos, rope_sin); qq = d; ldq = H * 128; }
+    }
     if (stage_k) { void* d = sg.take((size_t)B * Tk, H); if (d) pb.add(d, H * 128, k, ld_k, B * Tk, Tk, kn_w, rope_cos, rope_sin); kk = d; ldk = H * 128; }
     if (stage_v) { void* d = sg.take((size_t)B * Tk, H); if (d) pb.add(d, H * 128, v, ld_v, B * Tk, Tk, nullptr, nullptr, nullptr); vv = d; ldv = H * 128; }
     if (sg.overflow) return KB_ERR_WORKSPACE;
@@ -361,6 +378,7 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     p.n_items = ((Tq + 2 * BM - 1) / (2 * BM)) * H * B;
     p.scale_log2 = SCALE_LOG2;
     p.status = st->status;
+    if (q_in_kernel) set_raw_q(p, dtype, qn_w, eps);
     if (grad) { p.stats = grad->stats; p.dout = grad->dout; p.ld_do = grad->ld_do; }
     // Balanced schedule: worth it when equal (item, key block) ranges per SM beat whole items per SM by more than the
     // cost of writing and merging the cut items' partial results (about two key blocks), and the workspace has room for
@@ -511,7 +529,11 @@ static int nag_impl(void* out, const void* q, const void* qn_w, const void* k_po
     const void* kv[4] = {k_pos, v_pos, k_neg, v_neg};
     const int kv_rows[4] = {Tk_pos, Tk_pos, Tk_neg, Tk_neg};
     int ldq = ld_q, ldkv = ld_kv;
-    if (conv || qn_w) { void* d = sg.take((size_t)Tq, H); if (d) pb.add(d, H * 128, q, ld_q, Tq, Tq, qn_w, nullptr, nullptr); qq = d; ldq = H * 128; }
+    const bool q_in_kernel = (conv || qn_w) && prepares_q(dtype, nullptr);
+    if (conv || qn_w) {
+        void* d = sg.take((size_t)Tq, H);
+        if (!q_in_kernel) { if (d) pb.add(d, H * 128, q, ld_q, Tq, Tq, qn_w, nullptr, nullptr); qq = d; ldq = H * 128; }
+    }
     if (conv) {
         for (int i = 0; i < 4; i++) {
             void* d = sg.take((size_t)kv_rows[i], H);
@@ -543,6 +565,7 @@ static int nag_impl(void* out, const void* q, const void* qn_w, const void* k_po
     }
     p.scale_log2 = SCALE_LOG2;
     p.nag_s = scale; p.nag_tau = tau; p.nag_alpha = alpha;
+    if (q_in_kernel) set_raw_q(p, dtype, qn_w, eps);
     p.status = st->status;
     ProfScope ps(st, KB_PROF_NAG, stream);
     return launch_attn<MODE_NAG>(out_dtype, tq, tk0, tv0, tk1, tv1, p, st->sm_count, stream);

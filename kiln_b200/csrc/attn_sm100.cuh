@@ -147,13 +147,20 @@ struct AttnParams {
     int split;          // MODE_PAIR: balanced (item, key block) ranges per CTA with partial results merged
     float* part;        // split: [gridDim.x] slots of PART_CTA_BYTES
     unsigned int* part_flag;  // split: [gridDim.x][2 streams], zero before the launch; 1 = slot written
+    // Q as 16-bit rows that are not yet what the products read: the softmax warps take each Q tile from raw to fp16 in place,
+    // with the per-head RMSNorm when qn_w is set, before the first S product on it. q_raw: 0 = ready as it is, 1 = fp16, 2 = bf16
+    int q_raw;
+    const __nv_bfloat16* qn_w;   // [128] or null
+    float eps;
     uint32_t* status;   // device word, OR-ed with ST_* on failure
 };
 
 // barrier slots inside the control block
 enum { BAR_QFULL = 0, BAR_QEMPTY = 2, BAR_SFULL = 4, BAR_SREQ = 6, BAR_PFULL = 8, BAR_PEMPTY = 10, BAR_ODONE = 12, BAR_OFREE = 14,
-       BAR_SFREE = 16, BAR_PARKED = 17, BAR_NORMS = 18, BAR_KVFULL = 20, BAR_KVEMPTY = 20 + NSTAGE_KEYS, BAR_COUNT = 20 + 2 * NSTAGE_KEYS };
+       BAR_SFREE = 16, BAR_PARKED = 17, BAR_NORMS = 18, BAR_QREADY = 19, BAR_KVFULL = 20, BAR_KVEMPTY = 20 + NSTAGE_KEYS, BAR_COUNT = 20 + 2 * NSTAGE_KEYS };
 static_assert(BAR_COUNT * 8 <= 256, "the shared words of the control block start at byte 256");
+// the Q tile of stream i has been prepared in place (AttnParams::q_raw); MODE_PAIR has two and does not use BAR_NORMS
+__host__ __device__ constexpr int bar_q_ready(int mode, int i) { return mode == MODE_PAIR ? BAR_NORMS + i : BAR_QREADY; }
 // when a stream asks for its next S: 0 = before its exponentials, 1 = after the first half of them, 2 = with P (no overlap)
 #ifndef KB_SREQ_AT
 #define KB_SREQ_AT 1
@@ -206,6 +213,49 @@ __device__ __forceinline__ float dot32(const uint4 (&g)[4], const float (&v)[32]
         }
     }
     return s;
+}
+
+// Preparing a Q tile in shared memory (about 1 us per tile, next to the S product that it delays): N 16-byte pieces, from cc0 on, of row r of a tile of two 128-byte-swizzled halves
+template <bool BF16, int N>
+__device__ __forceinline__ void q_load(float (&x)[8 * N], const uint8_t* tile, int r, int cc0) {
+    uint4 u[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) u[c] = *reinterpret_cast<const uint4*>(tile + ((cc0 + c) >> 3) * HALF_BYTES + r * 128 + ((((cc0 + c) & 7) ^ (r & 7)) << 4));
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+        const uint32_t w[4] = {u[c].x, u[c].y, u[c].z, u[c].w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if constexpr (BF16) {                                          // a bf16 is the top half of an fp32
+                x[8 * c + 2 * e] = __uint_as_float(w[e] << 16);
+                x[8 * c + 2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+            } else {
+                const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                x[8 * c + 2 * e] = h.x;
+                x[8 * c + 2 * e + 1] = h.y;
+            }
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ float q_sumsq(const float (&x)[N]) {
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int e = 0; e < N; e += 4) {
+        s0 = fmaf(x[e], x[e], s0); s1 = fmaf(x[e + 1], x[e + 1], s1); s2 = fmaf(x[e + 2], x[e + 2], s2); s3 = fmaf(x[e + 3], x[e + 3], s3);
+    }
+    return (s0 + s1) + (s2 + s3);
+}
+// fp16(x * rs * w), as the pre-pass computes it (engine/src/kernels.cu:656-666); w: fp32 weights of the whole row in shared memory
+template <int N>
+__device__ __forceinline__ void q_store(const float (&x)[8 * N], uint8_t* tile, int r, int cc0, float rs, const float* w) {
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+        const float4 wa = *reinterpret_cast<const float4*>(w + 8 * (cc0 + c)), wb = *reinterpret_cast<const float4*>(w + 8 * (cc0 + c) + 4);
+        *reinterpret_cast<uint4*>(tile + ((cc0 + c) >> 3) * HALF_BYTES + r * 128 + ((((cc0 + c) & 7) ^ (r & 7)) << 4)) =
+            make_uint4(pack16<DT_F16>(x[8 * c] * rs * wa.x, x[8 * c + 1] * rs * wa.y), pack16<DT_F16>(x[8 * c + 2] * rs * wa.z, x[8 * c + 3] * rs * wa.w),
+                       pack16<DT_F16>(x[8 * c + 4] * rs * wb.x, x[8 * c + 5] * rs * wb.y), pack16<DT_F16>(x[8 * c + 6] * rs * wb.z, x[8 * c + 7] * rs * wb.w));
+    }
 }
 
 // One work segment: which rows, head and batch element, and which 128-key blocks [jb, je[i]) each stream runs
@@ -327,7 +377,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     volatile uint32_t* const sm_item = reinterpret_cast<volatile uint32_t*>(ctrl + 312);   // [1] NAG: query tile of the item just parked
     volatile uint32_t* const sm_store = reinterpret_cast<volatile uint32_t*>(ctrl + 316);  // [3] NAG: {a blended tile waits in the Q tile, its head, its first row}
     float* const fbuf = reinterpret_cast<float*>(ctrl + 512);     // MODE_NAG epilogue scratch: 1/l of both streams [2][128], norm totals [2][128]
-                                                                  // MODE_KEYS: m [2][128], l [2][128], partial D [128]
+                                                                  // MODE_KEYS: m [2][128], l [2][128], partial D [128] (RowStats, whose Q is never raw)
+    constexpr bool RAW_Q = !std::is_same<OutT, RowStats>::value;  // the backward pass stages its Q
+    float* const f_qw = fbuf + (MODE == MODE_PAIR ? 0 : 512);     // Q norm weights [128] (ones without a norm), when q_raw
     // key block j of stream i as a block of the stream's K/V sequence
     auto key_block = [](int i, int j) { return MODE == MODE_KEYS ? 2 * j + i : j; };
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
@@ -340,6 +392,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (i >= BAR_SREQ && i < BAR_SREQ + 2) count = 4;               // one arrival per softmax warp of the stream
             if (i >= BAR_PFULL && i < BAR_PFULL + 2) count = 4;
             if (i == BAR_SFREE) count = 4;
+            if (i == bar_q_ready(MODE, 0) || i == bar_q_ready(MODE, 1)) count = MODE == MODE_PAIR ? 4 : 8;
             if (i == BAR_QEMPTY && MODE == MODE_KEYS) count = 2;            // both warpgroups stage in the Q tile
             if (i >= BAR_KVEMPTY && i < BAR_KVEMPTY + NST) count = MODE == MODE_PAIR ? 2 : 1;   // PAIR: both streams use every K/V tile
             if (i >= BAR_OFREE && i < BAR_OFREE + 2) count = MODE != MODE_PAIR ? 8 : 4;   // NAG, KEYS: both warpgroups read both O
@@ -364,6 +417,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                                                   // nothing in global memory is touched before this
+    if (RAW_Q && p.q_raw && warp < 8) {                                    // (read by the softmax warps only)
+        if (tid < HD) f_qw[tid] = p.qn_w ? __bfloat162float(p.qn_w[tid]) : 1.f;
+        named_bar_sync(1, 256);
+    }
 
     // 384 threads start with 168 registers each; the MMA/TMA warpgroup gives most of its share to the
     // softmax ones. Everything a softmax thread runs from here on sits inside this branch so that the
@@ -381,6 +438,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const float c = p.scale_log2;
         uint32_t sf_cnt = 0, od_cnt = 0, pe_cnt = 0;               // uses of s_full[i] / o_done[i] / p_empty[i] so far (phase parity)
         uint32_t ring0 = 0;                                        // K/V ring entries of all earlier segments
+        uint32_t q_cnt = 0;                                        // Q tiles prepared so far
 
         // MODE_NAG, 16-bit output: the item parked in shared memory, waiting for its blend
         bool pend_valid = false, pend_go = false;
@@ -502,7 +560,36 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             };
             auto k_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) : (j == 0 ? (i == 1 && it.je[0] > 0 ? 1 : 0) : nag_entry(i, j - 1, it.je[0], it.je[1]) + 1)); };
             auto v_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) + 1 : nag_entry(i, j, it.je[0], it.je[1])); };
-            for (int j = jb; j < je; ++j) {
+            if (RAW_Q && p.q_raw && (MODE != MODE_PAIR || je > jb)) {
+                // MODE_PAIR: a thread takes a whole row of its stream's tile. One Q tile: a thread takes half a row, and the two
+                // halves of a row's sum of squares meet in shared memory (fbuf is free between items).
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_QFULL + (MODE == MODE_PAIR ? i : 0)), q_cnt & 1u, abort_flag));
+                ++q_cnt;
+                if constexpr (MODE == MODE_PAIR) {
+                    uint8_t* const tile = smem + i * TILE_BYTES;
+                    if (ok) {
+                        float x[128];
+                        if (p.q_raw == 2) q_load<true, 16>(x, tile, t, 0);
+                        else q_load<false, 16>(x, tile, t, 0);
+                        q_store<16>(x, tile, t, 0, p.qn_w ? rsqrtf(q_sumsq(x) * (1.f / 128.f) + p.eps) : 1.f, f_qw);
+                    }
+                } else {
+                    float x[64], rs = 1.f;
+                    if (p.q_raw == 2) q_load<true, 8>(x, smem, t, 8 * i);
+                    else q_load<false, 8>(x, smem, t, 8 * i);
+                    if (p.qn_w) {
+                        const float ss = q_sumsq(x);
+                        fbuf[i * 128 + t] = ss;
+                        named_bar_sync(1, 256);
+                        rs = rsqrtf((ss + fbuf[(i ^ 1) * 128 + t]) * (1.f / 128.f) + p.eps);
+                    }
+                    if (ok) q_store<8>(x, smem, t, 8 * i, rs, f_qw);
+                }
+                fence_proxy_async_smem();                          // the products read what was written here
+                __syncwarp();
+                if (lane == 0 && ok) mbar_arrive(bar(bar_q_ready(MODE, i)));
+            }
+            for (int j = jb; j < je && ok; ++j) {
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(BAR_SFULL + i), sf_cnt & 1u, abort_flag));
                 ++sf_cnt;
                 if (!ok) break;
@@ -1142,7 +1229,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 bool good = true;
                 auto kv_wait = [&](uint32_t idx) { return mbar_wait(bar(BAR_KVFULL + idx % NST), (idx / NST) & 1u, abort_flag); };
                 auto kv_addr = [&](uint32_t idx) { return sKV + (idx % NST) * TILE_BYTES; };
-                auto q_wait = [&]() { const bool r = mbar_wait(bar(BAR_QFULL + (MODE == MODE_PAIR ? i : 0)), qf_cnt & 1u, abort_flag); ++qf_cnt; return r; };
+                const uint32_t q_bar = bar(RAW_Q && p.q_raw ? bar_q_ready(MODE, i) : BAR_QFULL + (MODE == MODE_PAIR ? i : 0));
+                auto q_wait = [&]() { const bool r = mbar_wait(q_bar, qf_cnt & 1u, abort_flag); ++qf_cnt; return r; };
                 auto p_wait = [&]() { const bool r = mbar_wait(bar(BAR_PFULL + i), pf_cnt & 1u, abort_flag); ++pf_cnt; tc_fence_after(); return r; };
                 auto sreq_wait = [&]() { const bool r = mbar_wait(bar(BAR_SREQ + i), sr_cnt & 1u, abort_flag); ++sr_cnt; return r; };
                 // O_i (in NAG mode both O) of the previous segment has been read out; passes at once for the first one

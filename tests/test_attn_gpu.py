@@ -197,6 +197,29 @@ def test_self_with_norm_rope_small(kb, Hp, Wp, B, kind):
 
 
 @pytest.mark.parametrize("kind", ["f16", "bf16"])
+@pytest.mark.parametrize("Tq,Tk,norm", [(1, 26, True), (129, 77, True), (300, 128, False), (257, 300, True), (130, 129, False), (2500, 40, True)])
+def test_16_bit_q_prepared_in_the_kernel(kb, Tq, Tk, norm, kind):
+    """Q of a call without RoPE is normalised / converted on its tile in shared memory: one, two and one-and-a-bit tiles, a lone row,
+    one K/V block (two tiles per item), several (one tile, keys split over the streams), more items than SMs; Q a slice of a wider
+    buffer, one all-zero row (its norm divides by sqrt(eps)), magnitudes from 1e-3 to 8 by row."""
+    H, ld = 16 if Tq > 2000 else 3, 24 * 128
+    D = H * 128
+    q = oracle.round16(seeded(31, Tq, D, kind) * np.exp2(np.arange(Tq) % 14 - 10.0).astype(np.float32)[:, None], 0 if kind == "f16" else 1)
+    q[Tq // 2] = 0
+    k, v = seeded(32, Tk, D, kind), seeded(33, Tk, D, kind)
+    wq = oracle.round16(1 + 0.1 * oracle.randn(34, 128), 1)
+    wide = torch.full((Tq, ld), float("nan"), device="cuda", dtype=DT[kind])
+    wide[:, 128:128 + D] = dev(q, kind)
+    out = torch.full((Tq, D), float("nan"), device="cuda")
+    kb.attn_cross(out, wide[:, 128:128 + D], dev(k, kind), dev(v, kind), Tq, Tk, 512 - Tk, H, qn_w=dev(wq).bfloat16() if norm else None,
+                  workspace=_ws(kb, Tq, Tk, H, kind, norm=True))
+    assert kb.check_status() == 0
+    rows = sample_rows(Tq, 24)
+    qr = oracle.rmsnorm(q[rows], _bits(wq), H) if norm else q[rows]
+    assert_close(out.cpu().numpy()[rows], oracle.attention(qr, k, v, H, 512 - Tk), f"{Tq}x{Tk} {kind} norm {norm}")
+
+
+@pytest.mark.parametrize("kind", ["f16", "bf16"])
 def test_q_norm_only_strided_many_items(kb, kind):
     """The cross-attention call pattern on a self-sized problem: Q gets RMSNorm, K arrives normalised; Q/K/V are column
     slices of one buffer, the token count is ragged and there are more work items (160) than SMs."""
