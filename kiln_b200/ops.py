@@ -106,23 +106,40 @@ def lib():
     return _lib
 
 
+# The shortest calls (a cross-attention to a short prompt, 10.5 us of device time) are bound by what Python does per call: so no
+# ctypes objects per argument (the declared argument types take plain integers), no module and dictionary built per call, and the
+# stream as a raw handle. Host time of such a call: 16.5 -> 10.1 us.
+_DT = None       # torch dtype -> KB_* code, filled when torch is first needed
+_raw_stream = _cur_device = None
+
+
 def _dt(t):
-    import torch
-    return {torch.float16: KB_F16, torch.bfloat16: KB_BF16, torch.float32: KB_F32}[t.dtype]
+    global _DT
+    if _DT is None:
+        import torch
+        _DT = {torch.float16: KB_F16, torch.bfloat16: KB_BF16, torch.float32: KB_F32}
+    return _DT[t.dtype]
 
 
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _ld(t):
-    assert t.dim() == 2 and t.stride(1) == 1, "activations are row-major [rows, ld]"
-    return t.stride(0)
+    st = t.stride()
+    assert len(st) == 2 and st[1] == 1, "activations are row-major [rows, ld]"
+    return st[0]
 
 
 def _stream():
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Raw handle of the current stream of the current device."""
+    global _raw_stream, _cur_device
+    if _raw_stream is None:
+        import torch
+        handle = torch.cuda.current_stream().cuda_stream      # initialises CUDA
+        _raw_stream, _cur_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        return handle
+    return _raw_stream(_cur_device())
 
 
 def _check(code, what):
