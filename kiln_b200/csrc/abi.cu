@@ -42,6 +42,7 @@ struct DeviceState {
     int err = KB_OK;
     unsigned int* status = nullptr;
     int sm_count = 148;
+    int max_clusters[3] = {0, 0, 0};   // resident clusters of 2 ([1]) and 4 ([2]) CTAs of the GEMM kernel, one CTA per SM
     Prof prof;
 };
 
@@ -73,9 +74,10 @@ int set_smem(K kernel, int bytes) {
 
 template <int EPI>
 int set_gemm_smem() {
-    if (cudaFuncSetAttribute(gemm16_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm16_kernel<EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM) != cudaSuccess)
-        return KB_ERR_CUDA;
+    int rc;
+    if ((rc = set_smem(gemm16_kernel<EPI, true, false>, G_SMEM)) || (rc = set_smem(gemm16_kernel<EPI, false, false>, G_SMEM)) ||
+        (rc = set_smem(gemm16_kernel<EPI, true, true>, G_SMEM)) || (rc = set_smem(gemm16_kernel<EPI, false, true>, G_SMEM)))
+        return rc;
     return KB_OK;
 }
 
@@ -108,6 +110,17 @@ int init_device(DeviceState& st, int dev) {
     if ((rc = set_gemm_smem<EPI_F32>()) || (rc = set_gemm_smem<EPI_F16>()) || (rc = set_gemm_smem<EPI_GELU16>()) ||
         (rc = set_gemm_smem<EPI_RESID>()) || (rc = set_gemm_smem<EPI_HEADS16>()))
         return rc;
+    for (int i = 1; i <= 2; i++) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2 * i; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(2 * i); cfg.blockDim = dim3(G_THREADS); cfg.dynamicSmemBytes = G_SMEM; cfg.attrs = &attr; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&st.max_clusters[i], gemm16_kernel<EPI_F16, true, true>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            st.max_clusters[i] = 0;                    // no split K then
+        }
+    }
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) return KB_ERR_CUDA;
     st.status = static_cast<unsigned int*>(p);
@@ -630,31 +643,48 @@ int make_tmap_mat(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld) 
 
 // p.N is the width of ONE segment; the launch covers n_seg of them side by side
 template <int EPI, bool PAIR>
-int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, GemmParams p, int n_seg, cudaStream_t stream) {
+int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, GemmParams p, int n_seg, int split_k, cudaStream_t stream) {
     const int tile = PAIR ? 256 : 128, per_group = PAIR ? 2 : 1;
     p.tiles_m = (p.M + tile - 1) / tile;
     p.tiles_n_seg = (p.N + tile - 1) / tile;
     p.tiles_n = p.tiles_n_seg * n_seg;
     const int n_tiles = p.tiles_m * p.tiles_n, max_groups = st->sm_count / per_group;
-    const int groups = n_tiles < max_groups ? n_tiles : max_groups;
+    p.split_k = split_k;
+    const int groups = split_k > 1 || n_tiles < max_groups ? n_tiles : max_groups, ctas = per_group * split_k;   // split_k > 1: one tile per cluster
     cudaLaunchAttribute cluster;
     cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = per_group; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
+    cluster.val.clusterDim.x = ctas; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
     ProfScope ps(st, KB_PROF_LINEAR, stream);
-    return launch_dependent(gemm16_kernel<EPI, PAIR>, dim3((unsigned)(groups * per_group)), dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
+    return launch_dependent(split_k > 1 ? gemm16_kernel<EPI, PAIR, true> : gemm16_kernel<EPI, PAIR, false>, dim3((unsigned)(groups * ctas)),
+                            dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
 }
 
 // CTA pairs on 256x256 tiles when that fills the device better. Measured on B200 a CTA of a pair spends about 11/8 of the
-// time a single CTA spends per 64-wide k step while doing twice the work, so compare waves x time per step.
+// time a single CTA spends per 64-wide k step while doing twice the work, so compare waves x time per step (a step of a single CTA
+// = 8 units of ~43 ns). Either shape cuts the k steps of its tiles over split_k CTAs (pairs) of a cluster when all clusters are
+// resident at once; leaving, meeting and adding the parts costs about 3 us on single CTAs and 4 us on pairs (half of the warps run
+// the epilogue of twice the columns). Measured on B200 inside a CUDA graph, whole k range -> split (* without dependent launches,
+// which save 1.5 us): N 2048, K 8192: M 128 40.2* -> 16.3 us, 512 40.8* -> 25.3, 1024 41.6* -> 29.1; N 2048, K 2048: M 128 14.4* -> 9.2,
+// 512 15.0* -> 11.0; with M 1024 (pairs, head epilogue) 14.7 -> 17.1, so not taken there. N 96 (a stacked LoRA), K 2048, M 1536: 13.4* -> 10.1.
+constexpr int SPLIT_K_COST = 70, SPLIT_K_COST_PAIR = 95;
 template <int EPI>
 int launch_gemm(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, const GemmParams& p, int n_seg, cudaStream_t stream) {
-    if (p.N % 256 == 0 && p.M > 128) {
-        const long long tp = (long long)((p.M + 255) / 256) * (p.N / 256) * n_seg, ts = (long long)((p.M + 127) / 128) * (p.N / 128) * n_seg;
-        const long long gp = st->sm_count / 2, gs = st->sm_count;
-        const long long pair_cost = ((tp + gp - 1) / gp) * 11, single_cost = ((ts + gs - 1) / gs) * 8;
-        if (pair_cost <= single_cost) return launch_gemm_shape<EPI, true>(st, ta, maps, p, n_seg, stream);
+    const long long ksteps = p.K / GB_K;
+    long long best = -1;
+    int best_pair = 0, best_split = 1;
+    for (int pair = 1; pair >= 0; pair--) {
+        if (pair && (p.N % 256 || p.M <= 128)) continue;
+        const int tile = pair ? 256 : 128;
+        const long long tiles = (long long)((p.M + tile - 1) / tile) * ((p.N + tile - 1) / tile) * n_seg;
+        const long long unit = pair ? 11 : 8, groups = pair ? st->sm_count / 2 : st->sm_count;
+        for (int split = 1; split <= (pair ? 2 : 4); split *= 2) {
+            if (split > 1 && (ksteps < 2 * split || tiles > st->max_clusters[pair ? split : split / 2])) continue;
+            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + split - 1) / split) * unit + (split == 1 ? 0 : pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
+            if (best < 0 || cost < best) { best = cost; best_pair = pair; best_split = split; }
+        }
     }
-    return launch_gemm_shape<EPI, false>(st, ta, maps, p, n_seg, stream);
+    if (best_pair) return launch_gemm_shape<EPI, true>(st, ta, maps, p, n_seg, best_split, stream);
+    return launch_gemm_shape<EPI, false>(st, ta, maps, p, n_seg, best_split, stream);
 }
 
 // The second product of a segment (null = none): A2 [M, K2] with row stride lda2, W2 [N, K2] with row stride ldw2.

@@ -9,6 +9,11 @@
 // about 100 B/clk/SM), not by the tensor pipe. Single: one CTA per 128x128 tile, for N not a multiple of 256, M <= 128,
 // or when the pair shape would fill the device worse (the host decides).
 //
+// Split K (p.split_k = 2 or 4): with fewer tiles than half of the SMs the k steps of a tile are cut into split_k ranges, one CTA (or
+// pair) each, all of a tile in one cluster. Every CTA leaves the accumulator rows that it does not finish in its own shared memory
+// (the operand ring, which is free by then); after a cluster barrier the CTA that owns a quarter (split_k = 4) or a half of the rows
+// adds the others' parts from there, in a fixed order, and runs the epilogue on them. No scratch memory, no atomics.
+//
 // It takes the place of the reference's fp16-activation GEMM tc16::k_gemm16 (engine/src/tcgemm16.cuh:57-175,
 // host wrapper linear16 at engine/src/kernels.cu:559-609) with its four epilogues — fp32 store, fp16 store,
 // fp16 GELU, gated add into the fp32 residual stream (engine/src/tcgemm16.cuh:145-174) — and adds a fifth that the
@@ -51,6 +56,7 @@ struct GemmParams {
     // A2_s[M, K2_s] * W2_s[N, K2_s]^T, as further k steps after the first product's, so every epilogue sees the sum.
     // K2 = 0: none. A last partial k step reads zeros past column K2 (the tensor maps fill out-of-range elements).
     int K2[3];
+    int split_k;                   // CTAs (pairs) that share a tile's k steps: 1, 2, or 4 (not PAIR). > 1: one tile per cluster
     int tiles_m, tiles_n;          // in tiles of the launched shape (256x256 for PAIR, 128x128 otherwise)
     // Up to three weight matrices [N, K] share one launch (the q, k, v projections of one activation): column tile tn
     // belongs to segment tn / tiles_n_seg, which has its own W and C tensor maps and its own head epilogue settings.
@@ -94,7 +100,7 @@ __global__ void lora_pack_kernel(__half* dst, int ld, int col0, const __nv_bfloa
     dst[(size_t)r * ld + col0 + c] = __float2half_rn(scale * __bfloat162float(src[i]));
 }
 
-template <int EPI, bool PAIR>
+template <int EPI, bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ GemmMaps maps, const GemmParams p) {
     constexpr int BN = PAIR ? 256 : 128;                                  // accumulator columns per tile
@@ -117,9 +123,46 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;                  // 0 issues the MMAs
-    const int group = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-    const int n_groups = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int S = SPLIT ? p.split_k : 1;
+    const uint32_t crank = (PAIR || SPLIT) ? cluster_ctarank() : 0u;
+    const uint32_t rank = PAIR ? crank & 1u : 0u;                         // 0 issues the MMAs
+    const uint32_t lead = crank - rank;                                   // the issuing CTA of this pair
+    const int part = PAIR ? (int)(crank >> 1) : (int)crank;               // which range of the k steps
+    const int group = (int)blockIdx.x / ((PAIR ? 2 : 1) * S);
+    const int n_groups = (int)gridDim.x / ((PAIR ? 2 : 1) * S);
+    // split K: the part that finishes a lane quarter, and the others' share of its accumulator ([column / 4][row][4] in their rings)
+    auto owner = [&](int quarter) { return S == 4 ? quarter : S == 2 ? quarter >> 1 : 0; };
+    auto add_parts = [&](float (&v)[32], int col, int row) {
+        for (int o = 0; o < S; o++) {
+            if (o == part) continue;
+            const uint32_t src = mapa_u32(sRing, (uint32_t)o * (PAIR ? 2u : 1u) + rank) + (uint32_t)((col >> 2) * GB_M + row) * 16u;
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float4 x = ld_cluster_v4(src + (uint32_t)(e * GB_M * 16));
+                v[4 * e] += x.x; v[4 * e + 1] += x.y; v[4 * e + 2] += x.z; v[4 * e + 3] += x.w;
+            }
+        }
+    };
+    // split K, all epilogue warps: leave what other parts finish in the ring, meet them; true if this warp has rows to finish
+    auto exchange_parts = [&](uint32_t acc, int quarter, int half, bool ok) {
+        if (ok && owner(quarter) != part) {
+#pragma unroll 1
+            for (int col = half * (BN / 2); col < (half + 1) * (BN / 2); col += 32) {
+                uint32_t a[32];
+                tmem_ld32(acc + (uint32_t)col, a);
+                tmem_wait_ld();
+                reg_fence32(a);
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    *reinterpret_cast<uint4*>(smem + ((col >> 2) + e) * (GB_M * 16) + (quarter * 32 + (threadIdx.x & 31)) * 16) =
+                        make_uint4(a[4 * e], a[4 * e + 1], a[4 * e + 2], a[4 * e + 3]);
+            }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        return ok && owner(quarter) == part;
+    };
     const int n_tiles = p.tiles_m * p.tiles_n, ksteps1 = p.K / GB_K;
 
     if (tid == 0) {
@@ -195,6 +238,10 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 named_bar_sync(pair_bar, 64);
                 ok = ok_buf[0] != 0u && ok_buf[1] != 0u;
                 named_bar_sync(pair_bar, 64);
+                if (SPLIT) {
+                    tc_fence_after();
+                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BN), quarter, hs, ok);
+                }
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
@@ -210,11 +257,15 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
 #pragma unroll
                         for (int e = 0; e < 32; e++) { x0[e] = __uint_as_float(a0[e]); x1[e] = __uint_as_float(a1[e]); }
                     }
+                    if (SPLIT) {
+                        add_parts(x0, h * 128 + hs * 32, quarter * 32 + lane);
+                        add_parts(x1, h * 128 + 64 + hs * 32, quarter * 32 + lane);
+                    }
                     if (h == NH - 1) {                                    // this warp's share of the accumulator is in registers
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) {
-                            if (PAIR && rank != 0) mbar_arrive_cluster(mapa_u32(bar(GBAR_ACC_EMPTY + buf), 0));
+                            if (PAIR && rank != 0) mbar_arrive_cluster(mapa_u32(bar(GBAR_ACC_EMPTY + buf), lead));
                             else mbar_arrive(bar(GBAR_ACC_EMPTY + buf));
                         }
                     }
@@ -289,8 +340,12 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 gemm_tile(w, p, tm, tn);
                 const int seg = tn / p.tiles_n_seg;
                 const int m0 = tm * TILE_M + (int)rank * GB_M, n0 = (tn - seg * p.tiles_n_seg) * BN;
-                const bool ok = __all_sync(0xffffffffu, mbar_wait(bar(GBAR_ACC_FULL + buf), use[buf] & 1u, abort_flag));
+                bool ok = __all_sync(0xffffffffu, mbar_wait(bar(GBAR_ACC_FULL + buf), use[buf] & 1u, abort_flag));
                 ++use[buf];
+                if (SPLIT) {
+                    tc_fence_after();
+                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BN), quarter, chunk0, ok);
+                }
                 if (!ok) break;                                               // warps are independent from here on
                 tc_fence_after();
                 const int nrow = p.M - (m0 + quarter * 32);                      // rows of this warp inside the matrix
@@ -309,11 +364,22 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                             for (int e = 0; e < 32; e++) v[32 * q + e] = __uint_as_float(a[q][e]);
                         }
                     }
+                    if (SPLIT) {
+#pragma unroll
+                        for (int q = 0; q < CW / 32; q++) {
+                            float x[32];
+#pragma unroll
+                            for (int e = 0; e < 32; e++) x[e] = v[32 * q + e];
+                            add_parts(x, ch * CW + 32 * q, quarter * 32 + lane);
+#pragma unroll
+                            for (int e = 0; e < 32; e++) v[32 * q + e] = x[e];
+                        }
+                    }
                     if (ch + 2 >= NCH) {                                      // this warp's last chunk is in registers: the MMA warp may reuse it
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) {
-                            if (PAIR && rank != 0) mbar_arrive_cluster(mapa_u32(bar(GBAR_ACC_EMPTY + buf), 0));
+                            if (PAIR && rank != 0) mbar_arrive_cluster(mapa_u32(bar(GBAR_ACC_EMPTY + buf), lead));
                             else mbar_arrive(bar(GBAR_ACC_EMPTY + buf));
                         }
                     }
@@ -381,7 +447,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 int tm, tn;
                 gemm_tile(w, p, tm, tn);
                 const int ksteps = ksteps1 + (p.K2[tn / p.tiles_n_seg] + GB_K - 1) / GB_K;
-                for (int ks = 0; ks < ksteps && good; ++ks, ++ring) {
+                const int ks0 = ksteps * part / S, ks1 = ksteps * (part + 1) / S;
+                for (int ks = ks0; ks < ks1 && good; ++ks, ++ring) {
                     const uint32_t st = ring % G_STAGES;
                     good = mbar_wait(bar(GBAR_FULL + st), (ring / G_STAGES) & 1u, abort_flag);
                     if (!good) break;
@@ -390,18 +457,19 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     const uint64_t adesc = smem_desc_sw128(a_s, 16, 1024), wdesc = smem_desc_sw128(a_s + GB_M * GB_K * 2, 16, 1024);
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
-                        const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
+                        const uint32_t acc = (ks > ks0 || kk > 0) ? 1u : 0u;
                         if (PAIR) mma_ss_pair(tmem_base + (uint32_t)(buf * BN), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
                         else mma_ss(tmem_base + (uint32_t)(buf * BN), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
                     }
-                    if (PAIR) tc_commit_pair(bar(GBAR_EMPTY + st), 3); else tc_commit(bar(GBAR_EMPTY + st));
+                    if (PAIR) tc_commit_pair(bar(GBAR_EMPTY + st), (uint16_t)(3u << lead)); else tc_commit(bar(GBAR_EMPTY + st));
                 }
                 if (good) {
-                    if (PAIR) tc_commit_pair(bar(GBAR_ACC_FULL + buf), 3); else tc_commit(bar(GBAR_ACC_FULL + buf));
+                    if (PAIR) tc_commit_pair(bar(GBAR_ACC_FULL + buf), (uint16_t)(3u << lead)); else tc_commit(bar(GBAR_ACC_FULL + buf));
                 }
             }
         }
         __syncwarp();
+        if (SPLIT) { cluster_arrive(); cluster_wait(); }                  // the barrier of exchange_parts
     } else {
         setmaxnreg_dec<56>();
         // ------------------------------------------------------------------ TMA loads (one lane of every CTA)
@@ -414,7 +482,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 const int seg = tn / p.tiles_n_seg;
                 const int m0 = tm * TILE_M + (int)rank * GB_M, wrow0 = (tn - seg * p.tiles_n_seg) * BN + (int)rank * 128;
                 const int ksteps = ksteps1 + (p.K2[seg] + GB_K - 1) / GB_K;
-                for (int ks = 0; ks < ksteps && good; ++ks, ++ring) {
+                const int ks1 = ksteps * (part + 1) / S;
+                for (int ks = ksteps * part / S; ks < ks1 && good; ++ks, ++ring) {
                     const bool second = ks >= ksteps1;                    // the k steps of the second product follow the first's
                     const CUtensorMap* const tmL = second ? &maps.a2[seg] : &tmA;
                     const CUtensorMap* const tmW = second ? &maps.w2[seg] : &maps.w[seg];
@@ -426,7 +495,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     if (PAIR) {
                         // both CTAs' bytes complete on the issuing CTA's barrier
                         if (rank == 0) mbar_expect_tx(bar(GBAR_FULL + st), 2 * G_STAGE_BYTES);
-                        const uint32_t fb = mapa_u32(bar(GBAR_FULL + st), 0);
+                        const uint32_t fb = mapa_u32(bar(GBAR_FULL + st), lead);
                         tma_load_3d_pair(a_s, tmL, fb, k0, m0, 0);
                         tma_load_3d_pair(a_s + GB_M * GB_K * 2, tmW, fb, k0, wrow0, 0);
                     } else {
@@ -449,9 +518,10 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
             }
         }
         __syncwarp();
+        if (SPLIT) { cluster_arrive(); cluster_wait(); }                  // the barrier of exchange_parts
     }
     tc_fence_before();
-    if (PAIR) { cluster_arrive(); cluster_wait(); } else __syncthreads();
+    if (PAIR || SPLIT) { cluster_arrive(); cluster_wait(); } else __syncthreads();   // split K: nobody leaves while its ring is read
     if (warp == G_EPI_WARPS) {
         if (lane == 0 && *abort_flag) atomicOr(p.status, ST_TIMEOUT);
         tc_fence_after();

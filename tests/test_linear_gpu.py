@@ -319,6 +319,38 @@ def test_lora_second_product_vs_oracle_and_reference_golden(kb, gemm_golden, cas
         assert np.abs(out - g).max() <= tile_err + 2.0 ** -9 * np.abs(g).max(), f"{name}/lora_{ename} vs reference kernel: {np.abs(out - g).max():.3e}"
 
 
+@pytest.mark.parametrize("M,N,K,K2", [(77, 256, 2048, 0), (130, 96, 1088, 0), (200, 384, 1664, 72), (512, 2048, 1600, 0), (513, 1920, 2048, 40),
+                                      (1000, 2048, 4096, 24)],
+                         ids=["four_parts", "narrow_uneven_parts", "four_parts_second_product", "two_parts", "ragged_two_parts", "two_parts_of_pairs"])
+def test_split_k_every_epilogue(kb, M, N, K, K2):
+    """Few tiles and many k steps: the k steps of a tile run on two or four CTAs (two pairs) of a cluster, each of which finishes a
+    share of the rows. Step counts that do not divide, a second product whose steps fall into the last part, ragged rows, a narrow
+    last column tile; sampled rows against the oracle, nothing outside the M x N window, repeat runs bit-identical."""
+    from kiln_b200 import ops
+    x, w = seeded(600 + M, M, K, "f16"), seeded(601, N, K, "f16", 1.0 / np.sqrt(K))
+    lora = {}
+    rows = sample_rows(M, 20)
+    if K2:
+        t, b = seeded(602, M, K2, "f16"), seeded(603, N, K2, "f16", 1.0 / np.sqrt(K2))
+        lora = {"lora": (dev(t, "f16"), dev(b, "f16"))}
+    gate = oracle.randn(604, N)
+    resid = oracle.randn(605, M * N).reshape(M, N)
+    second = {"lora": (t[rows], b)} if K2 else {}
+    for epi in (ops.EPI_F32, ops.EPI_F16, ops.EPI_GELU16) + ((ops.EPI_RESID,) if N % 128 == 0 else ()):
+        g, r = (gate, resid) if epi == ops.EPI_RESID else (None, None)
+        out = _run(kb, x, w, epi, gate=g, resid=r, ldc_pad=8, **lora)
+        assert np.array_equal(out, _run(kb, x, w, epi, gate=g, resid=r, **lora)), "repeat run differs"
+        ref = oracle.linear16(x[rows], w, epi, g, None if r is None else r[rows], **second)
+        _close(out[rows], ref, K + K2, f"{M}x{N}x{K}+{K2} epi {epi}", epi in (1, 2))
+    if N % 128 == 0:
+        nw = oracle.round16(1.0 + 0.05 * oracle.randn(606, 128), 1)
+        plain = _run(kb, x, w, ops.EPI_F32, **lora)
+        out = _run(kb, x, w, ops.EPI_HEADS16, ldc_pad=8, head_w=dev(nw).to(torch.bfloat16), **lora)
+        ref = oracle.rmsnorm(plain[rows], (nw.view(np.uint32) >> 16).astype(np.uint16), N // 128)
+        # the same sums up to fp32 rounding (the two epilogues may take different shapes), then one fp16 rounding
+        assert np.all(np.abs(out[rows] - ref) <= 2.0 ** -10 * np.abs(ref) + 1e-4), f"{M}x{N}x{K}+{K2} heads16"
+
+
 @pytest.mark.parametrize("M,N,K,K2", [(300, 512, 128, 8), (300, 512, 128, 72), (70, 384, 64, 128), (4096, 2048, 2048, 32)],
                          ids=["pair_tiles_rank8", "pair_tiles_partial_k_step", "single_tiles_two_k_steps", "dit_size_rank32"])
 def test_second_product_shapes(kb, M, N, K, K2):
