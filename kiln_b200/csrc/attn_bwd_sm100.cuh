@@ -111,7 +111,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    constexpr uint32_t tmem_base = 0;                             // all 512 columns are this thread block's (see elect_one)
     pdl_wait();
 
     if (warp < 8) {
@@ -247,7 +247,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         }
     } else {
         setmaxnreg_dec<BWD_OTHER_REGS>();
-        if (warp == 8 && lane == 0) {
+        if (warp == 8 && elect_one()) {
             // ------------------------------------------------------------------ MMA issue
             constexpr uint32_t IDESC_T = idesc_f16(0, 0, 0, 0, BM, BN);   // T = R X^T, both operands K-major (rows of 128 head channels)
             constexpr uint32_t IDESC_A = idesc_f16(0, 0, 0, 1, BM, HD);   // acc += (fp16 in TMEM) X, X MN-major (rows = contraction index)
@@ -311,7 +311,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                 }
             }
             if (good) tc_commit(bar(BB_ACC));
-        } else if (warp == 9 && lane == 0) {
+        } else if (warp == 9 && elect_one()) {
             // ------------------------------------------------------------------ TMA loads
             auto load_tile = [&](uint32_t dst, const CUtensorMap* tm, uint32_t mbar, int row0) {
                 tma_load_3d(dst, tm, mbar, h * HD, row0, b);

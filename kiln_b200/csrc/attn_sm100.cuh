@@ -415,7 +415,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    constexpr uint32_t tmem_base = 0;                             // all 512 columns are this CTA's (see elect_one)
     pdl_wait();                                                   // nothing in global memory is touched before this
     if (RAW_Q && p.q_raw && warp < 8) {                                    // (read by the softmax warps only)
         if (tid < HD) f_qw[tid] = p.qn_w ? __bfloat162float(p.qn_w[tid]) : 1.f;
@@ -1211,8 +1211,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             // longer than the tensor core's instruction queue lasts: with a single issuer the pipe drained between batches
             // and paid its start-up latency every time (measured: ~850 cycles per batch against 520 back to back).
             // Now one thread's bookkeeping runs under the other's MMAs.
-            const int i = (warp - 8) >> 1;
-            if (lane == 0) {
+            const int i = __shfl_sync(0xffffffffu, (warp - 8) >> 1, 0);
+            if (elect_one()) {
                 // Operands are fp16 throughout (bf16/fp32 inputs are staged as fp16 by the pre-pass): with bf16
                 // P the 2^-9 rounding of each weight alone costs ~1e-3 relative error on outputs that are sums
                 // of random-sign terms, and tcgen05 does not take an fp16 A with a bf16 B.
@@ -1331,7 +1331,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             __syncwarp();
         } else if (warp == 9) {
             // ------------------------------------------------------------------ TMA loads (one lane)
-            if (lane == 0) {
+            if (elect_one()) {
                 uint32_t n = 0;
                 uint32_t qe_cnt[2] = {0, 0};
                 uint32_t q_loads[2] = {0, 0};                             // Q tiles requested so far, per stream

@@ -180,7 +180,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     tc_fence_before();
     if (PAIR) { cluster_arrive(); cluster_wait(); } else __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = PAIR ? 0u : *tmem_slot;                    // PAIR: all 512 columns are this CTA's (see elect_one)
     pdl_wait();
 
     if (warp < G_EPI_WARPS) {
@@ -432,7 +432,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     } else if (warp == G_EPI_WARPS) {
         setmaxnreg_dec<56>();
         // ------------------------------------------------------------------ MMA issue (one lane of the group's first CTA)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t IDESC = idesc_f16(0, 0, 0, 0, TILE_M, BN);
             uint32_t ring = 0, use[2] = {0, 0};
             bool good = true;
@@ -473,7 +473,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     } else {
         setmaxnreg_dec<56>();
         // ------------------------------------------------------------------ TMA loads (one lane of every CTA)
-        if (warp == G_EPI_WARPS + 1 && lane == 0) {
+        if (warp == G_EPI_WARPS + 1 && elect_one()) {
             uint32_t ring = 0;
             bool good = true;
             for (int w = group; w < n_tiles && good; w += n_groups) {
