@@ -31,7 +31,8 @@ extern "C" {
  * The tensor-core operands are always fp16 with fp32 accumulation, as in the reference kernel, which
  * converts its fp32 inputs to fp16 while staging (engine/src/tcflash.cuh:56-64): KB_F16 inputs that need
  * neither norm nor RoPE are read in place; KB_BF16 / KB_F32 inputs, and any tensor that gets RMSNorm or
- * RoPE, are staged once as fp16 in the caller's workspace by a fused pre-pass. KB_F32 inputs are what the
+ * RoPE, are staged once as fp16 in the caller's workspace by a fused pre-pass - except a 16-bit Q without
+ * RoPE, which the attention kernel normalises and converts itself. KB_F32 inputs are what the
  * engine holds today (engine/src/dit.cu:429-430). */
 enum { KB_F16 = 0, KB_BF16 = 1, KB_F32 = 2 };
 
@@ -254,8 +255,8 @@ int kb_linear16_qkv_lora(void* const* C3, int ldc, const void* A, int lda, const
  * materialises the [heads, Tq, Tk] probabilities and their gradients in the arena: here they are recomputed tile by tile on
  * the tensor cores (fp16 operands, fp32 accumulation; the engine's is fp32 throughout), nothing of size Tq x Tk is stored,
  * and every output element is written once in a fixed order (bit-identical from run to run). Launches: staging pre-pass
- * (unless dtype is KB_F16), the forward kernel (for the per-row softmax statistics and O), a reduction for
- * sum_d dout * O, and one launch whose thread blocks form dK/dV (one per key block) or dQ (one per query block). The workspace (kb_attn_bwd_workspace_bytes) is always required. */
+ * (unless dtype is KB_F16), the forward kernel (for the per-row softmax statistics and sum_d dout * O; O itself is not stored),
+ * and one launch whose thread blocks form dK/dV (one per key block) or dQ (one per query block). The workspace (kb_attn_bwd_workspace_bytes) is always required. */
 size_t kb_attn_bwd_workspace_bytes(int B, int Tq, int Tk, int H, int dtype);
 int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, const void* v, const void* dout, int B, int Tq, int Tk,
                 int npad, int H, int ld_q, int ld_k, int ld_v, int ld_do, int ld_dq, int ld_dk, int ld_dv, int dtype, void* workspace,

@@ -532,7 +532,7 @@ static int nag_impl(void* out, const void* q, const void* qn_w, const void* k_po
         nag_part = static_cast<float*>(sg.take_bytes((size_t)n_qt * H * NAG_NORM_FLOATS * sizeof(float)));
         nag_flag = static_cast<unsigned int*>(sg.take_bytes((size_t)n_qt * sizeof(unsigned int)));
         if (sg.overflow) return KB_ERR_WORKSPACE;
-        pb.zero(nag_flag, n_qt);                       // cleared by the pre-pass, or by a memset when nothing is staged
+        pb.zero(nag_flag, n_qt);                       // cleared by the pre-pass, or by a small kernel when nothing is staged
     } else {
         if ((conv || qn_w) && (!workspace || !aligned16(workspace))) return KB_ERR_WORKSPACE;
         nag_part = peers->part_peers[peers->self];     // the exchange lives in the peer-visible buffers; their counters only grow

@@ -27,9 +27,10 @@
 // the stats array (padded to whole query blocks) always holds.
 //
 // TMEM (512 columns): T0 [0,128) S or S^T, T1 [128,256) dP or dP^T, acc0 [256,384), acc1 [384,512). Measured on B200 (clock
-// stamps in a private build): the kernel is bound by the thread that issues the products - an SS product costs ~650 cycles
-// per 128x128x128 however its N is cut (the A operand is re-read from shared memory for every instruction), the softmax
-// warps need ~1100 per step. So the products keep N = 128 and the step is software-pipelined across the two products instead:
+// stamps in a private build, before the issuing thread was an elected one): the kernel is bound by the thread that issues the
+// products - a step of BWD_DKV took 3300 cycles, of which its four products took 3030 (~95 per instruction against 64 in the tensor
+// pipe; an SS product costs the same with half the N, and taking its A operand from TMEM changed nothing), the softmax warps ~2000
+// (phase 1 1400, phase 2 600). So the products keep N = 128 and the step is software-pipelined across the two products instead:
 //   softmax phase 1: S^T ready -> P^T = 2^(c S^T - L) (kept in registers), fp16 P^T stored, "P0" signalled;
 //   softmax phase 2: dP^T ready -> dS^T = P^T (dP^T - D) stored, "P1" signalled;
 //   issue order:     [P0] dV += P^T dO | S^T of the next step | [P1] dK += dS^T Q | dP^T of the next step
