@@ -126,8 +126,8 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         float Lr = 0.f, Dr = 0.f;                                   // BWD_DQ: this row's statistics
         if (MODE == BWD_DQ) {
             const float* st = p.stats + (((size_t)b * p.H + h) * nqb + blk) * 256;
-            Lr = __ldg(st + r);
-            Dr = __ldg(st + 128 + r);
+            Lr = __ldcg(st + r);
+            Dr = __ldcg(st + 128 + r);
         }
         bool ok = true;
         for (int it = 0; it < n_it; ++it) {

@@ -217,8 +217,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 if (head_w && seg != w_seg) {                             // L1 hits after the first tile of a segment
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        w0[q] = __ldg(reinterpret_cast<const uint4*>(head_w + hs * 32) + q);
-                        w1[q] = __ldg(reinterpret_cast<const uint4*>(head_w + 64 + hs * 32) + q);
+                        w0[q] = reinterpret_cast<const uint4*>(head_w + hs * 32)[q];
+                        w1[q] = reinterpret_cast<const uint4*>(head_w + 64 + hs * 32)[q];
                     }
                     w_seg = seg;
                 }
@@ -227,8 +227,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     int tr = min(row0, p.M - 1) % p.rope_T;
 #pragma unroll
                     for (int rr = 0; rr < 32; rr++) {
-                        cr[rr] = __ldg(p.rope_cos + (size_t)tr * 64 + hs * 32 + lane);
-                        sr[rr] = __ldg(p.rope_sin + (size_t)tr * 64 + hs * 32 + lane);
+                        cr[rr] = p.rope_cos[(size_t)tr * 64 + hs * 32 + lane];
+                        sr[rr] = p.rope_sin[(size_t)tr * 64 + hs * 32 + lane];
                         if (row0 + rr + 1 < p.M) tr = (tr + 1 == p.rope_T) ? 0 : tr + 1;
                     }
                 }
@@ -391,7 +391,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                         if (p.gate) {
 #pragma unroll
                             for (int c = 0; c < CW; c += 4) {
-                                const float4 gt = __ldg(reinterpret_cast<const float4*>(p.gate + n0 + ch * CW + c));
+                                const float4 gt = *reinterpret_cast<const float4*>(p.gate + n0 + ch * CW + c);
                                 v[c] *= gt.x; v[c + 1] *= gt.y; v[c + 2] *= gt.z; v[c + 3] *= gt.w;
                             }
                         }
