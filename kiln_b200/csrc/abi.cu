@@ -15,6 +15,7 @@
 #include "selfcheck.cuh"
 #include "gemm_sm100.cuh"
 #include "attn_bwd_sm100.cuh"
+#include "routes.h"
 
 namespace {
 
@@ -285,9 +286,6 @@ struct PeerSpec {
     int n_peers, col0;
 };
 
-#ifndef KB_SPLIT_MARGIN
-#define KB_SPLIT_MARGIN 7
-#endif
 constexpr int MAX_HEADS = 4096;   // keeps every byte count below in range
 constexpr size_t NAG_NORM_FLOATS = 512;   // per (query tile, head): [2 column halves][|Z+|_1, |g|_1][128 rows]
 
@@ -301,27 +299,6 @@ size_t staging_bytes(size_t rows_q, size_t rows_k, int n_ctx, int H, int dtype, 
     return n;
 }
 
-// Balanced (item, key block) ranges per SM against whole items per SM, in key-block steps on the slowest SM. Measured on B200
-// (4096 / 3456 / 2560 / 2048 / 1536 / 1024 tokens x 16 heads, device time inside a CUDA graph): a key-block step costs ~1.86 us
-// and the balanced schedule a fixed ~15 us on top (one more segment to fill and drain per SM, the partial results written and
-// merged; the cooperative launch itself measured free): it wins at 2560 and 3456 tokens (63.8 vs 83.5 us, 97.6 vs 111.7 us), ties
-// or wins at 4096 (128.2 vs 127.4 us on one GPU, 126.9 vs 140.0 us on another), ties at 2048 and loses at 1536 and 1024 (36.8 vs
-// 29.3 us, 28.7 vs 21.3 us). So it is taken when it saves at least eight steps.
-bool split_pays(int n_items, int nb, int sm_count) {
-    const long long steps = (long long)n_items * nb;
-    if (nb < 2 || steps < 2LL * sm_count) return false;
-    const long long whole = (long long)((n_items + sm_count - 1) / sm_count) * nb;
-    const long long balanced = (steps + sm_count - 1) / sm_count + KB_SPLIT_MARGIN;
-    return balanced < whole;
-}
-
-// One 128-row query tile per item with its keys split over both streams (MODE_KEYS), against 256 rows and all keys: taken while every
-// item has an SM to itself, where it halves the steps of the longest item. It reads every K/V tile twice as often (128 KB per step
-// and SM), so that a step takes 2.2 us against 1.85, and in more than one round the balanced or the whole-item schedule is as fast or
-// faster. Measured on B200, 16 heads, fp16, device time, whole items -> this: 256 tokens 9.4 -> 6.9 us, 512 12.9 -> 9.4, 1000
-// 20.7 -> 14.9, 1152 22.5 -> 15.6; beyond one round 1280 25.1 -> 28.4, 2048 35.3 -> 42.0, 3456 90.0 (balanced) -> 91.4.
-bool keys_pay(int items_keys, int nb, int sm_count) { return nb >= 2 && items_keys <= sm_count; }
-
 // A 16-bit Q that needs no rotation is normalised and converted by the attention kernel itself, in shared memory, and the pre-pass
 // leaves it out: it would read and write all of Q (T x 2048 x 2 bytes each way) and, for fp16 activations with K and V in fp16, it
 // would be a launch for nothing else. Measured on B200, 16 heads: cross 1536 x 26 fp16 15.2 -> 13.2 us back to back (device time
@@ -333,6 +310,8 @@ void set_raw_q(AttnParams& p, int dtype, const void* qn_w, float eps) {
     p.qn_w = static_cast<const __nv_bfloat16*>(qn_w);
     p.eps = eps;
 }
+
+static_assert(BM == ROUTE_TILE && BN == ROUTE_TILE, "the schedule rules count in these tiles");
 
 // what the backward pass wants from the forward one instead of O (AttnParams::stats)
 struct GradSpec {
@@ -393,20 +372,18 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     p.status = st->status;
     if (q_in_kernel) set_raw_q(p, dtype, qn_w, eps);
     if (grad) { p.stats = grad->stats; p.dout = grad->dout; p.ld_do = grad->ld_do; }
-    // Balanced schedule: worth it when equal (item, key block) ranges per SM beat whole items per SM by more than the
-    // cost of writing and merging the cut items' partial results (about two key blocks), and the workspace has room for
-    // those partial results; otherwise every CTA takes whole items.
-    const int nb = (Tk + BN - 1) / BN, items_keys = ((Tq + BM - 1) / BM) * H * B;
-    const bool keys = !peers && keys_pay(items_keys, nb, st->sm_count);
-    if (!keys && split_pays(p.n_items, nb, st->sm_count) && workspace && aligned16(workspace)) {
-        Stage trial = sg;
-        float* part = static_cast<float*>(trial.take_bytes((size_t)st->sm_count * PART_CTA_BYTES));
-        unsigned int* flags = static_cast<unsigned int*>(trial.take_bytes((size_t)st->sm_count * 2 * sizeof(unsigned int)));   // one per SM and stream
-        if (!trial.overflow) {
-            sg = trial;
-            p.split = 1; p.part = part; p.part_flag = flags;
-            pb.zero(flags, st->sm_count * 2);
-        }
+    // The balanced schedule needs room in the workspace for the partial results of cut items
+    Stage trial = sg;
+    float* part = nullptr;
+    unsigned int* flags = nullptr;
+    if (workspace && aligned16(workspace)) {
+        part = static_cast<float*>(trial.take_bytes((size_t)st->sm_count * PART_CTA_BYTES));
+        flags = static_cast<unsigned int*>(trial.take_bytes((size_t)st->sm_count * 2 * sizeof(unsigned int)));   // one per SM and stream
+    }
+    const Route route = attn_route(B, Tq, Tk, H, st->sm_count, !peers, flags != nullptr);
+    if (route == ROUTE_BALANCED) {
+        p.split = 1; p.part = part; p.part_flag = flags;
+        pb.zero(flags, st->sm_count * 2);
     }
     if ((rc = launch_prep(st, pb, dtype, KB_F16, stream))) return rc;
     CUtensorMap tq, tk, tv;
@@ -418,8 +395,8 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
         for (int i = 0; i < peers->n_peers; i++) { p.out_peers[i] = peers->out_peers[i]; p.ctr_peers[i] = peers->ctr_peers[i]; }
     }
     ProfScope ps(st, KB_PROF_ATTENTION, stream);
-    if (keys) {
-        p.n_items = items_keys;
+    if (route == ROUTE_KEYS) {
+        p.n_items = ((Tq + BM - 1) / BM) * H * B;
         return launch_attn<MODE_KEYS>(out_dtype, tq, tk, tv, tk, tv, p, st->sm_count, stream);
     }
     return launch_attn<MODE_PAIR>(out_dtype, tq, tk, tv, tk, tv, p, st->sm_count, stream);

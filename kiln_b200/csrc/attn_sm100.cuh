@@ -21,7 +21,7 @@
 //
 //   MODE_KEYS : one 128-row query tile of one (batch, head); stream 0 runs the even 128-key blocks of its K/V sequence, stream 1
 //               the odd ones, and the epilogue merges the two (m, l, O). Twice the items of MODE_PAIR at half the length: for
-//               few query tiles (keys_cost in abi.cu has the rule and what both sides measured).
+//               few query tiles (attn_route in routes.h has the rule and what both sides measured).
 //
 // Warp roles (384 threads): warps 0-3 / 4-7: softmax of stream 0 / 1 (warp w owns TMEM lanes 32*(w%4)..+31,
 // one query row per thread), warps 8 / 10 issue the MMAs of stream 0 / 1 (one lane each), warp 9 issues TMA loads

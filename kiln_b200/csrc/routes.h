@@ -1,0 +1,53 @@
+// Which schedule an attention call takes: rules on sizes only, plain host code (no CUDA headers), so that they can be tested without
+// a device.
+#pragma once
+
+namespace kb {
+
+#ifndef KB_SPLIT_MARGIN
+#define KB_SPLIT_MARGIN 7
+#endif
+constexpr int ROUTE_TILE = 128;   // query rows per tile, keys per block
+
+// Balanced (item, key block) ranges per SM against whole items per SM, in key-block steps on the slowest SM. Measured on B200
+// (4096 / 3456 / 2560 / 2048 / 1536 / 1024 tokens x 16 heads, device time inside a CUDA graph): a key-block step costs ~1.86 us
+// and the balanced schedule a fixed ~15 us on top (one more segment to fill and drain per SM, the partial results written and
+// merged; the cooperative launch itself measured free): it wins at 2560 and 3456 tokens (63.8 vs 83.5 us, 97.6 vs 111.7 us), ties
+// or wins at 4096 (128.2 vs 127.4 us on one GPU, 126.9 vs 140.0 us on another), ties at 2048 and loses at 1536 and 1024 (36.8 vs
+// 29.3 us, 28.7 vs 21.3 us). So it is taken when it saves at least eight steps.
+inline bool split_pays(int n_items, int nb, int sm_count) {
+    const long long steps = (long long)n_items * nb;
+    if (nb < 2 || steps < 2LL * sm_count) return false;
+    const long long whole = (long long)((n_items + sm_count - 1) / sm_count) * nb;
+    const long long balanced = (steps + sm_count - 1) / sm_count + KB_SPLIT_MARGIN;
+    return balanced < whole;
+}
+
+enum Route { ROUTE_WHOLE, ROUTE_BALANCED, ROUTE_KEYS };
+
+// One 128-row query tile per item with its keys split over both streams (MODE_KEYS), against 256 rows and all keys (MODE_PAIR): a
+// candidate while every item has an SM to itself, where it halves the steps of the longest item. It reads every K/V tile twice as
+// often (128 KB per step and SM), and in more than one round the balanced or the whole-item schedule is as fast or faster. Measured
+// on B200, 16 heads, fp16, device time, whole items -> this: 256 tokens 9.4 -> 6.9 us, 512 12.9 -> 9.4, 1000 20.7 -> 14.9,
+// 1152 22.5 -> 15.6; beyond one round 1280 25.1 -> 28.4, 2048 35.3 -> 42.0, 3456 90.0 (balanced) -> 91.4.
+//
+// With few tiles and many keys the balanced schedule spreads the keys of an item over more SMs than one, at the price of merging
+// sm_count / n_items parts. Both in units of 10 ns, fitted to 40 shapes: keys 5.5 us + 1.95 us per step of two blocks; balanced
+// 13.5 us (9 with a single query tile, which has one stream) + 1.9 us per block step + 1.8 us per part. Measured, queries x keys x
+// heads, balanced / keys: 128 x 16384 x 16 52 / 127 us, 256 x 16384 x 4 88 / 126, 512 x 8192 x 16 51 / 68, 4096 x 4096 x 2
+// 35.3 / 36.9; the other way 256 x 4096 x 16 37.6 / 36.0, 1024 x 8192 x 16 73 / 71, 4096 x 4096 x 4 46 / 39, 1024 x 1024 x 16 25 / 15.
+//
+// room: the workspace holds the balanced schedule's partial results; may_keys: the call has a MODE_KEYS form (no peers).
+inline Route attn_route(int B, int Tq, int Tk, int H, int sm_count, bool may_keys, bool room) {
+    const int nb = (Tk + ROUTE_TILE - 1) / ROUTE_TILE;
+    const int n_items = ((Tq + 2 * ROUTE_TILE - 1) / (2 * ROUTE_TILE)) * H * B, items_keys = ((Tq + ROUTE_TILE - 1) / ROUTE_TILE) * H * B;
+    const bool balanced = room && split_pays(n_items, nb, sm_count);
+    if (may_keys && nb >= 2 && items_keys <= sm_count) {
+        const long long keys_cost = 550 + 195LL * ((nb + 1) / 2);
+        const long long balanced_cost = (Tq > ROUTE_TILE ? 1350 : 900) + 190LL * (((long long)n_items * nb + sm_count - 1) / sm_count) + 180LL * sm_count / n_items;
+        return balanced && balanced_cost < keys_cost ? ROUTE_BALANCED : ROUTE_KEYS;
+    }
+    return balanced ? ROUTE_BALANCED : ROUTE_WHOLE;
+}
+
+}  // namespace kb

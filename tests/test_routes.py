@@ -1,0 +1,47 @@
+"""CPU test of the rule that picks an attention call's schedule (kiln_b200/csrc/routes.h, plain C++)."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "kiln_b200", "csrc")
+WHOLE, BALANCED, KEYS = 0, 1, 2
+SMS = 148
+
+# Device time (us) of one call on a B200, fp16 operands in place, inside a CUDA graph: whole items, balanced schedule, keys split
+# over both streams (None: the schedule does not exist there)
+MEASURED = [  # B, Tq, Tk, H, whole, balanced, keys
+    (1, 128, 4096, 16, 48.4, 33.9, 35.4), (1, 256, 4096, 16, 61.3, 37.6, 36.0), (1, 128, 8192, 16, 91.3, 39.9, 66.0), (1, 256, 16384, 4, 226.6, 87.8, 125.7),
+    (1, 128, 16384, 16, 176.6, 52.2, 126.9), (1, 4096, 4096, 2, 61.5, 35.3, 36.9), (1, 4096, 4096, 4, 63.3, 46.4, 39.0), (1, 2000, 2000, 3, 34.0, 30.2, 20.9),
+    (2, 2000, 2000, 2, 34.2, 29.3, 21.4), (1, 2048, 2048, 8, 35.1, 31.1, 23.0), (1, 1024, 1024, 16, 20.5, 25.1, 14.6), (1, 1152, 1152, 16, 22.9, 26.2, 15.6),
+    (1, 1024, 4096, 16, 63.0, 46.6, 39.1), (1, 1024, 8192, 16, 119.3, 73.0, 70.7), (1, 512, 2048, 16, 34.1, 29.1, 21.4), (1, 512, 4096, 16, 61.6, 35.3, 36.9),
+    (1, 512, 8192, 16, 117.9, 51.3, 67.5), (1, 2048, 4096, 2, 61.3, 37.3, 35.9), (1, 4096, 512, 4, 13.4, None, 10.2), (1, 256, 2048, 16, 33.6, None, 20.7),
+    (1, 128, 3000, 32, 38.1, 27.5, 28.2), (1, 2304, 4096, 8, 62.6, 47.8, 39.1), (1, 1500, 1500, 12, 28.0, 28.5, 18.9), (1, 1, 8192, 32, 91.2, 45.6, 66.5),
+    (1, 128, 4096, 148, 57.3, 58.3, 52.9), (1, 1280, 1280, 16, 25.8, 29.0, 28.7), (1, 2048, 2048, 16, 36.9, 43.8, 42.7), (1, 2560, 2560, 16, 81.3, 58.1, 71.8),
+    (1, 1280, 4096, 16, 66.5, 50.5, 71.4), (1, 1408, 8192, 16, 124.0, 94.1, 133.2)]
+
+
+@pytest.fixture(scope="module")
+def route(tmp_path_factory):
+    d = tmp_path_factory.mktemp("routes")
+    src = d / "routes.cpp"
+    src.write_text('#include "routes.h"\n'
+                   'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
+    return ctypes.CDLL(str(d / "routes.so")).route
+
+
+@pytest.mark.parametrize("case", MEASURED, ids=[f"{b}x{q}x{k}x{h}" for b, q, k, h, *_ in MEASURED])
+def test_the_schedule_taken_is_the_fastest_measured_one(route, case):
+    """Within 3 %, what one side differs by from run to run."""
+    B, Tq, Tk, H, *us = case
+    taken = route(B, Tq, Tk, H, SMS, 1, 1)
+    assert us[taken] is not None and us[taken] <= 1.03 * min(t for t in us if t is not None)
+
+
+def test_restrictions(route):
+    assert route(1, 128, 16384, 16, SMS, 1, 0) == KEYS and route(1, 2560, 2560, 16, SMS, 1, 0) == WHOLE      # no room for partial results
+    assert route(1, 1024, 1024, 16, SMS, 0, 1) == WHOLE and route(1, 4096, 4096, 2, SMS, 0, 1) == BALANCED   # a call with peers
+    for Tq in (1, 128, 129, 4096):
+        assert route(1, Tq, 128, 1, SMS, 1, 1) == WHOLE                                                      # one key block: one stream has none
