@@ -58,6 +58,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <float.h>
 #include <math.h>
 
 #include <type_traits>
@@ -616,7 +617,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         for (int e = 0; e < 32; e++)
                             if (q * 32 + e >= valid) s[q][e] = 0xff800000u;
                 }
-                float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+                // From the lowest finite value up: a block whose keys all score -inf then has weights 0 and not NaN, also as the first
+                // block of a stream (in MODE_KEYS that of stream 1 is the second of the sequence) or of a part of a cut item.
+                float mx0 = -FLT_MAX, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
                 for (int e = 0; e < 32; e += 2) {                  // 3-input max: two scores per instruction
                     mx0 = max3(mx0, __uint_as_float(s[0][e]), __uint_as_float(s[0][e + 1]));

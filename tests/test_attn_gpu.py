@@ -9,7 +9,7 @@ import torch
 
 import oracle
 from golden_inputs import gen
-from util_gpu import DT, assert_close, assert_close_bf16_storage, dev, sample_rows, seeded
+from util_gpu import DT, TOL_MAX_ABS, TOL_MEAN_REL, assert_close, assert_close_bf16_storage, dev, sample_rows, seeded
 
 pytestmark = pytest.mark.gpu
 
@@ -171,6 +171,23 @@ def test_self_large_scores_rescale_path(kb):
     k = oracle.round16(k, 0)
     v = seeded(3, T, H * 128, kind)
     assert_close(_self(kb, q, k, v, 1, T, H, kind, "f32"), oracle.attention(q, k, v, H), "rescale path")
+
+
+@pytest.mark.parametrize("Tq,Tk,H,npad,masked", [(300, 640, 2, 0, [(128, 256)]), (300, 640, 2, 0, [(0, 128), (512, 640)]), (300, 300, 2, 212, [(128, 300)]),
+                                                 (1500, 400, 16, 0, [(0, 128)]), (128, 8192, 16, 0, [(0, 256), (2048, 4096)]), (200, 128, 1, 384, [(0, 128)])],
+                         ids=["second_block", "first_and_last_block", "all_but_the_first_block", "first_block_whole_items", "parts_of_cut_items", "all_with_padding"])
+def test_blocks_of_keys_that_score_minus_infinity(kb, Tq, Tk, H, npad, masked):
+    """Keys masked by an infinite channel: their weight is 0, whichever stream or part of the keys they are all there is of."""
+    q, k, v = seeded(51, Tq, H * 128, "f16"), seeded(52, Tk, H * 128, "f16"), seeded(53, Tk, H * 128, "f16")
+    q[:, ::128] = 1
+    for lo, hi in masked:
+        k[lo:hi, ::128] = -np.inf
+    out = _cross(kb, q, k, v, Tq, Tk, npad, H, "f16", "f32")
+    keep = np.isfinite(k[:, 0])
+    rows = sample_rows(Tq, 24)
+    ref = oracle.attention(q[rows], k[keep], v[keep], H, npad) if keep.any() else np.zeros((len(rows), H * 128), np.float32)
+    d = np.abs(out[rows] - ref)
+    assert d.max() <= TOL_MAX_ABS and d.sum() <= TOL_MEAN_REL * np.abs(ref).sum(), f"max_abs {d.max():.3e}"
 
 
 # ---------------------------------------------------------------- fused Q/K RMSNorm + RoPE
