@@ -302,9 +302,19 @@ size_t staging_bytes(size_t rows_q, size_t rows_k, int n_ctx, int H, int dtype, 
 // A 16-bit Q that needs no rotation is normalised and converted by the attention kernel itself, in shared memory, and the pre-pass
 // leaves it out: it would read and write all of Q (T x 2048 x 2 bytes each way) and, for fp16 activations with K and V in fp16, it
 // would be a launch for nothing else. Measured on B200, 16 heads: cross 1536 x 26 fp16 15.2 -> 13.2 us back to back (device time
-// 13.7 -> 10.5), NAG 1536 x (378, 168) fp16 34.9 -> 33.1, NAG 4096 x (512, 512) bf16 75.5 -> 71.7. (With RoPE a thread would read 512 bytes of tables per row, one line per lane: slower than the
-// pre-pass. An fp32 tile does not fit into the 32 KB of a Q tile.)
-bool prepares_q(int dtype, const float* rope_cos) { return dtype != KB_F32 && !rope_cos; }
+// 13.7 -> 10.5), NAG 1536 x (378, 168) fp16 34.9 -> 33.1, NAG 4096 x (512, 512) bf16 75.5 -> 71.7. (With RoPE a thread would read
+// 512 bytes of tables per row, one line per lane: slower than the pre-pass. An fp32 tile does not fit into the 32 KB of a Q tile.)
+// Q is then read while earlier items already store their output, so an output that lies across Q's memory has Q staged as before.
+bool prepares_q(const void* q, size_t rows, int H, int ld_q, int dtype, const float* rope_cos, const void* const* outs, int n_outs, int col0, int ld_o,
+                int out_dtype) {
+    if (dtype == KB_F32 || rope_cos) return false;
+    const size_t eo = out_dtype == KB_F32 ? 4 : 2;
+    for (int i = 0; i < n_outs; i++)
+        if (!q_survives_output({q, rows, (size_t)ld_q * 2, (size_t)H * 256},
+                               {static_cast<const char*>(outs[i]) + (size_t)col0 * eo, rows, (size_t)ld_o * eo, (size_t)H * 128 * eo}))
+            return false;
+    return true;
+}
 void set_raw_q(AttnParams& p, int dtype, const void* qn_w, float eps) {
     p.q_raw = dtype == KB_BF16 ? 2 : 1;
     p.qn_w = static_cast<const __nv_bfloat16*>(qn_w);
@@ -355,8 +365,9 @@ int attn_pair(void* out, const void* q, const void* k, const void* v, const void
     pb.pp.H = H; pb.pp.eps = eps;
     const void *qq = q, *kk = k, *vv = v;
     int ldq = ld_q, ldk = ld_k, ldv = ld_v;
-    // The space for a staged Q is part of the workspace that a call asks for, used or not.
-    const bool q_in_kernel = stage_q && prepares_q(dtype, rope_cos);
+    // The space for a staged Q is part of the workspace that a call asks for, whether this call's output lets Q stay where it is or not.
+    const bool q_in_kernel = stage_q && (peers ? prepares_q(q, (size_t)B * Tq, H, ld_q, dtype, rope_cos, peers->out_peers, peers->n_peers, peers->col0, ld_o, out_dtype)
+                                               : prepares_q(q, (size_t)B * Tq, H, ld_q, dtype, rope_cos, &out, 1, 0, ld_o, out_dtype));
     if (stage_q) {
         void* d = sg.take((size_t)B * Tq, H);
         if (!q_in_kernel) { if (d) pb.add(d, H * 128, q, ld_q, B * Tq, Tq, qn_w, rope_cos, rope_sin); qq = d; ldq = H * 128; }
@@ -519,7 +530,8 @@ static int nag_impl(void* out, const void* q, const void* qn_w, const void* k_po
     const void* kv[4] = {k_pos, v_pos, k_neg, v_neg};
     const int kv_rows[4] = {Tk_pos, Tk_pos, Tk_neg, Tk_neg};
     int ldq = ld_q, ldkv = ld_kv;
-    const bool q_in_kernel = (conv || qn_w) && prepares_q(dtype, nullptr);
+    const bool q_in_kernel = (conv || qn_w) && (peers ? prepares_q(q, (size_t)Tq, H, ld_q, dtype, nullptr, peers->out_peers, peers->n_peers, peers->col0, ld_o, out_dtype)
+                                                      : prepares_q(q, (size_t)Tq, H, ld_q, dtype, nullptr, &out, 1, 0, ld_o, out_dtype));
     if (conv || qn_w) {
         void* d = sg.take((size_t)Tq, H);
         if (!q_in_kernel) { if (d) pb.add(d, H * 128, q, ld_q, Tq, Tq, qn_w, nullptr, nullptr); qq = d; ldq = H * 128; }

@@ -1,6 +1,8 @@
 // Which schedule an attention call takes: rules on sizes only, plain host code (no CUDA headers), so that they can be tested without
 // a device.
 #pragma once
+#include <stddef.h>
+#include <stdint.h>
 
 namespace kb {
 
@@ -48,6 +50,27 @@ inline Route attn_route(int B, int Tq, int Tk, int H, int sm_count, bool may_key
         return balanced && balanced_cost < keys_cost ? ROUTE_BALANCED : ROUTE_KEYS;
     }
     return balanced ? ROUTE_BALANCED : ROUTE_WHOLE;
+}
+
+// A row-major matrix in memory, in bytes
+struct MatBytes {
+    const void* p;
+    size_t rows, stride, width;
+};
+// Do two matrices share a byte? Exact for equal row strides (column slices of one buffer do not); for different ones, whether
+// their address ranges meet.
+inline bool share_bytes(const MatBytes& x, const MatBytes& y) {
+    const MatBytes &lo = (uintptr_t)x.p <= (uintptr_t)y.p ? x : y, &hi = (uintptr_t)x.p <= (uintptr_t)y.p ? y : x;
+    const size_t d = (uintptr_t)hi.p - (uintptr_t)lo.p;
+    if (d >= (lo.rows - 1) * lo.stride + lo.width) return false;
+    if (lo.stride != hi.stride) return true;
+    const size_t off = d % lo.stride;
+    return off < lo.width || off + hi.width > lo.stride;
+}
+// May an item read its raw Q tile while other items store their output? Yes if no output byte is a byte of Q, or if every (row,
+// head) of the output lies exactly on its own Q, which only the item itself reads.
+inline bool q_survives_output(const MatBytes& q, const MatBytes& out) {
+    return !share_bytes(q, out) || (q.p == out.p && q.stride == out.stride && q.width == out.width);
 }
 
 }  // namespace kb

@@ -236,6 +236,34 @@ def test_16_bit_q_prepared_in_the_kernel(kb, Tq, Tk, norm, kind):
     assert_close(out.cpu().numpy()[rows], oracle.attention(qr, k, v, H, 512 - Tk), f"{Tq}x{Tk} {kind} norm {norm}")
 
 
+@pytest.mark.parametrize("nag", [False, True])
+@pytest.mark.parametrize("layout", ["fp32_over_q", "in_place"])
+def test_output_in_the_memory_of_a_normalised_q(kb, nag, layout):
+    """More items than SMs, so that the last ones read their Q after the first have stored: an fp32 output whose row r starts where
+    row r of the fp16 Q does (a head of it covers two heads of Q), and an fp16 output exactly in place of Q."""
+    T, Tk, H = 4096, 40, 16
+    D = H * 128
+    q, k, v, kn, vn = (seeded(s, n, D, "f16") for s, n in ((61, T), (62, Tk), (63, Tk), (64, Tk), (65, Tk)))
+    wq = oracle.round16(1 + 0.1 * oracle.randn(66, 128), 1)
+    buf = torch.empty(T, D, device="cuda")
+    dq = buf.view(torch.float16)[:, :D]
+    dq.copy_(dev(q, "f16"))
+    out = buf if layout == "fp32_over_q" else dq
+    w = dev(wq).bfloat16()
+    ws = torch.empty(kb.workspace_bytes(T, Tk, H, torch.float16, True, False, n_ctx=2 if nag else 1), dtype=torch.uint8, device="cuda")
+    if nag:
+        kb.attn_nag(out, dq, dev(k, "f16"), dev(v, "f16"), Tk, 512 - Tk, dev(kn, "f16"), dev(vn, "f16"), Tk, 512 - Tk, 5.0, 2.5, 0.25, T, H, qn_w=w, workspace=ws)
+    else:
+        kb.attn_cross(out, dq, dev(k, "f16"), dev(v, "f16"), T, Tk, 512 - Tk, H, qn_w=w, workspace=ws)
+    assert kb.check_status() == 0
+    rows = sample_rows(T, 24)
+    qr = oracle.rmsnorm(q[rows], _bits(wq), H)
+    ref = oracle.attention(qr, k, v, H, 512 - Tk)
+    if nag:
+        ref = oracle.nag(ref, oracle.attention(qr, kn, vn, H, 512 - Tk), 5.0, 2.5, 0.25)
+    assert_close(out.float().cpu().numpy()[rows], ref, f"{layout} nag {nag}")
+
+
 @pytest.mark.parametrize("kind", ["f16", "bf16"])
 def test_q_norm_only_strided_many_items(kb, kind):
     """The cross-attention call pattern on a self-sized problem: Q gets RMSNorm, K arrives normalised; Q/K/V are column

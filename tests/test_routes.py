@@ -23,13 +23,22 @@ MEASURED = [  # B, Tq, Tk, H, whole, balanced, keys
 
 
 @pytest.fixture(scope="module")
-def route(tmp_path_factory):
+def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("routes")
     src = d / "routes.cpp"
     src.write_text('#include "routes.h"\n'
-                   'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n')
+                   'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n'
+                   'extern "C" int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {\n'
+                   '    return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth}); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
-    return ctypes.CDLL(str(d / "routes.so")).route
+    lib = ctypes.CDLL(str(d / "routes.so"))
+    lib.survives.argtypes = [ctypes.c_size_t] * 7
+    return lib
+
+
+@pytest.fixture(scope="module")
+def route(rules):
+    return rules.route
 
 
 @pytest.mark.parametrize("case", MEASURED, ids=[f"{b}x{q}x{k}x{h}" for b, q, k, h, *_ in MEASURED])
@@ -45,3 +54,19 @@ def test_restrictions(route):
     assert route(1, 1024, 1024, 16, SMS, 0, 1) == WHOLE and route(1, 4096, 4096, 2, SMS, 0, 1) == BALANCED   # a call with peers
     for Tq in (1, 128, 129, 4096):
         assert route(1, Tq, 128, 1, SMS, 1, 1) == WHOLE                                                      # one key block: one stream has none
+
+
+def test_raw_q_needs_an_output_that_leaves_it_alone(rules):
+    """Against a count of shared bytes, over all offsets of small matrices with equal and different strides."""
+    rows = 3
+    for stride, width, ostride, owidth in [(16, 4, 16, 4), (16, 8, 16, 8), (16, 6, 16, 12), (16, 16, 16, 16), (16, 4, 32, 8), (24, 8, 16, 8)]:
+        q0 = 200
+        q = {q0 + r * stride + c for r in range(rows) for c in range(width)}
+        for o0 in range(q0 - 120, q0 + 120):
+            o = {o0 + r * ostride + c for r in range(rows) for c in range(owidth)}
+            got = bool(rules.survives(q0, rows, stride, width, o0, ostride, owidth))
+            in_place = (o0, ostride, owidth) == (q0, stride, width)
+            if stride == ostride:
+                assert got == (in_place or not (q & o)), (stride, width, owidth, o0 - q0)
+            else:                                              # different strides: never wrongly allowed, and allowed when the ranges are apart
+                assert not (got and q & o) and (got or not (min(o) > max(q) or min(q) > max(o)))
