@@ -815,7 +815,9 @@ void bwd_qsplit(int B, int Tq, int Tk, int H, int sm_count, int* qsplit, int* q_
 }
 size_t bwd_partial_bytes(int B, int Tk, int H, int qsplit) { return qsplit > 1 ? 2 * align256((size_t)qsplit * B * Tk * H * 128 * sizeof(float)) : 0; }
 size_t bwd_fixed_bytes(int B, int Tq, int Tk, int H, int dtype) {
-    size_t n = bwd_stats_bytes(B, Tq, H);
+    // statistics; room for an fp16 O, which nothing uses since the forward pass leaves D itself: the least workspace that a call
+    // accepts stays what callers know
+    size_t n = bwd_stats_bytes(B, Tq, H) + align256((size_t)B * Tq * H * 128 * 2);
     if (dtype != KB_F16) n += 2 * align256((size_t)B * Tq * H * 128 * 2) + 2 * align256((size_t)B * Tk * H * 128 * 2);   // fp16 Q, dO, K, V
     return n;
 }
@@ -849,6 +851,7 @@ int kb_attn_bwd(void* dq, void* dk, void* dv, const void* q, const void* k, cons
     if ((rc = get_state(&st))) return rc;
     Stage sg{static_cast<char*>(workspace), workspace_bytes};
     float* stats = static_cast<float*>(sg.take_bytes(bwd_stats_bytes(B, Tq, H)));
+    sg.take_bytes((size_t)B * Tq * H * 128 * 2);                  // see bwd_fixed_bytes
     int qsplit, q_per;
     bwd_qsplit(B, Tq, Tk, H, st->sm_count, &qsplit, &q_per);
     float* part_dk = nullptr;

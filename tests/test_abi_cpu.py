@@ -46,18 +46,6 @@ def test_error_strings_and_sizes(built_lib):
     assert kiln_b200.workspace_bytes(1536, 512, 16, F16, n_ctx=2) == 12 * 16 * 2048 + 256
 
 
-def test_backward_workspace_is_what_the_call_uses(built_lib):
-    """Row statistics (two floats per row of whole query blocks), fp16 q, dout, k, v unless they are fp16 already, the partial dK / dV of a
-    cut query range, and room for the partial results of the balanced schedule; no fp16 O."""
-    import kiln_b200
-    L = kiln_b200.lib()
-    split = 148 * 2 * (128 * 128 + 256) * 4 + 1280
-    assert L.kb_attn_bwd_workspace_bytes(1, 4096, 4096, 16, kiln_b200.KB_F16) == 4096 * 16 * 8 + split
-    assert L.kb_attn_bwd_workspace_bytes(1, 4096, 4096, 16, kiln_b200.KB_F32) == 4096 * 16 * 8 + 4 * 4096 * 4096 + split
-    assert L.kb_attn_bwd_workspace_bytes(2, 300, 300, 8, kiln_b200.KB_BF16) == 2 * 384 * 8 * 8 + 4 * 600 * 2048 + 2 * (3 * 600 * 1024 * 4) + split
-    assert L.kb_attn_bwd_workspace_bytes(1, 1024, 77, 16, kiln_b200.KB_F16) == 1024 * 16 * 8 + 2 * (8 * 77 * 2048 * 4) + split
-
-
 @pytest.mark.skipif(torch.cuda.is_available(), reason="checks the no-GPU behaviour")
 def test_no_device_fails_loudly(built_lib):
     """There is no CPU fallback: without a device every launch entry point returns KB_ERR_DEVICE."""

@@ -121,27 +121,6 @@ def test_equal_keys_give_zero_dq(kb):
     assert np.abs(dq).max() <= 2e-3, f"{np.abs(dq).max():.3e}"
 
 
-@pytest.mark.parametrize("kind", [None, "f16"])
-def test_least_workspace(kb, kind):
-    """Statistics, staged operands and partial dK / dV are all that a call needs: the same gradients with exactly that, an error code
-    with a little less."""
-    Tq, Tk, H = 300, 200, 2
-    D = H * 128
-    q, k, v, dout = (dev(seeded(80 + i, n, D, "f16"), kind) for i, n in enumerate((Tq, Tk, Tk, Tq)))
-    full = torch.empty(kb.lib().kb_attn_bwd_workspace_bytes(1, Tq, Tk, H, kb.KB_F16 if kind else kb.KB_F32), dtype=torch.uint8, device="cuda")
-    # 2 heads x 2 key blocks are few: three query blocks, each a part of its own
-    least = 384 * H * 8 + 2 * (3 * Tk * D * 4) + (0 if kind else 2 * (Tq + Tk) * D * 2)
-    runs = []
-    for ws in (full, full[:least]):
-        outs = [torch.full((T, D), float("nan"), device="cuda") for T in (Tq, Tk, Tk)]
-        kb.attn_bwd(*outs, q, k, v, dout, 1, Tq, Tk, 0, H, workspace=ws)
-        assert kb.check_status() == 0
-        runs.append(outs)
-    assert all(torch.equal(a, b) for a, b in zip(*runs))
-    with pytest.raises(kb.KilnError):
-        kb.attn_bwd(*outs, q, k, v, dout, 1, Tq, Tk, 0, H, workspace=full[:least - 256])
-
-
 def test_argument_errors(kb):
     import ctypes
     L = kb.lib()
