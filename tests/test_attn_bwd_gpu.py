@@ -60,6 +60,29 @@ def test_small_cases_vs_oracle(kb, Tq, Tk, H, npad, kind):
     assert_close(dv, rv, f"dv {Tq}x{Tk}x{H} npad {npad}")
 
 
+@pytest.mark.parametrize("Tq,Tk,H,npad,B,kind", [(1500, 1500, 16, 0, 1, "f16"), (2000, 300, 16, 212, 1, None), (1300, 1300, 8, 0, 2, "bf16"), (2500, 2500, 8, 0, 1, "f16")],
+                         ids=["whole_items", "whole_items_cross_pad_f32", "whole_items_batch_bf16", "cut_items_ragged"])
+def test_many_query_tiles_and_several_key_blocks(kb, Tq, Tk, H, npad, B, kind):
+    """More 128-row query tiles than SMs: the forward pass inside runs pairs of tiles over all keys, or cuts them. Sampled dq rows with
+    the full K / V, and one head's dk / dv on all queries (an image per case), against the oracle."""
+    D = H * 128
+    q, k = seeded(40, B * Tq, D, kind or "f16", 1.5), seeded(41, B * Tk, D, kind or "f16", 1.5)
+    v, dout = seeded(42, B * Tk, D, kind or "f16"), seeded(43, B * Tq, D, kind or "f16")
+    dq, dk, dv = _run(kb, q, k, v, dout, B, Tq, Tk, npad, H, kind)
+    for b in range(B):
+        sq, sk = slice(b * Tq, (b + 1) * Tq), slice(b * Tk, (b + 1) * Tk)
+        rows = sample_rows(Tq, 12)
+        rq, _, _ = oracle.attention_bwd(q[sq][rows], k[sk], v[sk], dout[sq][rows], H, npad, key_rows=(0, 0))
+        assert_close(dq[sq][rows], rq, f"dq rows {Tq}x{Tk}x{H} image {b}")
+        cs = slice((3 + b) * 128, (4 + b) * 128)
+        j0 = Tk - 140                                          # the ragged last block and the end of the one before
+        _, rk, rv = oracle.attention_bwd(q[sq, cs], k[sk, cs], v[sk, cs], dout[sq, cs], 1, npad, key_rows=(j0, Tk))
+        # dS and P are rounded to fp16 relative to themselves, so an error grows with the gradient row it enters, and with few keys
+        # and many queries a row's rms reaches 2: in float64 the rounding of dS alone moves an element of dk by up to 1.4e-3 of it
+        for name, g, r in (("dk", dk, rk), ("dv", dv, rv)):
+            assert_close(g[sk][j0:, cs], r, f"{name} {Tq}x{Tk}x{H} image {b}", max_abs=2e-3 * max(1.0, float(np.sqrt((r * r).mean(1)).max())))
+
+
 def test_batch_equals_per_image_calls(kb):
     B, T, H = 2, 200, 2
     D = H * 128

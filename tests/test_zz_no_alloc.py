@@ -54,7 +54,7 @@ def test_static_scratch_matches_workspace_entry_point_twice(built_lib):
         assert not np.isnan(out).any()
         e_max, e_rel, _ = errors(out, ref)
         assert e_max <= TOL_MAX_ABS and e_rel <= TOL_MEAN_REL, f"static vs workspace entry point: max_abs {e_max:.3e} mean_rel {e_rel:.3e}"
-        assert np.array_equal(out, ref)          # same kernels, same schedule (whole items per SM at these sizes), same bytes
+        assert np.array_equal(out, ref)          # same kernels, same schedule (no cut items at these sizes), same bytes
 
 
 def test_static_scratch_call_allocates_nothing(built_lib):
