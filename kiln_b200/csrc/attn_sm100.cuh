@@ -917,7 +917,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                 for (int q = 0; q < 4; q++) {
                                     uint4 g4[4];
 #pragma unroll
-                                    for (int cc = 0; cc < 4; cc++) g4[cc] = __ldcg(g + 4 * q + cc);
+                                    for (int cc = 0; cc < 4; cc++) g4[cc] = g[4 * q + cc];
                                     float v[32];
                                     chunk(q, v);
                                     D += dot32(g4, v);
@@ -1012,7 +1012,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         for (int q = 0; q < 2; q++) {
                             uint4 g4[4];
 #pragma unroll
-                            for (int cc = 0; cc < 4; cc++) g4[cc] = __ldcg(g + 4 * q + cc);
+                            for (int cc = 0; cc < 4; cc++) g4[cc] = g[4 * q + cc];
                             float v[32];
                             chunk(q, v);
                             D += dot32(g4, v);
