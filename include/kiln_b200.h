@@ -32,7 +32,8 @@ extern "C" {
  * converts its fp32 inputs to fp16 while staging (engine/src/tcflash.cuh:56-64): KB_F16 inputs that need
  * neither norm nor RoPE are read in place; KB_BF16 / KB_F32 inputs, and any tensor that gets RMSNorm or
  * RoPE, are staged once as fp16 in the caller's workspace by a fused pre-pass - except a 16-bit Q without
- * RoPE, which the attention kernel normalises and converts itself. KB_F32 inputs are what the
+ * RoPE, which the attention kernel normalises and converts itself (unless the output lies across Q's memory
+ * in any other way than exactly in place: then it is staged too). KB_F32 inputs are what the
  * engine holds today (engine/src/dit.cu:429-430). */
 enum { KB_F16 = 0, KB_BF16 = 1, KB_F32 = 2 };
 
@@ -59,7 +60,8 @@ int kb_init(void);
 /* Bytes of scratch an attention call needs: room for the fp16 staging copies of Q (when dtype is not
  * KB_F16 or norm_q != 0), of K per context (dtype not KB_F16 or norm_k != 0) and of V per context
  * (dtype not KB_F16). rows_q = B*Tq, rows_k = B*Tk (the largest context for NAG), n_ctx = 1, or 2 for
- * kb_attn_nag. norm_q / norm_k: that tensor gets RMSNorm and/or RoPE. */
+ * kb_attn_nag. norm_q / norm_k: that tensor gets RMSNorm and/or RoPE. The room for Q is asked for whether the
+ * call at hand stages Q or its kernel prepares it. */
 size_t kb_attn_workspace_bytes(int rows_q, int rows_k, int n_ctx, int H, int dtype, int norm_q, int norm_k);
 
 /* Self-attention of B images, T tokens each (Tq = Tk = T), no padding.
@@ -67,7 +69,9 @@ size_t kb_attn_workspace_bytes(int rows_q, int rows_k, int n_ctx, int H, int dty
  * attention16() (engine/src/dit.cu:464-470; ops at engine/src/kernels.cu:668-673, 773-777, 868-873).
  *   qn_w / kn_w : bf16 RMSNorm weight[128] for Q / K, or NULL for "already normalised"
  *   rope_cos / rope_sin : fp32 tables [T, 64] (engine/src/dit.cu:196-215), or NULL for no RoPE
- * q, k, v: [B*T, ld_*]; out: [B*T, ld_o]. */
+ * q, k, v: [B*T, ld_*]; out: [B*T, ld_o].
+ * How the work is divided over the SMs follows from B, T, H and the room in the workspace, and with it the order of the
+ * sums: repeats of a call are bit-identical, but an image alone and the same image in a batch may differ in the last bits. */
 int kb_attn_self(void* out, const void* q, const void* k, const void* v,
                  const void* qn_w, const void* kn_w, const float* rope_cos, const float* rope_sin,
                  int B, int T, int H, int ld_q, int ld_k, int ld_v, int ld_o,

@@ -105,14 +105,14 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
     }
     if (warp == 9 && lane == 0) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO); }
     if (warp == 8) {
-        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_alloc(smem_u32(tmem_slot), TMEM_ALL_COLUMNS);
         tmem_relinquish();
     }
     pdl_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    constexpr uint32_t tmem_base = 0;                             // all 512 columns are this thread block's (see elect_one)
+    constexpr uint32_t tmem_base = 0;                             // see TMEM_ALL_COLUMNS and elect_one
     pdl_wait();
 
     if (warp < 8) {

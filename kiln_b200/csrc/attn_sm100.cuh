@@ -25,7 +25,7 @@
 //
 // Warp roles (384 threads): warps 0-3 / 4-7: softmax of stream 0 / 1 (warp w owns TMEM lanes 32*(w%4)..+31,
 // one query row per thread), warps 8 / 10 issue the MMAs of stream 0 / 1 (one lane each), warp 9 issues TMA loads
-// (one lane), warp 11 idle.
+// (one lane; NAG: the bulk stores too), warp 11 runs the NAG norm exchange (idle in the other modes).
 //
 // TMEM (512 columns): R [0,128) P0 [128,192) P1 [192,256) O0 [256,384) O1 [384,512).
 // R is ONE score staging area shared by both streams: an S = Q K^T lands there, the stream's softmax threads
@@ -84,8 +84,9 @@ constexpr int POLY_PAIRS = KB_POLY_PAIRS; // of every 8 score pairs, this many t
 constexpr int ATTN_THREADS = 384;
 // Registers per thread after the warpgroups re-divide the 384 x 168 the block starts with: 256 softmax threads x 224 + 128
 // threads of the MMA / TMA / helper warps x 56 = 64512 exactly (a larger second number would leave the softmax warps'
-// increase waiting forever). At 224 the softmax code compiles without a spill, which matters more than usual here: with
-// 227 KB of the SM's 256 KB configured as shared memory there is almost no L1 left, so every spill access is an L2 round trip.
+// increase waiting forever). Spills matter more than usual here: with 227 KB of the SM's 256 KB configured as shared memory there is
+// almost no L1 left, so every spill access is an L2 round trip. At 224 -Xptxas -v reports none for MODE_KEYS and for MODE_PAIR with
+// stored outputs, 28 bytes of stores and 24 of loads for MODE_PAIR with RowStats, 52 and 44 for MODE_NAG with a 16-bit output.
 #ifndef KB_SOFTMAX_REGS
 #define KB_SOFTMAX_REGS 224
 #endif
@@ -409,14 +410,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (MODE == MODE_NAG) { tma_prefetch_desc(&tmK1); tma_prefetch_desc(&tmV1); }
     }
     if (warp == 8) {
-        tmem_alloc(smem_u32(tmem_slot), 512);
+        tmem_alloc(smem_u32(tmem_slot), TMEM_ALL_COLUMNS);
         tmem_relinquish();
     }
     pdl_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    constexpr uint32_t tmem_base = 0;                             // all 512 columns are this CTA's (see elect_one)
+    constexpr uint32_t tmem_base = 0;                             // see TMEM_ALL_COLUMNS and elect_one
     pdl_wait();                                                   // nothing in global memory is touched before this
     if (RAW_Q && p.q_raw && warp < 8) {                                    // (read by the softmax warps only)
         if (tid < HD) f_qw[tid] = p.qn_w ? __bfloat162float(p.qn_w[tid]) : 1.f;
@@ -1216,7 +1217,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             // Now one thread's bookkeeping runs under the other's MMAs.
             const int i = __shfl_sync(0xffffffffu, (warp - 8) >> 1, 0);
             if (elect_one()) {
-                // Operands are fp16 throughout (bf16/fp32 inputs are staged as fp16 by the pre-pass): with bf16
+                // Operands are fp16 throughout (bf16/fp32 inputs are staged as fp16 by the pre-pass, a raw Q is
+                // converted on its tile): with bf16
                 // P the 2^-9 rounding of each weight alone costs ~1e-3 relative error on outputs that are sums
                 // of random-sign terms, and tcgen05 does not take an fp16 A with a bf16 B.
                 constexpr uint32_t IDESC_S = idesc_f16(0, 0, 0, 0, BM, BN);   // S = Q K^T, both K-major

@@ -180,7 +180,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     tc_fence_before();
     if (PAIR) { cluster_arrive(); cluster_wait(); } else __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = PAIR ? 0u : *tmem_slot;                    // PAIR: all 512 columns are this CTA's (see elect_one)
+    static_assert(!PAIR || TMEM_COLS == TMEM_ALL_COLUMNS, "a pair's accumulators are addressed from column 0");
+    const uint32_t tmem_base = PAIR ? 0u : *tmem_slot;                    // see elect_one
     pdl_wait();
 
     if (warp < G_EPI_WARPS) {

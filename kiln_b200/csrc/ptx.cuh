@@ -17,7 +17,8 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 }
 
 // ---------------------------------------------------------------- dependent launches
-// Kernels of this library are launched with programmatic stream serialization: a kernel may be placed on SMs that its predecessor on
+// The pre-pass, attention, backward (and its reduction), flag-clearing and GEMM kernels are launched with programmatic stream
+// serialization (launch_dependent in abi.cu; the others are plain launches, have no pdl_wait and must stay plain): a kernel may be placed on SMs that its predecessor on
 // the stream has left while the predecessor's last blocks still run. pdl_launch() allows that for the kernel behind this one;
 // pdl_wait() returns once every kernel in front has completed and its writes are visible. A kernel touches no global memory before
 // its pdl_wait(), and every thread that touches any executes it; only its own set-up (barriers, TMEM, tensor map prefetch) runs ahead.
@@ -125,6 +126,9 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------- tcgen05: TMEM management
+// An allocation of all columns can only begin at column 0, so a kernel that makes one takes 0 as its base and leaves the word that
+// the allocation writes unread.
+constexpr uint32_t TMEM_ALL_COLUMNS = 512;
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
 }
