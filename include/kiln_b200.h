@@ -216,7 +216,9 @@ const void* kb_unit_norm_weight(void);
  *                  that need no further pass.
  * N must be a multiple of 128 and K of 64 (the engine asks N % 128 == 0, K % 32 == 0; every DiT weight
  * has K = 2048 or 8192); M is free. The three plain store epilogues (F32, F16, GELU16) also take any N that is a
- * multiple of 8: a LoRA down-projection t = x . A_cat^T has the stacked rank for its width. Pointers 16-byte aligned, strides multiples of 8 (fp16) / 4 (fp32). */
+ * multiple of 8: a LoRA down-projection t = x . A_cat^T has the stacked rank for its width. Pointers 16-byte aligned, strides multiples of 8 (fp16) / 4 (fp32).
+ * With few output tiles the K range is summed in two or four parts; their number follows from the epilogue, M, N and K, so repeats are
+ * bit-identical, but a row may differ in the last bits between calls of different M. */
 enum { KB_EPI_F32 = 0, KB_EPI_F16 = 1, KB_EPI_GELU16 = 2, KB_EPI_RESID = 3, KB_EPI_HEADS16 = 4 };
 int kb_linear16(void* C, int ldc, const void* A, int lda, const void* W, int ldw, int M, int N, int K, int epi,
                 const float* gate, const void* head_w_bf16, const float* rope_cos, const float* rope_sin, int rope_T,

@@ -649,32 +649,13 @@ int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& ma
                             dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
 }
 
-// CTA pairs on 256x256 tiles when that fills the device better. Measured on B200 a CTA of a pair spends about 11/8 of the
-// time a single CTA spends per 64-wide k step while doing twice the work, so compare waves x time per step (a step of a single CTA
-// = 8 units of ~43 ns). Either shape cuts the k steps of its tiles over split_k CTAs (pairs) of a cluster when all clusters are
-// resident at once; leaving, meeting and adding the parts costs about 3 us on single CTAs and 4 us on pairs (half of the warps run
-// the epilogue of twice the columns). Measured on B200 inside a CUDA graph, whole k range -> split (* without dependent launches,
-// which save 1.5 us): N 2048, K 8192: M 128 40.2* -> 16.3 us, 512 40.8* -> 25.3, 1024 41.6* -> 29.1; N 2048, K 2048: M 128 14.4* -> 9.2,
-// 512 15.0* -> 11.0; with M 1024 (pairs, head epilogue) 14.7 -> 17.1, so not taken there. N 96 (a stacked LoRA), K 2048, M 1536: 13.4* -> 10.1.
-constexpr int SPLIT_K_COST = 70, SPLIT_K_COST_PAIR = 95;
 template <int EPI>
 int launch_gemm(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, const GemmParams& p, int n_seg, cudaStream_t stream) {
-    const long long ksteps = p.K / GB_K;
-    long long best = -1;
-    int best_pair = 0, best_split = 1;
-    for (int pair = 1; pair >= 0; pair--) {
-        if (pair && (p.N % 256 || p.M <= 128)) continue;
-        const int tile = pair ? 256 : 128;
-        const long long tiles = (long long)((p.M + tile - 1) / tile) * ((p.N + tile - 1) / tile) * n_seg;
-        const long long unit = pair ? 11 : 8, groups = pair ? st->sm_count / 2 : st->sm_count;
-        for (int split = 1; split <= (pair ? 2 : 4); split *= 2) {
-            if (split > 1 && (ksteps < 2 * split || tiles > st->max_clusters[pair ? split : split / 2])) continue;
-            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + split - 1) / split) * unit + (split == 1 ? 0 : pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
-            if (best < 0 || cost < best) { best = cost; best_pair = pair; best_split = split; }
-        }
-    }
-    if (best_pair) return launch_gemm_shape<EPI, true>(st, ta, maps, p, n_seg, best_split, stream);
-    return launch_gemm_shape<EPI, false>(st, ta, maps, p, n_seg, best_split, stream);
+    // the epilogues that a launch of several projections and a call per projection both have
+    const bool any_n_seg = (EPI == EPI_HEADS16 || EPI == EPI_F16) && p.N % 128 == 0;
+    const GemmShape g = gemm_shape(p.M, p.N, p.K / GB_K, n_seg, any_n_seg, st->sm_count, st->max_clusters);
+    if (g.pair) return launch_gemm_shape<EPI, true>(st, ta, maps, p, n_seg, g.split, stream);
+    return launch_gemm_shape<EPI, false>(st, ta, maps, p, n_seg, g.split, stream);
 }
 
 // The second product of a segment (null = none): A2 [M, K2] with row stride lda2, W2 [N, K2] with row stride ldw2.

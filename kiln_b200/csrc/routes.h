@@ -1,5 +1,5 @@
-// Which schedule an attention call takes: rules on sizes only, plain host code (no CUDA headers), so that they can be tested without
-// a device.
+// Which schedule an attention call takes and which tile shape a GEMM: rules on sizes only, plain host code (no CUDA headers), so that
+// they can be tested without a device.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -71,6 +71,44 @@ inline bool share_bytes(const MatBytes& x, const MatBytes& y) {
 // head) of the output lies exactly on its own Q, which only the item itself reads.
 inline bool q_survives_output(const MatBytes& q, const MatBytes& out) {
     return !share_bytes(q, out) || (q.p == out.p && q.stride == out.stride && q.width == out.width);
+}
+
+// GEMM: CTA pairs on 256x256 tiles when that fills the device better. Measured on B200 a CTA of a pair spends about 11/8 of the
+// time a single CTA spends per 64-wide k step while doing twice the work, so compare waves x time per step (a step of a single CTA
+// = 8 units of ~43 ns). Either shape cuts the k steps of its tiles over `split` CTAs (pairs) of a cluster when all clusters are
+// resident at once; leaving, meeting and adding the parts costs about 3 us on single CTAs and 4 us on pairs (half of the warps run
+// the epilogue of twice the columns). Measured on B200 inside a CUDA graph, whole k range -> split (* without dependent launches,
+// which save 1.5 us): N 2048, K 8192: M 128 40.2* -> 16.3 us, 512 40.8* -> 25.3, 1024 41.6* -> 29.1; N 2048, K 2048: M 128 14.4* -> 9.2,
+// 512 15.0* -> 11.0; with M 1024 (pairs, head epilogue) 14.7 -> 17.1, so not taken there. N 96 (a stacked LoRA), K 2048, M 1536: 13.4* -> 10.1.
+constexpr int SPLIT_K_COST = 70, SPLIT_K_COST_PAIR = 95;
+struct GemmShape {
+    bool pair;
+    int split;
+};
+// The cheapest shape among those with `split` parts (0: any). max_clusters[1], [2]: resident clusters of 2 and 4 CTAs.
+inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int split, int sm_count, const int* max_clusters) {
+    long long best = -1;
+    GemmShape shape = {false, 1};
+    for (int pair = 1; pair >= 0; pair--) {
+        if (pair && (N % 256 || M <= 128)) continue;
+        const int tile = pair ? 256 : 128;
+        const long long tiles = (long long)((M + tile - 1) / tile) * ((N + tile - 1) / tile) * n_seg;
+        const long long unit = pair ? 11 : 8, groups = pair ? sm_count / 2 : sm_count;
+        for (int s = 1; s <= (pair ? 2 : 4); s *= 2) {
+            if ((split && s != split) || (s > 1 && (ksteps < 2 * s || tiles > max_clusters[pair ? s : s / 2]))) continue;
+            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + s - 1) / s) * unit + (s == 1 ? 0 : pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
+            if (best < 0 || cost < best) { best = cost; shape = {pair != 0, s}; }
+        }
+    }
+    return shape;
+}
+// n_seg weight matrices in one launch. any_n_seg: the outputs have to be the same to the bit whether the projections of an activation
+// share a launch or not. The number of parts is the order of the sums (the tile shape is not), so it is then the one that suits three
+// segments, for one and two as well: a split that would pay for a single projection only is left out (N 2048, K 2048: four parts up to
+// M 256, two up to M 512; below M 128 two parts are left).
+inline GemmShape gemm_shape(int M, int N, long long ksteps, int n_seg, bool any_n_seg, int sm_count, const int* max_clusters) {
+    const int split = any_n_seg ? gemm_cheapest(M, N, ksteps, 3, 0, sm_count, max_clusters).split : 0;
+    return gemm_cheapest(M, N, ksteps, n_seg, split, sm_count, max_clusters);
 }
 
 }  // namespace kb

@@ -224,7 +224,8 @@ def test_edge_shapes_every_epilogue(kb, M, N, K):
     assert np.all(np.abs(out - ref) <= 2.0 ** -10 * np.abs(ref) + 1e-4), f"{M}x{N}x{K} heads16: {np.abs(out - ref).max():.3e}"
 
 
-@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (4096, 16, 2048)], ids=["pair_tiles", "single_tiles", "dit_size"])
+@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (4096, 16, 2048), (100, 2, 2048), (128, 16, 2048), (300, 16, 2048), (512, 16, 2048), (200, 16, 8192)],
+                         ids=["pair_tiles", "single_tiles", "dit_size", "four_parts", "two_parts", "split_for_one_only", "split_for_one_only_512", "long_k"])
 def test_qkv_one_launch_equals_three_calls(kb, M, H, K):
     """kb_linear16_qkv: q and k with their own norm weights and RoPE, v plain — bit-identical to three kb_linear16 calls."""
     from kiln_b200 import ops
@@ -324,7 +325,8 @@ def test_lora_second_product_vs_oracle_and_reference_golden(kb, gemm_golden, cas
                          ids=["four_parts", "narrow_uneven_parts", "four_parts_second_product", "two_parts", "ragged_two_parts", "two_parts_of_pairs"])
 def test_split_k_every_epilogue(kb, M, N, K, K2):
     """Few tiles and many k steps: the k steps of a tile run on two or four CTAs (two pairs) of a cluster, each of which finishes a
-    share of the rows. Step counts that do not divide, a second product whose steps fall into the last part, ragged rows, a narrow
+    share of the rows (the two fp16 store epilogues that a launch of several projections has too only where that one is cut as well).
+    Step counts that do not divide, a second product whose steps fall into the last part, ragged rows, a narrow
     last column tile; sampled rows against the oracle, nothing outside the M x N window, repeat runs bit-identical."""
     from kiln_b200 import ops
     x, w = seeded(600 + M, M, K, "f16"), seeded(601, N, K, "f16", 1.0 / np.sqrt(K))
@@ -370,7 +372,7 @@ def test_second_product_shapes(kb, M, N, K, K2):
     _close(c[torch.as_tensor(rows, device="cuda")].cpu().numpy(), ref, K + K2, f"{M}x{N}x{K}+{K2}", False)
 
 
-@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192)], ids=["pair_tiles", "single_tiles"])
+@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (128, 16, 2048), (300, 16, 2048)], ids=["pair_tiles", "single_tiles", "two_parts", "split_for_one_only"])
 def test_qkv_lora_one_launch_equals_three_calls(kb, M, H, K):
     """kb_linear16_qkv_lora with a different rank per projection (none on v) — bit-identical to three kb_linear16_lora /
     kb_linear16 calls, and the head epilogue sees the LoRA-adjusted value (checked against the oracle on q)."""

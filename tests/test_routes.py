@@ -1,4 +1,4 @@
-"""CPU test of the rule that picks an attention call's schedule (kiln_b200/csrc/routes.h, plain C++)."""
+"""CPU tests of the rules that pick an attention call's schedule and a GEMM's tile shape (kiln_b200/csrc/routes.h, plain C++)."""
 import ctypes
 import os
 import subprocess
@@ -28,6 +28,8 @@ def rules(tmp_path_factory):
     src = d / "routes.cpp"
     src.write_text('#include "routes.h"\n'
                    'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n'
+                   'extern "C" int gemm(int M, int N, int ksteps, int n_seg, int any, int mc2, int mc4) {\n'
+                   '    const int mc[3] = {0, mc2, mc4}; const kb::GemmShape g = kb::gemm_shape(M, N, ksteps, n_seg, any, 148, mc); return g.pair * 8 + g.split; }\n'
                    'extern "C" int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {\n'
                    '    return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth}); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
@@ -54,6 +56,23 @@ def test_restrictions(route):
     assert route(1, 1024, 1024, 16, SMS, 0, 1) == WHOLE and route(1, 4096, 4096, 2, SMS, 0, 1) == BALANCED   # a call with peers
     for Tq in (1, 128, 129, 4096):
         assert route(1, Tq, 128, 1, SMS, 1, 1) == WHOLE                                                      # one key block: one stream has none
+
+
+def test_projections_sum_in_one_order_whether_they_share_a_launch_or_not(rules):
+    """The number of k ranges is the same for one, two and three segments; a split that is chosen has room for all its clusters."""
+    splits = set()
+    for mc2, mc4 in ((74, 37), (70, 32), (0, 0)):
+        for M in (1, 77, 128, 129, 200, 256, 300, 512, 700, 1000, 1536, 4096):
+            for N in (128, 256, 384, 1920, 2048):
+                for ksteps in (2, 16, 32, 33, 128):
+                    shapes = [rules.gemm(M, N, ksteps, n, 1, mc2, mc4) for n in (1, 2, 3)]
+                    assert len({g & 7 for g in shapes}) == 1, (M, N, ksteps, shapes)
+                    splits.add(shapes[0] & 7)
+                    for n, g in zip((1, 2, 3), shapes):
+                        tile, split = (256 if g & 8 else 128), g & 7
+                        assert split == 1 or -(-M // tile) * -(-N // tile) * n <= (mc2 if not g & 8 and split == 2 else mc4)
+    assert splits == {1, 2, 4}
+    assert rules.gemm(256, 2048, 32, 1, 0, 74, 37) & 7 == 4          # without that duty a few tiles still split
 
 
 def test_raw_q_needs_an_output_that_leaves_it_alone(rules):
