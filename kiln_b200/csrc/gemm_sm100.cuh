@@ -106,8 +106,11 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     constexpr int BN = PAIR ? 256 : 128;                                  // accumulator columns per tile
     constexpr int TILE_M = PAIR ? 256 : 128;                              // tile rows over the CTA group
     constexpr bool OUT32 = (EPI == EPI_F32 || EPI == EPI_RESID);
-    constexpr int CW = OUT32 ? 64 : 128;                                  // columns per 256-byte output row chunk
-    constexpr int NCH = BN / CW;
+    // columns per output chunk: 256-byte rows, or 128-byte rows where a tile would be a single chunk (16-bit output of one CTA), so that
+    // both warps of a lane quarter have one: every epilogue warp has to hand its share of the accumulator back
+    constexpr int CW = OUT32 || !PAIR ? 64 : 128;
+    constexpr int NCH = BN / CW, CHUNK_BOXES = CW * (OUT32 ? 4 : 2) / 128;
+    static_assert(NCH >= 2, "a chunk for both warps of a lane quarter");
     constexpr uint32_t TMEM_COLS = 2 * BN;
 
     extern __shared__ uint8_t smem_raw[];
@@ -397,13 +400,13 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                             }
                         }
                     }
-                    // the 32 x 256-byte piece of the output goes through shared memory as two 128-byte-swizzled boxes and
+                    // the 32 rows of the chunk go through shared memory as one or two 128-byte-swizzled boxes and
                     // leaves by TMA (measured: 32 row stores per warp took 3 us, the issue rate of plain global stores from
                     // eight warps; the bulk copy takes them off the warp)
                     if (lane == 0) tma_store_wait_read();                     // the boxes of the last chunk have been read
                     __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
+                    for (int c = 0; c < 8 * CHUNK_BOXES; c++) {
                         uint4 pk;
                         if constexpr (OUT32) {
                             pk = make_uint4(__float_as_uint(v[4 * c]), __float_as_uint(v[4 * c + 1]), __float_as_uint(v[4 * c + 2]), __float_as_uint(v[4 * c + 3]));
@@ -419,10 +422,10 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     if (lane == 0 && nrow > 0 && x < p.N) {                   // a narrow last column tile stores only the boxes that begin inside it
                         if constexpr (EPI == EPI_RESID) {
                             tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage), x, y, 0);
-                            tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
+                            if (CHUNK_BOXES == 2) tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
                         } else {
                             tma_store_3d(&maps.c[seg], smem_u32(my_stage), x, y, 0);
-                            if (x + CW / 2 < p.N) tma_store_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
+                            if (CHUNK_BOXES == 2 && x + CW / 2 < p.N) tma_store_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
                         }
                         tma_store_commit();
                     }

@@ -421,6 +421,19 @@ def test_narrow_outputs_of_the_store_epilogues(kb, N):
         _close(out, oracle.linear16(x, w, epi), K, f"N={N} epi {epi}", epi in (1, 2))
 
 
+@pytest.mark.parametrize("M,N", [(2561, 1920), (19001, 200)], ids=lambda v: str(v))
+def test_more_than_two_tiles_per_thread_block(kb, M, N):
+    """Widths that 256 does not divide run one 128 x 128 tile per thread block: beyond 2 x 148 tiles a block comes back to its first
+    accumulator, which every epilogue warp has to have handed back. Fp64 reference of the same product, bounds as elsewhere."""
+    from kiln_b200 import ops
+    K = 64
+    x, w = seeded(700, M, K, "f16"), seeded(701, N, K, "f16", 1.0 / np.sqrt(K))
+    ref = x.astype(np.float64) @ w.astype(np.float64).T
+    for epi in (ops.EPI_F32, ops.EPI_F16, ops.EPI_GELU16):
+        r = torch.nn.functional.gelu(torch.from_numpy(ref)).numpy() if epi == ops.EPI_GELU16 else ref
+        _close(_run(kb, x, w, epi), r, K, f"M={M} N={N} epi {epi}", epi != ops.EPI_F32)
+
+
 def test_lora_argument_errors(kb):
     import ctypes
     L = kb.lib()
