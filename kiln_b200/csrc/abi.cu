@@ -79,6 +79,8 @@ int set_gemm_smem() {
     if ((rc = set_smem(gemm16_kernel<EPI, true, false>, G_SMEM)) || (rc = set_smem(gemm16_kernel<EPI, false, false>, G_SMEM)) ||
         (rc = set_smem(gemm16_kernel<EPI, true, true>, G_SMEM)) || (rc = set_smem(gemm16_kernel<EPI, false, true>, G_SMEM)))
         return rc;
+    if constexpr (EPI != EPI_HEADS16)
+        if ((rc = set_smem(gemm16_kernel<EPI, true, false, 224>, G_SMEM)) || (rc = set_smem(gemm16_kernel<EPI, true, false, 192>, G_SMEM))) return rc;
     return KB_OK;
 }
 
@@ -606,24 +608,26 @@ int kb_qk_prep(void* out, int ld_out, int out_dtype, const void* in, int ld_in, 
 namespace {
 
 // [rows][cols] view of the output with row stride ld; box = 128 bytes of columns x 32 rows with 128-byte swizzle, or
-// (half_heads: the fused head epilogue stores 32-column half-heads) 64 bytes x 32 rows unswizzled
-int make_tmap_out(CUtensorMap* tm, void* ptr, int rows, int cols, int ld, bool f32, bool half_heads) {
+// (half_heads: the fused head epilogue stores 32-column half-heads) 64 bytes x 32 rows unswizzled, or (narrow tiles) 32 columns x 32
+// rows, swizzled over a row
+int make_tmap_out(CUtensorMap* tm, void* ptr, int rows, int cols, int ld, bool f32, bool half_heads, bool narrow) {
     const cuuint64_t esz = f32 ? 4 : 2;
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * esz, (cuuint64_t)rows * (cuuint64_t)ld * esz};
-    const cuuint32_t box[3] = {half_heads ? 32u : (cuuint32_t)(128 / esz), 32, 1};
+    const cuuint32_t box[3] = {half_heads || narrow ? 32u : (cuuint32_t)(128 / esz), 32, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = g_encode(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, ptr, dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, half_heads ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          half_heads ? CU_TENSOR_MAP_SWIZZLE_NONE : narrow && !f32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? KB_OK : KB_ERR_CUDA;
 }
 
-// [rows][cols] view of a row-major fp16 matrix with row stride ld; box = 64 columns x 128 rows, 128-byte swizzle
-int make_tmap_mat(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld) {
+// [rows][cols] view of a row-major fp16 matrix with row stride ld; box = 64 columns x box_rows rows, 128-byte swizzle
+int make_tmap_mat(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_rows = 128) {
     const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
     const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * (cuuint64_t)ld * 2};
-    const cuuint32_t box[3] = {64, 128, 1};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -632,11 +636,11 @@ int make_tmap_mat(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld) 
 }
 
 // p.N is the width of ONE segment; the launch covers n_seg of them side by side
-template <int EPI, bool PAIR>
+template <int EPI, bool PAIR, int BN>
 int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, GemmParams p, int n_seg, int split_k, cudaStream_t stream) {
-    const int tile = PAIR ? 256 : 128, per_group = PAIR ? 2 : 1;
-    p.tiles_m = (p.M + tile - 1) / tile;
-    p.tiles_n_seg = (p.N + tile - 1) / tile;
+    const int tile_m = PAIR ? 256 : 128, per_group = PAIR ? 2 : 1;
+    p.tiles_m = (p.M + tile_m - 1) / tile_m;
+    p.tiles_n_seg = (p.N + BN - 1) / BN;
     p.tiles_n = p.tiles_n_seg * n_seg;
     const int n_tiles = p.tiles_m * p.tiles_n, max_groups = st->sm_count / per_group;
     p.split_k = split_k;
@@ -645,17 +649,20 @@ int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& ma
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = ctas; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
     ProfScope ps(st, KB_PROF_LINEAR, stream);
-    return launch_dependent(split_k > 1 ? gemm16_kernel<EPI, PAIR, true> : gemm16_kernel<EPI, PAIR, false>, dim3((unsigned)(groups * ctas)),
-                            dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
+    auto kernel = gemm16_kernel<EPI, PAIR, false, BN>;
+    if constexpr (BN == (PAIR ? 256 : 128))
+        if (split_k > 1) kernel = gemm16_kernel<EPI, PAIR, true, BN>;
+    return launch_dependent(kernel, dim3((unsigned)(groups * ctas)), dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
 }
 
 template <int EPI>
-int launch_gemm(DeviceState* st, const CUtensorMap& ta, const GemmMaps& maps, const GemmParams& p, int n_seg, cudaStream_t stream) {
-    // the epilogues that a launch of several projections and a call per projection both have
-    const bool any_n_seg = (EPI == EPI_HEADS16 || EPI == EPI_F16) && p.N % 128 == 0;
-    const GemmShape g = gemm_shape(p.M, p.N, p.K / GB_K, n_seg, any_n_seg, st->sm_count, st->max_clusters);
-    if (g.pair) return launch_gemm_shape<EPI, true>(st, ta, maps, p, n_seg, g.split, stream);
-    return launch_gemm_shape<EPI, false>(st, ta, maps, p, n_seg, g.split, stream);
+int launch_gemm(DeviceState* st, const GemmShape& g, const CUtensorMap& ta, const GemmMaps& maps, const GemmParams& p, int n_seg, cudaStream_t stream) {
+    if constexpr (EPI != EPI_HEADS16) {
+        if (g.width == 224) return launch_gemm_shape<EPI, true, 224>(st, ta, maps, p, n_seg, g.split, stream);
+        if (g.width == 192) return launch_gemm_shape<EPI, true, 192>(st, ta, maps, p, n_seg, g.split, stream);
+    }
+    if (g.pair) return launch_gemm_shape<EPI, true, 256>(st, ta, maps, p, n_seg, g.split, stream);
+    return launch_gemm_shape<EPI, false, 128>(st, ta, maps, p, n_seg, g.split, stream);
 }
 
 // The second product of a segment (null = none): A2 [M, K2] with row stride lda2, W2 [N, K2] with row stride ldw2.
@@ -703,18 +710,24 @@ int linear16_segments(void* const* C, int ldc, const void* A, int lda, const voi
     DeviceState* st;
     int rc;
     if ((rc = get_state(&st))) return rc;
+    // F16, HEADS16: the epilogues that a launch of several projections and a call per projection both have
+    const bool any_n_seg = (epi == KB_EPI_HEADS16 || epi == KB_EPI_F16) && N % 128 == 0;
+    const GemmShape g = gemm_shape(M, N, K / GB_K, n_seg, any_n_seg, st->sm_count, st->max_clusters, epi != KB_EPI_HEADS16);
+    const bool narrow = g.pair && g.width != 256;
+    const int w_rows = narrow ? g.width / 2 : 128;               // W rows per load
     CUtensorMap ta;
     GemmMaps maps;
     memset(&maps, 0, sizeof(maps));
     if ((rc = make_tmap_mat(&ta, A, M, K, lda))) return rc;
     GemmParams p = {};
     for (int i = 0; i < n_seg; i++) {
-        if ((rc = make_tmap_mat(&maps.w[i], W[i], N, K, ldw)) || (rc = make_tmap_out(&maps.c[i], C[i], M, N, ldc, c32, epi == KB_EPI_HEADS16))) return rc;
+        if ((rc = make_tmap_mat(&maps.w[i], W[i], N, K, ldw, w_rows)) ||
+            (rc = make_tmap_out(&maps.c[i], C[i], M, N, ldc, c32, epi == KB_EPI_HEADS16, narrow))) return rc;
         p.head_w[i] = static_cast<const __nv_bfloat16*>(head_w[i]);
         p.rope_on[i] = rope_on[i] ? 1 : 0;
         if (sp.K2 && sp.K2[i] > 0) {
             p.K2[i] = sp.K2[i];
-            if ((rc = make_tmap_mat(&maps.a2[i], sp.A2[i], M, sp.K2[i], sp.lda2[i])) || (rc = make_tmap_mat(&maps.w2[i], sp.W2[i], N, sp.K2[i], sp.ldw2[i]))) return rc;
+            if ((rc = make_tmap_mat(&maps.a2[i], sp.A2[i], M, sp.K2[i], sp.lda2[i])) || (rc = make_tmap_mat(&maps.w2[i], sp.W2[i], N, sp.K2[i], sp.ldw2[i], w_rows))) return rc;
         }
     }
     p.C = C[0]; p.ldc = ldc; p.M = M; p.N = N; p.K = K;
@@ -722,11 +735,11 @@ int linear16_segments(void* const* C, int ldc, const void* A, int lda, const voi
     p.rope_cos = rope_cos; p.rope_sin = rope_sin; p.rope_T = rope_T > 0 ? rope_T : 1; p.eps = eps;
     p.status = st->status;
     switch (epi) {
-        case KB_EPI_F32: return launch_gemm<EPI_F32>(st, ta, maps, p, n_seg, stream);
-        case KB_EPI_F16: return launch_gemm<EPI_F16>(st, ta, maps, p, n_seg, stream);
-        case KB_EPI_GELU16: return launch_gemm<EPI_GELU16>(st, ta, maps, p, n_seg, stream);
-        case KB_EPI_RESID: return launch_gemm<EPI_RESID>(st, ta, maps, p, n_seg, stream);
-        default: return launch_gemm<EPI_HEADS16>(st, ta, maps, p, n_seg, stream);
+        case KB_EPI_F32: return launch_gemm<EPI_F32>(st, g, ta, maps, p, n_seg, stream);
+        case KB_EPI_F16: return launch_gemm<EPI_F16>(st, g, ta, maps, p, n_seg, stream);
+        case KB_EPI_GELU16: return launch_gemm<EPI_GELU16>(st, g, ta, maps, p, n_seg, stream);
+        case KB_EPI_RESID: return launch_gemm<EPI_RESID>(st, g, ta, maps, p, n_seg, stream);
+        default: return launch_gemm<EPI_HEADS16>(st, g, ta, maps, p, n_seg, stream);
     }
 }
 

@@ -9,6 +9,10 @@
 // about 100 B/clk/SM), not by the tensor pipe. Single: one CTA per 128x128 tile, for N not a multiple of 256, M <= 128,
 // or when the pair shape would fill the device worse (the host decides).
 //
+// NARROW: the same pair on 224 or 192 columns, where that fills a round of tiles better (gemm_shape in routes.h has the rule and both sides
+// measured). Each CTA then loads 112 or 96 W rows per k step, and a tile leaves in chunks of 32 columns: one fp32 box of 128-byte rows,
+// or one fp16 box of 64-byte rows. Not for the head epilogue, whose tiles are whole heads.
+//
 // Split K (p.split_k = 2 or 4): with fewer tiles than half of the SMs the k steps of a tile are cut into split_k ranges, one CTA (or
 // pair) each, all of a tile in one cluster. Every CTA leaves the accumulator rows that it does not finish in its own shared memory
 // (the operand ring, which is free by then); after a cluster barrier the CTA that owns a quarter (split_k = 4) or a half of the rows
@@ -100,18 +104,22 @@ __global__ void lora_pack_kernel(__half* dst, int ld, int col0, const __nv_bfloa
     dst[(size_t)r * ld + col0 + c] = __float2half_rn(scale * __bfloat162float(src[i]));
 }
 
-template <int EPI, bool PAIR, bool SPLIT>
+template <int EPI, bool PAIR, bool SPLIT, int BN = PAIR ? 256 : 128>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ GemmMaps maps, const GemmParams p) {
-    constexpr int BN = PAIR ? 256 : 128;                                  // accumulator columns per tile
+    static_assert(BN == (PAIR ? 256 : 128) || (PAIR && !SPLIT && EPI != EPI_HEADS16 && BN % 32 == 0 && BN < 256), "tile width");
+    constexpr int BUF_COLS = PAIR ? 256 : 128;                            // TMEM columns from one accumulator buffer (BN of them used) to the next
+    constexpr int W_ROWS = PAIR ? BN / 2 : BN;                            // W rows this CTA loads per k step
+    constexpr uint32_t STAGE_TX = (GB_M + W_ROWS) * GB_K * 2;             // bytes of a stage in use
     constexpr int TILE_M = PAIR ? 256 : 128;                              // tile rows over the CTA group
     constexpr bool OUT32 = (EPI == EPI_F32 || EPI == EPI_RESID);
+    constexpr bool NARROW = BN != BUF_COLS;                               // tiles that leave in chunks of one box, 32 columns wide
     // columns per output chunk: 256-byte rows, or 128-byte rows where a tile would be a single chunk (16-bit output of one CTA), so that
     // both warps of a lane quarter have one: every epilogue warp has to hand its share of the accumulator back
-    constexpr int CW = OUT32 || !PAIR ? 64 : 128;
-    constexpr int NCH = BN / CW, CHUNK_BOXES = CW * (OUT32 ? 4 : 2) / 128;
+    constexpr int CW = NARROW ? 32 : OUT32 || !PAIR ? 64 : 128;
+    constexpr int NCH = BN / CW, CHUNK_BOXES = NARROW ? 1 : CW * (OUT32 ? 4 : 2) / 128;
     static_assert(NCH >= 2, "a chunk for both warps of a lane quarter");
-    constexpr uint32_t TMEM_COLS = 2 * BN;
+    constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -244,7 +252,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 named_bar_sync(pair_bar, 64);
                 if (SPLIT) {
                     tc_fence_after();
-                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BN), quarter, hs, ok);
+                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BUF_COLS), quarter, hs, ok);
                 }
                 if (!ok) break;
                 tc_fence_after();
@@ -253,8 +261,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     float x0[32], x1[32];
                     {
                         uint32_t a0[32], a1[32];
-                        tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BN + h * 128 + hs * 32), a0);
-                        tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BN + h * 128 + 64 + hs * 32), a1);
+                        tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BUF_COLS + h * 128 + hs * 32), a0);
+                        tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BUF_COLS + h * 128 + 64 + hs * 32), a1);
                         tmem_wait_ld();
                         reg_fence32(a0);
                         reg_fence32(a1);
@@ -337,7 +345,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
             const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
             uint8_t* const my_stage = stage_out + warp * 32 * 256;           // this warp's 32 rows x 256 bytes on their way out
             uint32_t use[2] = {0, 0};
-            int k = 0;
+            int k = 0, box_use = 0;
             for (int w = group; w < n_tiles; w += n_groups, ++k) {
                 const int buf = k & 1;
                 int tm, tn;
@@ -348,7 +356,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 ++use[buf];
                 if (SPLIT) {
                     tc_fence_after();
-                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BN), quarter, chunk0, ok);
+                    ok = exchange_parts(tmem_base + lane_base + (uint32_t)(buf * BUF_COLS), quarter, chunk0, ok);
                 }
                 if (!ok) break;                                               // warps are independent from here on
                 tc_fence_after();
@@ -359,7 +367,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     {
                         uint32_t a[CW / 32][32];
 #pragma unroll
-                        for (int q = 0; q < CW / 32; q++) tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BN + ch * CW + 32 * q), a[q]);
+                        for (int q = 0; q < CW / 32; q++) tmem_ld32(tmem_base + lane_base + (uint32_t)(buf * BUF_COLS + ch * CW + 32 * q), a[q]);
                         tmem_wait_ld();
 #pragma unroll
                         for (int q = 0; q < CW / 32; q++) {
@@ -392,13 +400,41 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                         for (int c = 0; c < CW; c++) v[c] = gelu_erf(v[c]);
                     }
                     if constexpr (EPI == EPI_RESID) {
-                        if (p.gate) {
+                        if (p.gate && (!NARROW || n0 + ch * CW < p.N)) {
 #pragma unroll
                             for (int c = 0; c < CW; c += 4) {
                                 const float4 gt = *reinterpret_cast<const float4*>(p.gate + n0 + ch * CW + c);
                                 v[c] *= gt.x; v[c + 1] *= gt.y; v[c + 2] *= gt.z; v[c + 3] *= gt.w;
                             }
                         }
+                    }
+                    const int x = n0 + ch * CW, y = m0 + quarter * 32;
+                    if constexpr (NARROW) {
+                        // one box of 32 columns (128-byte rows of fp32, 64-byte rows of fp16, swizzled likewise) in the two halves of
+                        // this warp's stage in turn: the box before the last has been read when the last one is all that is in flight
+                        uint8_t* const box = my_stage + box_use * 4096;
+                        box_use ^= 1;
+                        if (lane == 0) tma_store_wait_read_1();
+                        __syncwarp();
+#pragma unroll
+                        for (int c = 0; c < (OUT32 ? 8 : 4); c++) {
+                            if constexpr (OUT32)
+                                *reinterpret_cast<float4*>(box + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                            else
+                                *reinterpret_cast<uint4*>(box + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+                                    make_uint4(pack16<DT_F16>(v[8 * c], v[8 * c + 1]), pack16<DT_F16>(v[8 * c + 2], v[8 * c + 3]),
+                                               pack16<DT_F16>(v[8 * c + 4], v[8 * c + 5]), pack16<DT_F16>(v[8 * c + 6], v[8 * c + 7]));
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {                                      // an empty group where nothing is stored: the count above holds
+                            if (nrow > 0 && x < p.N) {
+                                if constexpr (EPI == EPI_RESID) tma_reduce_add_3d(&maps.c[seg], smem_u32(box), x, y, 0);
+                                else tma_store_3d(&maps.c[seg], smem_u32(box), x, y, 0);
+                            }
+                            tma_store_commit();
+                        }
+                        continue;
                     }
                     // the 32 rows of the chunk go through shared memory as one or two 128-byte-swizzled boxes and
                     // leaves by TMA (measured: 32 row stores per warp took 3 us, the issue rate of plain global stores from
@@ -418,7 +454,6 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    const int x = n0 + ch * CW, y = m0 + quarter * 32;
                     if (lane == 0 && nrow > 0 && x < p.N) {                   // a narrow last column tile stores only the boxes that begin inside it
                         if constexpr (EPI == EPI_RESID) {
                             tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage), x, y, 0);
@@ -462,8 +497,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
                         const uint32_t acc = (ks > ks0 || kk > 0) ? 1u : 0u;
-                        if (PAIR) mma_ss_pair(tmem_base + (uint32_t)(buf * BN), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
-                        else mma_ss(tmem_base + (uint32_t)(buf * BN), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
+                        if (PAIR) mma_ss_pair(tmem_base + (uint32_t)(buf * BUF_COLS), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
+                        else mma_ss(tmem_base + (uint32_t)(buf * BUF_COLS), adesc + (uint64_t)(kk * 2), wdesc + (uint64_t)(kk * 2), IDESC, acc);
                     }
                     if (PAIR) tc_commit_pair(bar(GBAR_EMPTY + st), (uint16_t)(3u << lead)); else tc_commit(bar(GBAR_EMPTY + st));
                 }
@@ -484,7 +519,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                 int tm, tn;
                 gemm_tile(w, p, tm, tn);
                 const int seg = tn / p.tiles_n_seg;
-                const int m0 = tm * TILE_M + (int)rank * GB_M, wrow0 = (tn - seg * p.tiles_n_seg) * BN + (int)rank * 128;
+                const int m0 = tm * TILE_M + (int)rank * GB_M, wrow0 = (tn - seg * p.tiles_n_seg) * BN + (int)rank * W_ROWS;
                 const int ksteps = ksteps1 + (p.K2[seg] + GB_K - 1) / GB_K;
                 const int ks1 = ksteps * (part + 1) / S;
                 for (int ks = ksteps * part / S; ks < ks1 && good; ++ks, ++ring) {
@@ -498,7 +533,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     const uint32_t a_s = sRing + st * G_STAGE_BYTES;
                     if (PAIR) {
                         // both CTAs' bytes complete on the issuing CTA's barrier
-                        if (rank == 0) mbar_expect_tx(bar(GBAR_FULL + st), 2 * G_STAGE_BYTES);
+                        if (rank == 0) mbar_expect_tx(bar(GBAR_FULL + st), 2 * STAGE_TX);
                         const uint32_t fb = mapa_u32(bar(GBAR_FULL + st), lead);
                         tma_load_3d_pair(a_s, tmL, fb, k0, m0, 0);
                         tma_load_3d_pair(a_s + GB_M * GB_K * 2, tmW, fb, k0, wrow0, 0);

@@ -80,24 +80,34 @@ inline bool q_survives_output(const MatBytes& q, const MatBytes& out) {
 // the epilogue of twice the columns). Measured on B200 inside a CUDA graph, whole k range -> split (* without dependent launches,
 // which save 1.5 us): N 2048, K 8192: M 128 40.2* -> 16.3 us, 512 40.8* -> 25.3, 1024 41.6* -> 29.1; N 2048, K 2048: M 128 14.4* -> 9.2,
 // 512 15.0* -> 11.0; with M 1024 (pairs, head epilogue) 14.7 -> 17.1, so not taken there. N 96 (a stacked LoRA), K 2048, M 1536: 13.4* -> 10.1.
-constexpr int SPLIT_K_COST = 70, SPLIT_K_COST_PAIR = 95;
+//
+// Narrow tiles: a CTA pair takes 224 or 192 columns where whole rounds of 256 would leave SMs without a tile. A k step takes in proportion
+// to the width (330, 285, 240 ns in a round that is not full), so the rounds decide. Measured on B200 inside a CUDA graph, 256 columns ->
+// the width taken: N 2048, K 2048 (residual): M 1536 18.8 -> 15.1 us (192: 66 tiles on 74 pairs, not 48), 1792 18.5 -> 16.6 (224), 2560 29.0 ->
+// 22.9 (192), 3456 29.3 -> 26.5 (224); K 8192: M 1536 48.4 -> 40.9, 3456 96.7 -> 95.0; N 8192, K 2048 (GELU): M 512 21.1 -> 18.4, 1024 31.3 ->
+// 28.0, 1536 42.8 -> 40.4, 3456 94.9 -> 92.8; the other way N 2048, K 2048, M 2048 18.8 (256) against 22.8 (224) and 22.4 (192).
+constexpr int SPLIT_K_COST = 560, SPLIT_K_COST_PAIR = 760;
 struct GemmShape {
     bool pair;
     int split;
+    int width;   // columns of a tile
 };
-// The cheapest shape among those with `split` parts (0: any). max_clusters[1], [2]: resident clusters of 2 and 4 CTAs.
-inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int split, int sm_count, const int* max_clusters) {
+// The cheapest shape among those with `split` parts (0: any). max_clusters[1], [2]: resident clusters of 2 and 4 CTAs. any_width: the
+// epilogue has the narrow tiles (of a single matrix). unit: time of a k step, in eighths of the unit above.
+inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int split, int sm_count, const int* max_clusters, bool any_width = false) {
+    static constexpr struct { bool pair; int width, unit, max_split; } kinds[] = {{true, 256, 88, 2}, {true, 224, 78, 1}, {true, 192, 67, 1}, {false, 128, 64, 4}};
     long long best = -1;
-    GemmShape shape = {false, 1};
-    for (int pair = 1; pair >= 0; pair--) {
-        if (pair && (N % 256 || M <= 128)) continue;
-        const int tile = pair ? 256 : 128;
-        const long long tiles = (long long)((M + tile - 1) / tile) * ((N + tile - 1) / tile) * n_seg;
-        const long long unit = pair ? 11 : 8, groups = pair ? sm_count / 2 : sm_count;
-        for (int s = 1; s <= (pair ? 2 : 4); s *= 2) {
-            if ((split && s != split) || (s > 1 && (ksteps < 2 * s || tiles > max_clusters[pair ? s : s / 2]))) continue;
-            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + s - 1) / s) * unit + (s == 1 ? 0 : pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
-            if (best < 0 || cost < best) { best = cost; shape = {pair != 0, s}; }
+    GemmShape shape = {false, 1, 128};
+    for (const auto& kind : kinds) {
+        const bool narrow = kind.pair && kind.width != 256;
+        if (kind.pair && (M <= 128 || (narrow ? !any_width || n_seg > 1 : N % 256 != 0))) continue;
+        const int height = kind.pair ? 256 : 128;
+        const long long tiles = (long long)((M + height - 1) / height) * ((N + kind.width - 1) / kind.width) * n_seg;
+        const long long groups = kind.pair ? sm_count / 2 : sm_count;
+        for (int s = 1; s <= kind.max_split; s *= 2) {
+            if ((split && s != split) || (s > 1 && (ksteps < 2 * s || tiles > max_clusters[kind.pair ? s : s / 2]))) continue;
+            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + s - 1) / s) * kind.unit + (s == 1 ? 0 : kind.pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
+            if (best < 0 || cost < best) { best = cost; shape = {kind.pair, s, kind.width}; }
         }
     }
     return shape;
@@ -107,9 +117,9 @@ inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int sp
 // segments, for one and two as well: a split that would pay for a single projection only is left out (N 2048, K 2048: four parts up to
 // M 256, two up to M 512; up to M 128 two parts are left). What that costs the single call, head epilogue, device time: M 128
 // 9.1 us either way, M 256 10.2 -> 10.7, M 512 10.3 -> 11.1.
-inline GemmShape gemm_shape(int M, int N, long long ksteps, int n_seg, bool any_n_seg, int sm_count, const int* max_clusters) {
+inline GemmShape gemm_shape(int M, int N, long long ksteps, int n_seg, bool any_n_seg, int sm_count, const int* max_clusters, bool any_width = false) {
     const int split = any_n_seg ? gemm_cheapest(M, N, ksteps, 3, 0, sm_count, max_clusters).split : 0;
-    return gemm_cheapest(M, N, ksteps, n_seg, split, sm_count, max_clusters);
+    return gemm_cheapest(M, N, ksteps, n_seg, split, sm_count, max_clusters, any_width);
 }
 
 }  // namespace kb

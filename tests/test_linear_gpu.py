@@ -421,10 +421,10 @@ def test_narrow_outputs_of_the_store_epilogues(kb, N):
         _close(out, oracle.linear16(x, w, epi), K, f"N={N} epi {epi}", epi in (1, 2))
 
 
-@pytest.mark.parametrize("M,N", [(2561, 1920), (19001, 200)], ids=lambda v: str(v))
+@pytest.mark.parametrize("M,N", [(128, 38400), (2561, 1920), (19001, 200)], ids=lambda v: str(v))
 def test_more_than_two_tiles_per_thread_block(kb, M, N):
-    """Widths that 256 does not divide run one 128 x 128 tile per thread block: beyond 2 x 148 tiles a block comes back to its first
-    accumulator, which every epilogue warp has to have handed back. Fp64 reference of the same product, bounds as elsewhere."""
+    """Beyond two tiles a thread block comes back to its first accumulator, which every epilogue warp has to have handed back: 300 tiles
+    of 128 x 128, and two or three rounds of narrow tiles of CTA pairs. Fp64 reference of the same product, bounds as elsewhere."""
     from kiln_b200 import ops
     K = 64
     x, w = seeded(700, M, K, "f16"), seeded(701, N, K, "f16", 1.0 / np.sqrt(K))
@@ -432,6 +432,28 @@ def test_more_than_two_tiles_per_thread_block(kb, M, N):
     for epi in (ops.EPI_F32, ops.EPI_F16, ops.EPI_GELU16):
         r = torch.nn.functional.gelu(torch.from_numpy(ref)).numpy() if epi == ops.EPI_GELU16 else ref
         _close(_run(kb, x, w, epi), r, K, f"M={M} N={N} epi {epi}", epi != ops.EPI_F32)
+
+
+@pytest.mark.parametrize("M,N,K,epi", [(1281, 2048, 128, "RESID"), (1792, 2048, 192, "RESID"), (1300, 2048, 64, "F32"), (700, 1928, 64, "F16"), (400, 8192, 64, "GELU16"),
+                                       (257, 8000, 128, "GELU16"), (1537, 2056, 64, "F32")], ids=str)
+def test_narrow_tiles(kb, M, N, K, epi):
+    """Tiles of 224 and 192 columns: last row and column tiles that are cut, every epilogue that has them, a second product; nothing
+    written outside the matrix. Fp64 reference of the same products, bounds as elsewhere."""
+    from kiln_b200 import ops
+    e = getattr(ops, "EPI_" + epi)
+    x, w = seeded(710, M, K, "f16"), seeded(711, N, K, "f16", 1.0 / np.sqrt(K))
+    t, b = seeded(712, M, 40, "f16"), seeded(713, N, 40, "f16", 1.0 / np.sqrt(40))
+    gate = oracle.randn(714, N).astype(np.float32) if epi == "RESID" else None
+    resid = oracle.randn(715, M * N).reshape(M, N).astype(np.float32) if epi == "RESID" else None
+    for lora in (False, True):
+        kw = {"lora": (dev(t, "f16"), dev(b, "f16"))} if lora else {}
+        ref = x.astype(np.float64) @ w.astype(np.float64).T + (t.astype(np.float64) @ b.astype(np.float64).T if lora else 0.0)
+        if epi == "GELU16":
+            ref = torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()
+        if epi == "RESID":
+            ref = resid + gate * ref
+        out = _run(kb, x, w, e, gate=gate, resid=resid, ldc_pad=64, **kw)
+        _close(out, ref, K + 40, f"{epi} {M}x{N}x{K} lora {lora}", epi in ("F16", "GELU16"))
 
 
 def test_lora_argument_errors(kb):

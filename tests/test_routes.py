@@ -30,11 +30,14 @@ def rules(tmp_path_factory):
                    'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n'
                    'extern "C" int gemm(int M, int N, int ksteps, int n_seg, int any, int mc2, int mc4) {\n'
                    '    const int mc[3] = {0, mc2, mc4}; const kb::GemmShape g = kb::gemm_shape(M, N, ksteps, n_seg, any, 148, mc); return g.pair * 8 + g.split; }\n'
+                   'extern "C" int width(int M, int N, int ksteps, int any) {\n'
+                   '    const int mc[3] = {0, 74, 37}; return kb::gemm_shape(M, N, ksteps, 1, false, 148, mc, any).width; }\n'
                    'extern "C" int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {\n'
                    '    return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth}); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
     lib = ctypes.CDLL(str(d / "routes.so"))
     lib.survives.argtypes = [ctypes.c_size_t] * 7
+    lib.width.argtypes = [ctypes.c_int] * 4
     return lib
 
 
@@ -89,3 +92,15 @@ def test_raw_q_needs_an_output_that_leaves_it_alone(rules):
                 assert got == (in_place or not (q & o)), (stride, width, owidth, o0 - q0)
             else:                                              # different strides: never wrongly allowed, and allowed when the ranges are apart
                 assert not (got and q & o) and (got or not (min(o) > max(q) or min(q) > max(o)))
+
+
+def test_narrow_gemm_tiles_where_they_measured_faster(rules):
+    """Width of the tiles against device times on a B200 (us): 256, 224 and 192 columns forced in turn."""
+    for M, N, ksteps, times in [(1280, 2048, 32, (18.8, 16.4, 14.9)), (1536, 2048, 32, (18.8, 16.6, 15.1)), (1792, 2048, 32, (18.5, 16.6, 21.6)), (2048, 2048, 32, (18.8, 22.8, 22.4)),
+                                (2304, 2048, 32, (19.0, 25.3, 22.7)), (2560, 2048, 32, (29.0, 25.5, 22.9)), (3456, 2048, 32, (29.3, 26.5, 30.4)), (4096, 2048, 32, (29.8, 33.7, 31.5)),
+                                (1536, 2048, 128, (48.4, 43.2, 40.9)), (3456, 2048, 128, (96.7, 95.0, 112.0)), (4096, 2048, 128, (104.4, 124.7, 119.7)),
+                                (512, 8192, 32, (21.1, 18.4, 25.1)), (1024, 8192, 32, (31.3, 28.0, 33.9)), (1536, 8192, 32, (42.8, 40.4, 46.0)), (2304, 8192, 32, (59.2, 63.1, 67.7)),
+                                (3456, 8192, 32, (94.9, 92.8, 103.9)), (4096, 8192, 32, (104.0, 106.7, 118.0))]:
+        assert rules.width(M, N, ksteps, 1) == (256, 224, 192)[times.index(min(times))], (M, N, ksteps)
+        assert rules.width(M, N, ksteps, 0) in (128, 256)            # the head epilogue has no narrow tiles
+    assert rules.width(128, 8192, 32, 1) == 128
