@@ -204,10 +204,28 @@ struct PrepBatch {
         sg.in = in; sg.out = out; sg.w = static_cast<const __nv_bfloat16*>(w); sg.cos_t = c; sg.sin_t = s;
         sg.rows = rows; sg.ld_in = ld_in; sg.ld_out = ld_out; sg.T = T > 0 ? T : 1;
         sg.block0 = pp.blocks;
-        const int per_block = c ? PREP_ITEMS_PER_BLOCK_ROPE : PREP_ITEMS_PER_BLOCK;
-        pp.blocks += (unsigned)(((long long)rows * pp.H + per_block - 1) / per_block);
+        pp.blocks += (unsigned)((rows + (long long)PREP_WARPS - 1) / PREP_WARPS);
+    }
+    long long rows() const {
+        long long n = 0;
+        for (int i = 0; i < pp.nseg; i++) n += pp.seg[i].rows;
+        return n;
     }
 };
+
+template <typename InT, typename OutT>
+int launch_prep_t(DeviceState* st, const PrepBatch& pb, cudaStream_t stream) {
+    // Pieces per lane (prep.cuh has what they measured): four of 16 bytes, two of 32; one where all of it is a few rows, as a lane with
+    // less to do is done sooner
+    constexpr int MANY = sizeof(InT) == 2 ? 4 : 2;
+    bool rope = false;
+    for (int i = 0; i < pb.pp.nseg; i++) rope = rope || pb.pp.seg[i].cos_t;
+    const int np = rope || pb.rows() * pb.pp.H >= 64LL * st->sm_count ? MANY : 1;
+    const int groups = (pb.pp.H + 2 * np - 1) / (2 * np);
+    const dim3 grid(pb.pp.blocks, (unsigned)(groups < 65535 ? groups : 65535)), block(PREP_THREADS);
+    if (np == 1) return launch_dependent(qk_prep_kernel<InT, OutT, 1>, grid, block, 0, stream, nullptr, pb.pp);
+    return launch_dependent(qk_prep_kernel<InT, OutT, MANY>, grid, block, 0, stream, nullptr, pb.pp);
+}
 
 int launch_prep(DeviceState* st, const PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {
     if (pb.pp.blocks == 0) {
@@ -216,13 +234,14 @@ int launch_prep(DeviceState* st, const PrepBatch& pb, int in_dtype, int out_dtyp
         return KB_OK;
     }
     ProfScope ps(st, KB_PROF_NORM_ROPE, stream);
-    const unsigned grid = pb.pp.blocks;
-#define KB_PREP(IN, OUT) launch_dependent(qk_prep_kernel<IN, OUT>, dim3(grid), dim3(256), 0, stream, nullptr, pb.pp)
-    if (out_dtype == KB_F32) return KB_PREP(float, float);   // in-place fp32 norm / RoPE as the engine's own ops do (validated by the caller)
+    if (out_dtype == KB_F32) return launch_prep_t<float, float>(st, pb, stream);   // in-place fp32 norm / RoPE as the engine's own ops do (validated by the caller)
     if (out_dtype == KB_F16)
-        return in_dtype == KB_F16 ? KB_PREP(__half, __half) : in_dtype == KB_BF16 ? KB_PREP(__nv_bfloat16, __half) : KB_PREP(float, __half);
-    return in_dtype == KB_F16 ? KB_PREP(__half, __nv_bfloat16) : in_dtype == KB_BF16 ? KB_PREP(__nv_bfloat16, __nv_bfloat16) : KB_PREP(float, __nv_bfloat16);
-#undef KB_PREP
+        return in_dtype == KB_F16    ? launch_prep_t<__half, __half>(st, pb, stream)
+               : in_dtype == KB_BF16 ? launch_prep_t<__nv_bfloat16, __half>(st, pb, stream)
+                                     : launch_prep_t<float, __half>(st, pb, stream);
+    return in_dtype == KB_F16    ? launch_prep_t<__half, __nv_bfloat16>(st, pb, stream)
+           : in_dtype == KB_BF16 ? launch_prep_t<__nv_bfloat16, __nv_bfloat16>(st, pb, stream)
+                                 : launch_prep_t<float, __nv_bfloat16>(st, pb, stream);
 }
 
 template <int MODE, typename OutT>
@@ -649,10 +668,10 @@ int launch_gemm_shape(DeviceState* st, const CUtensorMap& ta, const GemmMaps& ma
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = ctas; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
     ProfScope ps(st, KB_PROF_LINEAR, stream);
-    auto kernel = gemm16_kernel<EPI, PAIR, false, BN>;
+    const dim3 grid((unsigned)(groups * ctas)), block(G_THREADS);
     if constexpr (BN == (PAIR ? 256 : 128))
-        if (split_k > 1) kernel = gemm16_kernel<EPI, PAIR, true, BN>;
-    return launch_dependent(kernel, dim3((unsigned)(groups * ctas)), dim3(G_THREADS), G_SMEM, stream, &cluster, ta, maps, p);
+        if (split_k > 1) return launch_dependent(gemm16_kernel<EPI, PAIR, true, BN>, grid, block, G_SMEM, stream, &cluster, ta, maps, p);
+    return launch_dependent(gemm16_kernel<EPI, PAIR, false, BN>, grid, block, G_SMEM, stream, &cluster, ta, maps, p);
 }
 
 template <int EPI>

@@ -14,86 +14,63 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "ptx.cuh"
 
 namespace kb {
 
-// eight consecutive elements as fp32
+// eight consecutive elements as fp32, and as they lie in memory
 struct F8 { float v[8]; };
-struct F4 { float v[4]; };
-template <typename T> struct Io;
-template <> struct Io<float> {
-    static __device__ __forceinline__ F4 ld4(const float* p) { const float4 a = *reinterpret_cast<const float4*>(p); return F4{{a.x, a.y, a.z, a.w}}; }
-    static __device__ __forceinline__ void st4(float* p, const F4& r) { *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]); }
-    static __device__ __forceinline__ F8 ld8(const float* p) {
-        F8 r;
-        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-        r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w; r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
+template <typename T> struct Raw8 { uint4 u[sizeof(T) / 2]; };
+template <typename T> struct Io {
+    static __device__ __forceinline__ Raw8<T> raw8(const T* p) {
+        Raw8<T> r;
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T) / 2; i++) r.u[i] = reinterpret_cast<const uint4*>(p)[i];
         return r;
     }
-    static __device__ __forceinline__ void st8(float* p, const F8& r) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(r.v[4], r.v[5], r.v[6], r.v[7]);
-    }
-};
-template <> struct Io<__half> {
-    static __device__ __forceinline__ F4 ld4(const __half* p) {
-        const uint2 u = *reinterpret_cast<const uint2*>(p);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-        return F4{{a.x, a.y, b.x, b.y}};
-    }
-    static __device__ __forceinline__ void st4(__half* p, const F4& r) {
-        const __half2 a = __floats2half2_rn(r.v[0], r.v[1]), b = __floats2half2_rn(r.v[2], r.v[3]);
-        *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-    }
-    static __device__ __forceinline__ F8 ld8(const __half* p) {
-        F8 r;
-        const uint4 u = *reinterpret_cast<const uint4*>(p);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    static __device__ __forceinline__ F8 f8(const Raw8<T>& r) {
+        F8 f;
+        if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            r.v[2 * i] = f.x; r.v[2 * i + 1] = f.y;
-        }
-        return r;
-    }
-    static __device__ __forceinline__ void st8(__half* p, const F8& r) {
-        uint32_t w[4];
+            for (int i = 0; i < 2; i++) {
+                f.v[4 * i] = __uint_as_float(r.u[i].x); f.v[4 * i + 1] = __uint_as_float(r.u[i].y);
+                f.v[4 * i + 2] = __uint_as_float(r.u[i].z); f.v[4 * i + 3] = __uint_as_float(r.u[i].w);
+            }
+        } else {
+            const uint32_t w[4] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const __half2 h = __floats2half2_rn(r.v[2 * i], r.v[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            for (int i = 0; i < 4; i++) {
+                if constexpr (std::is_same<T, __nv_bfloat16>::value) {   // a bf16 is the top half of an fp32
+                    f.v[2 * i] = __uint_as_float(w[i] << 16); f.v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                } else {
+                    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                    f.v[2 * i] = h.x; f.v[2 * i + 1] = h.y;
+                }
+            }
         }
-        *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+        return f;
     }
-};
-template <> struct Io<__nv_bfloat16> {
-    static __device__ __forceinline__ F4 ld4(const __nv_bfloat16* p) {
-        const uint2 u = *reinterpret_cast<const uint2*>(p);
-        return F4{{__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u)}};
-    }
-    static __device__ __forceinline__ void st4(__nv_bfloat16* p, const F4& r) {
-        const __nv_bfloat162 a = __floats2bfloat162_rn(r.v[0], r.v[1]), b = __floats2bfloat162_rn(r.v[2], r.v[3]);
-        *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-    }
-    static __device__ __forceinline__ F8 ld8(const __nv_bfloat16* p) {
-        F8 r;
-        const uint4 u = *reinterpret_cast<const uint4*>(p);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    static __device__ __forceinline__ F8 ld8(const T* p) { return f8(raw8(p)); }
+    static __device__ __forceinline__ void st8(T* p, const F8& f) {
+        if constexpr (sizeof(T) == 4) {
+            reinterpret_cast<float4*>(p)[0] = make_float4(f.v[0], f.v[1], f.v[2], f.v[3]);
+            reinterpret_cast<float4*>(p)[1] = make_float4(f.v[4], f.v[5], f.v[6], f.v[7]);
+        } else {
+            uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {   // a bf16 is the top half of an fp32
-            r.v[2 * i] = __uint_as_float(w[i] << 16); r.v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            for (int i = 0; i < 4; i++) {
+                if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(f.v[2 * i], f.v[2 * i + 1]);
+                    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                } else {
+                    const __half2 h = __floats2half2_rn(f.v[2 * i], f.v[2 * i + 1]);
+                    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+            }
+            *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        return r;
-    }
-    static __device__ __forceinline__ void st8(__nv_bfloat16* p, const F8& r) {
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(r.v[2 * i], r.v[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 };
 
@@ -123,87 +100,101 @@ __global__ void zero_words_kernel(unsigned int* ptr, int n) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) ptr[i] = 0u;
 }
 
-// Measured on B200: a plain one-16-byte-load-per-thread conversion runs at the speed of a device copy
-// (101 MB in 18.6 us), and unrolling for more loads in flight buys nothing; what costs bandwidth is
-// occupancy and narrow accesses. So: no loop, one pass, 16-byte accesses for 16-bit data everywhere, and a thread
-// block belongs to exactly one tensor so the tensor lookup is block-uniform.
-//   without RoPE: one (row, head) per half-warp, lane `sub` holds elements [8 sub, 8 sub + 8);
-//   with RoPE   : one (row, head) per quarter-warp, lane `sub` holds elements [8 sub, 8 sub + 8) AND their rotation
-//                 partners [64 + 8 sub, ...), so the rotation needs no shuffle and each table entry is loaded once.
-constexpr int PREP_ITEMS_PER_BLOCK = 16;        // 256 threads / 16 lanes
-constexpr int PREP_ITEMS_PER_BLOCK_ROPE = 32;   // 256 threads / 8 lanes
+// A warp takes 2 NP heads of a row: all its loads first (NP pieces of eight elements per lane), then head after head.
+//   without RoPE: two heads side by side, lane `sub` of 16 holds elements [8 sub, 8 sub + 8);
+//   with RoPE   : four heads side by side, lane `sub` of 8 holds elements [8 sub, 8 sub + 8) AND their rotation partners [64 + 8 sub, ...),
+//                 so the rotation needs no shuffle, and a lane's 8 + 8 table values serve all its heads (NP = 1: never with RoPE).
+// Bound by memory: the rows come from HBM, the 16-bit copies go to L2. NP (launch_prep_t) sets what a lane has in flight against how many
+// lanes there are. Measured on B200 with three sets of inputs in turn, whole attention call, one piece per lane (two with RoPE) -> this:
+// self-attention with norm and RoPE, bf16, 256 tokens 11.1 -> 10.0 us, 1000 21.6 -> 20.7, 1536 39.5 -> 38.0, 4096 144.5 -> 141.2 (NP 2: 10.2,
+// 21.1, 38.5, 142.1; NP 8: 10.9, 21.7, 38.2, 143.8); fp32, whose pieces are 32 bytes, NP 2: 1000 tokens 23.4 -> 23.4, gradients at 1024
+// 101.7 -> 100.0 (NP 4: 23.5, 100.0; 4096 tokens 151.8 -> 152.6); a context of 512 x 1024 fp32 for cross_kv 11.1 us with NP 1, 11.5 with 2.
+constexpr int PREP_WARPS = 4;                               // rows per thread block; blockIdx.y: which 2 NP heads of them
+constexpr int PREP_THREADS = 32 * PREP_WARPS;
 
-template <typename InT, typename OutT>
-__global__ void __launch_bounds__(256)
+template <typename InT, typename OutT, int NP>
+__global__ void __launch_bounds__(PREP_THREADS)
 qk_prep_kernel(const __grid_constant__ PrepParams pp) {
+    constexpr int HEADS = 2 * NP, NI = NP > 1 ? NP / 2 : 1;
     pdl_launch();
     pdl_wait();
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < pp.zero_n; i += 256) pp.zero_ptr[i] = 0u;
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < pp.zero_n; i += PREP_THREADS) pp.zero_ptr[i] = 0u;
     int si = 0;
 #pragma unroll
     for (int i = 1; i < 5; i++)
         if (i < pp.nseg && blockIdx.x >= pp.seg[i].block0) si = i;
     const PrepSeg& sg = pp.seg[si];
-    if (sg.cos_t) {
-        const int sub = threadIdx.x & 7;
-        const long long item = (long long)(blockIdx.x - sg.block0) * PREP_ITEMS_PER_BLOCK_ROPE + (threadIdx.x >> 3);
-        const bool live = item < (long long)sg.rows * pp.H;  // uniform across a quarter-warp
-        const int r = live ? (int)(item / pp.H) : 0, h = live ? (int)(item % pp.H) : 0;
-        F8 a, b;
+    const int lane = threadIdx.x & 31;
+    const unsigned row = PREP_WARPS * (blockIdx.x - sg.block0) + (threadIdx.x >> 5);
+    if (row >= (unsigned)sg.rows) return;
+    const int r = (int)row;
+    const InT* const src = static_cast<const InT*>(sg.in) + (size_t)r * sg.ld_in;
+    OutT* const dst = static_cast<OutT*>(sg.out) + (size_t)r * sg.ld_out;
+    for (int h0 = (int)blockIdx.y * HEADS; h0 < pp.H; h0 += (int)gridDim.y * HEADS) {   // one round up to 65535 groups of heads
+        if (NP > 1 && sg.cos_t) {
+            const int sub = lane & 7, hl = h0 + (lane >> 3);     // heads hl, hl + 4, ...
+            Raw8<InT> ra[NI], rb[NI];
 #pragma unroll
-        for (int e = 0; e < 8; e++) a.v[e] = b.v[e] = 0.f;
-        const InT* src = static_cast<const InT*>(sg.in) + (size_t)r * sg.ld_in + h * 128 + 8 * sub;
-        if (live) { a = Io<InT>::ld8(src); b = Io<InT>::ld8(src + 64); }
-        if (sg.w) {
-            float ss = 0.f;
+            for (int i = 0; i < NI; i++) {
+                const int h = min(hl + 4 * i, pp.H - 1);         // past the last head: read again, not stored
+                ra[i] = Io<InT>::raw8(src + h * 128 + 8 * sub);
+                rb[i] = Io<InT>::raw8(src + h * 128 + 64 + 8 * sub);
+            }
+            const size_t tr = (size_t)(r % sg.T) * 64 + 8 * sub;
+            const F8 c = Io<float>::ld8(sg.cos_t + tr), s = Io<float>::ld8(sg.sin_t + tr);
+            Raw8<__nv_bfloat16> wa, wb;
+            if (sg.w) { wa = Io<__nv_bfloat16>::raw8(sg.w + 8 * sub); wb = Io<__nv_bfloat16>::raw8(sg.w + 64 + 8 * sub); }
 #pragma unroll
-            for (int e = 0; e < 8; e++) ss += a.v[e] * a.v[e] + b.v[e] * b.v[e];
+            for (int i = 0; i < NI; i++) {
+                F8 a = Io<InT>::f8(ra[i]), b = Io<InT>::f8(rb[i]);
+                if (sg.w) {
+                    float ss = 0.f;
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
-            const F8 wa = Io<__nv_bfloat16>::ld8(sg.w + 8 * sub), wb = Io<__nv_bfloat16>::ld8(sg.w + 64 + 8 * sub);
+                    for (int e = 0; e < 8; e++) ss += a.v[e] * a.v[e] + b.v[e] * b.v[e];
 #pragma unroll
-            for (int e = 0; e < 8; e++) { a.v[e] = a.v[e] * rs * wa.v[e]; b.v[e] = b.v[e] * rs * wb.v[e]; }
+                    for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
+                    const F8 fa = Io<__nv_bfloat16>::f8(wa), fb = Io<__nv_bfloat16>::f8(wb);
+#pragma unroll
+                    for (int e = 0; e < 8; e++) { a.v[e] = a.v[e] * rs * fa.v[e]; b.v[e] = b.v[e] * rs * fb.v[e]; }
+                }
+                F8 x, y;
+#pragma unroll
+                for (int e = 0; e < 8; e++) {                    // engine/src/kernels.cu:769-771
+                    x.v[e] = a.v[e] * c.v[e] - b.v[e] * s.v[e];
+                    y.v[e] = b.v[e] * c.v[e] + a.v[e] * s.v[e];
+                }
+                if (hl + 4 * i < pp.H) {
+                    Io<OutT>::st8(dst + (hl + 4 * i) * 128 + 8 * sub, x);
+                    Io<OutT>::st8(dst + (hl + 4 * i) * 128 + 64 + 8 * sub, y);
+                }
+            }
+            continue;
         }
-        const size_t tr = (size_t)(r % sg.T) * 64 + 8 * sub;
-        const F8 c = Io<float>::ld8(sg.cos_t + tr), s = Io<float>::ld8(sg.sin_t + tr);
-        F8 x, y;
+        const int sub = lane & 15, hl = h0 + (lane >> 4);        // heads hl, hl + 2, ...
+        Raw8<InT> rx[NP];
 #pragma unroll
-        for (int e = 0; e < 8; e++) {                         // engine/src/kernels.cu:769-771
-            x.v[e] = a.v[e] * c.v[e] - b.v[e] * s.v[e];
-            y.v[e] = b.v[e] * c.v[e] + a.v[e] * s.v[e];
+        for (int i = 0; i < NP; i++) rx[i] = Io<InT>::raw8(src + min(hl + 2 * i, pp.H - 1) * 128 + 8 * sub);
+        Raw8<__nv_bfloat16> w;
+        if (sg.w) w = Io<__nv_bfloat16>::raw8(sg.w + 8 * sub);
+#pragma unroll
+        for (int i = 0; i < NP; i++) {
+            F8 x = Io<InT>::f8(rx[i]);
+            if (sg.w) {                                           // block-uniform
+                float ss = 0.f;
+#pragma unroll
+                for (int e = 0; e < 8; e++) ss += x.v[e] * x.v[e];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
+                const F8 fw = Io<__nv_bfloat16>::f8(w);
+#pragma unroll
+                for (int e = 0; e < 8; e++) x.v[e] = x.v[e] * rs * fw.v[e];
+            }
+            if (hl + 2 * i < pp.H) Io<OutT>::st8(dst + (hl + 2 * i) * 128 + 8 * sub, x);
         }
-        if (live) {
-            OutT* dst = static_cast<OutT*>(sg.out) + (size_t)r * sg.ld_out + h * 128 + 8 * sub;
-            Io<OutT>::st8(dst, x);
-            Io<OutT>::st8(dst + 64, y);
-        }
-        return;
     }
-    const int sub = threadIdx.x & 15;
-    const long long item = (long long)(blockIdx.x - sg.block0) * PREP_ITEMS_PER_BLOCK + (threadIdx.x >> 4);
-    const bool live = item < (long long)sg.rows * pp.H;      // uniform across a half-warp
-    const int r = live ? (int)(item / pp.H) : 0, h = live ? (int)(item % pp.H) : 0;
-    // no RoPE: lane `sub` holds elements [8 sub, 8 sub + 8) (16-byte accesses for 16-bit data)
-    F8 x;
-    if (live) x = Io<InT>::ld8(static_cast<const InT*>(sg.in) + (size_t)r * sg.ld_in + h * 128 + 8 * sub);
-    else {
-#pragma unroll
-        for (int e = 0; e < 8; e++) x.v[e] = 0.f;
-    }
-    if (sg.w) {                                               // block-uniform
-        float ss = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; e++) ss += x.v[e] * x.v[e];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
-        const F8 w = Io<__nv_bfloat16>::ld8(sg.w + 8 * sub);
-#pragma unroll
-        for (int e = 0; e < 8; e++) x.v[e] = x.v[e] * rs * w.v[e];
-    }
-    if (live) Io<OutT>::st8(static_cast<OutT*>(sg.out) + (size_t)r * sg.ld_out + h * 128 + 8 * sub, x);
 }
 
 }  // namespace kb

@@ -323,6 +323,38 @@ def test_qk_prep_vs_reference_kernels_golden(kb, golden):
     assert kb.check_status() == 0
 
 
+@pytest.mark.parametrize("H", [1, 3, 8, 9, 17])
+@pytest.mark.parametrize("rows", [1, 6, 333, 3001])
+def test_qk_prep_head_and_row_remainders(kb, H, rows):
+    """Heads that no group of 2, 4 or 8 divides, a last thread block with fewer rows, tables shorter than the rows, every form of the
+    kernel, padding left alone. Reference in float64; bounds: one rounding of the result, and fp32 arithmetic in front of it (norm: a
+    sum of 128 squares, then three products and a sum: below 2^-19 of the largest value of a row)."""
+    g = torch.Generator(device="cuda").manual_seed(rows * 31 + H)
+    T = max(1, rows - 2)
+    w = (1 + 0.1 * torch.randn(128, generator=g, device="cuda")).bfloat16()
+    ang = torch.rand(T, 64, generator=g, device="cuda") * 6.28
+    cos, sin = ang.cos(), ang.sin()
+    for it, ot in ((torch.float16,) * 2, (torch.bfloat16, torch.float16), (torch.float32, torch.float16), (torch.float32, torch.float32), (torch.float32, torch.bfloat16)):
+        x = torch.randn(rows, H * 128 + 8, generator=g, device="cuda").to(it)[:, :H * 128]
+        for norm in (False, True):
+            for rope in (False, True):
+                y = x.double().reshape(rows, H, 128)
+                if norm:
+                    y = y * torch.rsqrt((y * y).mean(-1, keepdim=True) + 1e-6) * w.double()
+                if rope:
+                    r = torch.arange(rows, device="cuda") % T
+                    c, s = cos.double()[r][:, None], sin.double()[r][:, None]
+                    a, b = y[..., :64], y[..., 64:]
+                    y = torch.cat([a * c - b * s, b * c + a * s], -1)
+                full = torch.full((rows, H * 128 + 8), float("nan"), device="cuda", dtype=ot)
+                kb.qk_prep(full[:, :H * 128], x, rows, H, T, w=w if norm else None, rope_cos=cos if rope else None, rope_sin=sin if rope else None)
+                assert kb.check_status() == 0 and torch.isnan(full[:, H * 128:].float()).all()
+                y = y.reshape(rows, H * 128)
+                ulp = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[ot]
+                bound = y.abs() * ulp + y.abs().amax(1, keepdim=True) * 2.0 ** -19 + 2.0 ** -24
+                assert ((full[:, :H * 128].double() - y).abs() <= bound).all(), (it, ot, norm, rope)
+
+
 def test_self_config4_full_size(kb):
     """Benchmark configuration 4: bf16, B=2, T=3456 (48x72 patches), per-head Q/K RMSNorm (1 + N(0,0.02)) and 3D RoPE."""
     Hp, Wp, B, H, kind = 48, 72, 2, 16, "bf16"
