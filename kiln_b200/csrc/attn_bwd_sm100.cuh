@@ -11,9 +11,9 @@
 // D_i = sum_d dO[i, d] O[i, d] (= sum_j P_ij dP_ij, what k_dsoftmax sums; dO as the tensor cores see it, O in fp32), and this
 // file's kernel, whose thread blocks play one of two roles:
 //
-//   BWD_DKV  one thread block per (key block j, head, image), query blocks i streamed through a two-stage ring:
+//   BWD_DKV  one thread block per (key block j, head, image), query blocks i streamed through a ring:
 //              S^T  = K_j Q_i^T            dP^T = V_j dO_i^T                      (two SS products into TMEM)
-//              P^T  = 2^(c S^T - L_i)      dS^T = P^T (dP^T - D_i)                (softmax warps; fp16, written over S^T / dP^T)
+//              P^T  = 2^(c S^T - L_i)      dS^T = P^T (dP^T - D_i)                (softmax warps; fp16, written over dP^T)
 //              dV_j += P^T dO_i            dK_j += dS^T Q_i                       (A operand from TMEM, B the same shared-memory
 //                                                                                  tiles read MN-major)
 //   BWD_DQ   one thread block per (query block i, head, image), key blocks j streamed:
@@ -26,19 +26,20 @@
 // adds nothing to dK / dV, a zero K row adds nothing to dQ, so ragged sizes need no masking - only finite statistics, which
 // the stats array (padded to whole query blocks) always holds.
 //
-// TMEM (512 columns): T0 [0,128) S or S^T, T1 [128,256) dP or dP^T, acc0 [256,384), acc1 [384,512). Measured on B200 (clock
-// stamps in a private build, before the issuing thread was an elected one): the kernel is bound by the thread that issues the
-// products - a step of BWD_DKV took 3300 cycles, of which its four products took 3030 (~95 per instruction against 64 in the tensor
-// pipe; an SS product costs the same with half the N, and taking its A operand from TMEM changed nothing), the softmax warps ~2000
-// (phase 1 1400, phase 2 600). So the products keep N = 128 and the step is software-pipelined across the two products instead:
-//   softmax phase 1: S^T ready -> P^T = 2^(c S^T - L) (kept in registers), fp16 P^T stored, "P0" signalled;
-//   softmax phase 2: dP^T ready -> dS^T = P^T (dP^T - D) stored, "P1" signalled;
-//   issue order:     [P0] dV += P^T dO | S^T of the next step | [P1] dK += dS^T Q | dP^T of the next step
-// so that phase 1 of the next step runs under the dK and dP^T products and phase 2 under the dV and S^T products of the step
-// after (in-order execution of one thread's tcgen05.mma keeps a product from overwriting what the one before still reads).
-// BWD_DQ has one accumulating product: S of the next step is issued as soon as the softmax warps have read S (phase 1
-// signals that), under phase 2. Each of the eight softmax warps (lane quarter x column half) owns 64 columns of T0 / T1 and
-// writes its fp16 results over the first 32 of those same columns, so no warp overwrites what another still has to read.
+// TMEM (512 columns): T0 [0,128) S or S^T, T1 [128,256) dP or dP^T, acc0 [256,384), acc1 [384,512) (BWD_DQ: its first half holds dS).
+// A step is a chain through the softmax warps (~2100 cycles: 1024 of them the MUFU unit's) next to four (BWD_DQ: three) products of 512
+// cycles, so nothing but the products that have to may stand in that chain:
+//   softmax phase 1: S^T read (T0 is free: the next step's S^T may go), P^T = 2^(c S^T - L) kept in registers;
+//   softmax phase 2: dP^T read, P^T stored as fp16 over it ("READ1": dV may go), dS^T = P^T (dP^T - D) stored over it too ("DS");
+//   issue order:     [READ0] S^T of the next step | [READ1] dV += P^T dO | [DS] dK += dS^T Q | dP^T of the next step
+// (in-order execution of one thread's tcgen05.mma keeps dP^T from overwriting what dV and dK still read). Phase 1 of the next step
+// runs under dV, dK and dP^T. Each of the eight softmax warps (lane quarter x column half) owns 64 columns of T0 / T1 and writes its
+// fp16 results over those same columns, so no warp overwrites what another still has to read. In BWD_DQ dS has columns of its own, and
+// dP of the next step need not wait for dQ. The streamed tiles have three and two stages: with two of each the tile of the next S was
+// asked for when the step in front had freed it and came after it was wanted.
+// Measured on B200 by clock stamps, cycles per step: P^T stored over S^T, whose next product therefore waited for dV, and two stages: BWD_DKV
+// 3050, BWD_DQ 2780 -> 2580 and 2080 (with S^T and dP^T in one place in turn, so that S^T waited for dP^T to be read: 3090). An SS product costs the
+// same with half the N, and taking its A operand from TMEM changed nothing.
 #pragma once
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -51,8 +52,10 @@ namespace kb {
 constexpr int BWD_DKV = 0, BWD_DQ = 1;
 constexpr int BWD_THREADS = 384;                              // warps 0-7 softmax / epilogue, 8 MMA issue, 9 TMA loads, 10-11 idle
 constexpr int BWD_SOFTMAX_REGS = 224, BWD_OTHER_REGS = 56;    // 384 x 168 = 256 x 224 + 128 x 56
-constexpr int BWD_STAGE_BYTES = 2 * TILE_BYTES + 1024;        // two streamed tiles + the statistics of a query block
-constexpr int BWD_SMEM = 2 * TILE_BYTES + 2 * BWD_STAGE_BYTES + 1024;   // resident pair, two stages, control block
+constexpr int BWD_X0_STAGES = 3, BWD_X1_STAGES = 2;           // of the streamed tiles: X0 (Q_i or K_j), X1 (dO_i or V_j, with the statistics)
+constexpr int BWD_STATS_BYTES = 1024;                         // the statistics of a query block
+constexpr int BWD_SMEM = (2 + BWD_X0_STAGES + BWD_X1_STAGES) * TILE_BYTES + BWD_X1_STAGES * BWD_STATS_BYTES + 1024;   // resident pair, rings, control block
+static_assert(BWD_SMEM <= 232448, "shared memory per thread block on sm_100");
 
 struct BwdParams {
     int B, H, Tq, Tk;
@@ -66,7 +69,9 @@ struct BwdParams {
     uint32_t* status;
 };
 
-enum { BB_RES = 0, BB_XFULL = 1, BB_XEMPTY = 3, BB_TFULL = 5, BB_PFULL = 7, BB_ACC = 9, BB_COUNT = 10 };   // TFULL/PFULL: [0] first product / phase 1, [1] second
+// T is the first product (S or S^T) or the second (dP or dP^T) of a step. READ, DS: one arrival per softmax warp
+enum { BB_RES = 0, BB_X0FULL = 1, BB_X0EMPTY = BB_X0FULL + BWD_X0_STAGES, BB_X1FULL = BB_X0EMPTY + BWD_X0_STAGES, BB_X1EMPTY = BB_X1FULL + BWD_X1_STAGES,
+       BB_TFULL = BB_X1EMPTY + BWD_X1_STAGES, BB_READ = BB_TFULL + 2, BB_DS = BB_READ + 2, BB_DSFREE, BB_ACC, BB_COUNT };
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -85,11 +90,13 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         return;
     }
     const uint32_t sR0 = base, sR1 = base + TILE_BYTES;            // resident: K_j, V_j (BWD_DKV) or Q_i, dO_i (BWD_DQ)
-    const uint32_t sX = base + 2 * TILE_BYTES;                     // stages: X0 (Q_i or K_j), X1 (dO_i or V_j), statistics
-    uint8_t* const ctrl = smem_raw + 2 * TILE_BYTES + 2 * BWD_STAGE_BYTES;
-    const uint32_t bars = sX + 2 * BWD_STAGE_BYTES;
-    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 128);
-    volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(ctrl + 132);
+    constexpr int OFF_X1 = (2 + BWD_X0_STAGES) * TILE_BYTES, OFF_STATS = OFF_X1 + BWD_X1_STAGES * TILE_BYTES;
+    const uint32_t sX0 = base + 2 * TILE_BYTES, sX1 = base + OFF_X1;
+    uint8_t* const ctrl = smem_raw + OFF_STATS + BWD_X1_STAGES * BWD_STATS_BYTES;
+    const uint32_t bars = smem_u32(ctrl);
+    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 256);
+    volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(ctrl + 260);
+    static_assert(BB_COUNT * 8 <= 256, "barriers in front of the shared words");
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -98,7 +105,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
     const int n_it = MODE == BWD_DKV ? min(nqb - i0, p.q_per) : (p.Tk + BN - 1) / BN;
 
     if (tid == 0) {
-        for (int i = 0; i < BB_COUNT; i++) mbar_init(bar(i), (i == BB_PFULL || i == BB_PFULL + 1) ? 8u : 1u);   // P: one arrival per softmax warp
+        for (int i = 0; i < BB_COUNT; i++) mbar_init(bar(i), (i == BB_READ || i == BB_READ + 1 || i == BB_DS) ? 8u : 1u);   // one arrival per softmax warp
         *abort_flag = 0u;
         mbar_fence_init();
         fence_proxy_async_smem();
@@ -113,6 +120,10 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
     __syncthreads();
     tc_fence_after();
     constexpr uint32_t tmem_base = 0;                             // see TMEM_ALL_COLUMNS and elect_one
+    constexpr uint32_t T0 = 0u, T1 = 128u;
+    // fp16 operands: BWD_DKV: a warp stores its P^T and its dS^T over its own 64 columns of dP^T, which it has read (contraction elements
+    // [64 hh, 64 hh + 64) in columns [64 hh, 64 hh + 32) and [64 hh + 32, 64 hh + 64)); BWD_DQ: dS in columns of its own
+    constexpr uint32_t TP = T1, TDS = MODE == BWD_DKV ? T1 + 32u : 384u, PIECE = MODE == BWD_DKV ? 64u : 32u;
     pdl_wait();
 
     if (warp < 8) {
@@ -121,7 +132,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         const int quarter = warp & 3, half = warp >> 2;
         const int r = quarter * 32 + lane;                          // row of the resident block (= TMEM lane)
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        const uint32_t tT0 = tmem_base + lane_base, tT1 = tmem_base + lane_base + 128u;
+        const uint32_t tT0 = tmem_base + lane_base + T0, tT1 = tmem_base + lane_base + T1, tP = tmem_base + lane_base + TP, tDS = tmem_base + lane_base + TDS;
         const float c = p.scale_log2;
         float Lr = 0.f, Dr = 0.f;                                   // BWD_DQ: this row's statistics
         if (MODE == BWD_DQ) {
@@ -131,16 +142,16 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
         }
         bool ok = true;
         for (int it = 0; it < n_it; ++it) {
-            const int st = it & 1;
+            const int st1 = it % BWD_X1_STAGES;
+            if (MODE == BWD_DKV) {                                  // the statistics come with the X1 tile
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(BB_X1FULL + st1), (uint32_t)(it / BWD_X1_STAGES) & 1u, abort_flag));
+                if (!ok) break;
+            }
             // ---- phase 1: P = 2^(c S - L) for this warp's 64 columns
             ok = __all_sync(0xffffffffu, mbar_wait(bar(BB_TFULL + 0), (uint32_t)it & 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
-            const float* sStats = reinterpret_cast<const float*>(smem_raw + 2 * TILE_BYTES + st * BWD_STAGE_BYTES + 2 * TILE_BYTES);
-            if (MODE == BWD_DKV) {                                  // the statistics came with the stage's tiles (already complete: the
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(BB_XFULL + st), ((uint32_t)it >> 1) & 1u, abort_flag));   // products read them)
-                if (!ok) break;
-            }
+            const float* sStats = reinterpret_cast<const float*>(smem_raw + OFF_STATS + st1 * BWD_STATS_BYTES) + half * 64;
             float pv[64];
             {
                 uint32_t s0[32], s1[32];
@@ -148,36 +159,28 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                 tmem_ld32(tT0 + (uint32_t)(half * 64 + 32), s1);
                 tmem_wait_ld();
                 reg_fence32(s0); reg_fence32(s1);
-                if (MODE == BWD_DQ) {                               // S has been read: the next step's S may be formed
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(BB_PFULL + 0));
-                }
+                tc_fence_before();                                  // S has been read: the next step's S may be formed
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(BB_READ + 0));
 #pragma unroll
-                for (int e = 0; e < 64; e += 2) {
-                    float L0 = Lr, L1 = Lr;
-                    if (MODE == BWD_DKV) {                          // per column: the query row's statistic (a broadcast read)
-                        const float2 l2 = *reinterpret_cast<const float2*>(sStats + half * 64 + e);
-                        L0 = l2.x; L1 = l2.y;
-                    }
-                    const uint32_t a = e < 32 ? s0[e & 31] : s1[e & 31], bq = e < 32 ? s0[(e & 31) + 1] : s1[(e & 31) + 1];
-                    pv[e] = ex2(fmaf(__uint_as_float(a), c, -L0));
-                    pv[e + 1] = ex2(fmaf(__uint_as_float(bq), c, -L1));
+                for (int e = 0; e < 64; e += 4) {
+                    float4 L4 = make_float4(Lr, Lr, Lr, Lr);
+                    if (MODE == BWD_DKV) L4 = *reinterpret_cast<const float4*>(sStats + e);   // per column: the query row's statistic (a broadcast read)
+                    const uint32_t* const sv = e < 32 ? s0 : s1;
+                    pv[e] = ex2(fmaf(__uint_as_float(sv[e & 31]), c, -L4.x));
+                    pv[e + 1] = ex2(fmaf(__uint_as_float(sv[(e & 31) + 1]), c, -L4.y));
+                    pv[e + 2] = ex2(fmaf(__uint_as_float(sv[(e & 31) + 2]), c, -L4.z));
+                    pv[e + 3] = ex2(fmaf(__uint_as_float(sv[(e & 31) + 3]), c, -L4.w));
                 }
             }
+            uint32_t pk[32];
             if (MODE == BWD_DKV) {
-                uint32_t pk[32];
 #pragma unroll
                 for (int e = 0; e < 32; e++) pk[e] = pack16<DT_F16>(pv[2 * e], pv[2 * e + 1]);
-                // element pair (2c, 2c+1) of this warp's contraction range in column c of its OWN columns: only what this
-                // thread has just read is overwritten
-                tmem_st32(tT0 + (uint32_t)(half * 64), pk);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(BB_PFULL + 0));
+                reg_fence32(pk);
             }
             // ---- phase 2: dS = P (dP - D)
+            // The second product of this step is complete and with it every product in front of it, the previous step's dV and dK among them
             ok = __all_sync(0xffffffffu, mbar_wait(bar(BB_TFULL + 1), (uint32_t)it & 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
@@ -187,22 +190,34 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                 tmem_ld32(tT1 + (uint32_t)(half * 64 + 32), d1);
                 tmem_wait_ld();
                 reg_fence32(d0); reg_fence32(d1);
-#pragma unroll
-                for (int e = 0; e < 64; e += 2) {
-                    float D0 = Dr, D1 = Dr;
-                    if (MODE == BWD_DKV) {
-                        const float2 dd = *reinterpret_cast<const float2*>(sStats + 128 + half * 64 + e);
-                        D0 = dd.x; D1 = dd.y;
-                    }
-                    const uint32_t a = e < 32 ? d0[e & 31] : d1[e & 31], bq = e < 32 ? d0[(e & 31) + 1] : d1[(e & 31) + 1];
-                    dk[e >> 1] = pack16<DT_F16>(pv[e] * (__uint_as_float(a) - D0), pv[e + 1] * (__uint_as_float(bq) - D1));
+                if (MODE == BWD_DKV) {                              // element pair (2c, 2c+1) of the contraction in column c
+                    tmem_st32(tP + (uint32_t)half * PIECE, pk);
+                    tmem_wait_st();
                 }
-                tmem_st32(tT1 + (uint32_t)(half * 64), dk);
+                tc_fence_before();                                  // BWD_DKV: P^T is stored; BWD_DQ: dP has been read, the next step's may be formed
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(BB_READ + 1));
+                if (MODE == BWD_DQ && tid == 0) mbar_arrive(bar(BB_X1EMPTY + st1));   // V_j has been multiplied
+#pragma unroll
+                for (int e = 0; e < 64; e += 4) {
+                    float4 D4 = make_float4(Dr, Dr, Dr, Dr);
+                    if (MODE == BWD_DKV) D4 = *reinterpret_cast<const float4*>(sStats + 128 + e);
+                    const uint32_t* const dv = e < 32 ? d0 : d1;
+                    dk[e >> 1] = pack16<DT_F16>(pv[e] * (__uint_as_float(dv[e & 31]) - D4.x), pv[e + 1] * (__uint_as_float(dv[(e & 31) + 1]) - D4.y));
+                    dk[(e >> 1) + 1] = pack16<DT_F16>(pv[e + 2] * (__uint_as_float(dv[(e & 31) + 2]) - D4.z), pv[e + 3] * (__uint_as_float(dv[(e & 31) + 3]) - D4.w));
+                }
+                if (MODE == BWD_DQ && it > 0) {                     // the previous step's dQ has read dS and its K_j
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar(BB_DSFREE), (uint32_t)(it - 1) & 1u, abort_flag));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (tid == 0) mbar_arrive(bar(BB_X0EMPTY + (it - 1) % BWD_X0_STAGES));
+                }
+                tmem_st32(tDS + (uint32_t)half * PIECE, dk);
             }
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(BB_PFULL + 1));
+            if (lane == 0) mbar_arrive(bar(BB_DS));
         }
         // ------------------------------------------------------------------ epilogue: accumulators -> global
         // Each warp turns its 32 rows x 64 columns of an accumulator into two 32 x 32 fp32 boxes (128-byte rows, 128-byte
@@ -262,53 +277,68 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                     mma_ss_w<1>(d_tmem, alo + off, blo + off, DESC_HI, IDESC_T);
                 }
             };
-            // the fp16 A operand sits in two pieces: contraction elements [64 hh, 64 hh + 64) at columns [64 hh, 64 hh + 32)
             auto issue_A = [&](uint32_t d_tmem, uint32_t a_region, uint32_t b_saddr, bool first) {
                 const uint32_t blo = smem_desc_lo(b_saddr, HALF_BYTES);
 #pragma unroll
                 for (int kk = 0; kk < 8; kk++) {
-                    const uint32_t a_t = a_region + (uint32_t)(64 * (kk >> 2) + 8 * (kk & 3));
+                    const uint32_t a_t = a_region + PIECE * (uint32_t)(kk >> 2) + (uint32_t)(8 * (kk & 3));
                     if (kk == 0 && first) mma_ts_w<0>(d_tmem, a_t, blo, DESC_HI, IDESC_A);
                     else mma_ts_w<1>(d_tmem, a_t, blo + (uint32_t)(kk * 128), DESC_HI, IDESC_A);
                 }
             };
-            auto xaddr = [&](int st) { return sX + (uint32_t)st * BWD_STAGE_BYTES; };
-            bool good = mbar_wait(bar(BB_RES), 0u, abort_flag);
+            auto x0 = [&](int it) { return sX0 + (uint32_t)(it % BWD_X0_STAGES) * TILE_BYTES; };
+            auto x1 = [&](int it) { return sX1 + (uint32_t)(it % BWD_X1_STAGES) * TILE_BYTES; };
+            auto x0_wait = [&](int it) { return mbar_wait(bar(BB_X0FULL + it % BWD_X0_STAGES), (uint32_t)(it / BWD_X0_STAGES) & 1u, abort_flag); };
+            auto x1_wait = [&](int it) { return mbar_wait(bar(BB_X1FULL + it % BWD_X1_STAGES), (uint32_t)(it / BWD_X1_STAGES) & 1u, abort_flag); };
+            auto step_wait = [&](int which, int it) { return mbar_wait(bar(which), (uint32_t)it & 1u, abort_flag); };
+            auto first_T = [&](int it) { issue_T(tmem_base + T0, sR0, x0(it)); tc_commit(bar(BB_TFULL + 0)); };    // S / S^T
+            auto second_T = [&](int it) { issue_T(tmem_base + T1, sR1, x1(it)); tc_commit(bar(BB_TFULL + 1)); };   // dP / dP^T
+            bool good = mbar_wait(bar(BB_RES), 0u, abort_flag) && x0_wait(0);
             if (good) {
-                good = mbar_wait(bar(BB_XFULL + 0), 0u, abort_flag);
+                tc_fence_after();
+                first_T(0);
+                good = x1_wait(0);
                 if (good) {
                     tc_fence_after();
-                    issue_T(tmem_base, sR0, xaddr(0));
-                    tc_commit(bar(BB_TFULL + 0));
-                    issue_T(tmem_base + 128u, sR1, xaddr(0) + TILE_BYTES);
-                    tc_commit(bar(BB_TFULL + 1));
+                    second_T(0);
                 }
             }
+            // tiles are waited for in front of the softmax warps, whose signal is what the next product hangs on
             for (int it = 0; it < n_it && good; ++it) {
-                const int st = it & 1;
-                const uint32_t x0 = xaddr(st), x1 = x0 + TILE_BYTES;
                 const bool more = it + 1 < n_it;
-                // phase 1 of this step is over: P^T is stored (BWD_DKV) / S has been read (BWD_DQ)
-                good = mbar_wait(bar(BB_PFULL + 0), (uint32_t)it & 1u, abort_flag);
-                if (!good) break;
-                tc_fence_after();
-                if (MODE == BWD_DKV) issue_A(tmem_base + 256u, tmem_base, x1, it == 0);               // dV += P^T dO_i
                 if (more) {
-                    good = mbar_wait(bar(BB_XFULL + (st ^ 1)), ((uint32_t)(it + 1) >> 1) & 1u, abort_flag);
+                    good = x0_wait(it + 1) && step_wait(BB_READ + 0, it);
                     if (!good) break;
                     tc_fence_after();
-                    issue_T(tmem_base, sR0, xaddr(st ^ 1));                                           // the next step's S / S^T
-                    tc_commit(bar(BB_TFULL + 0));
+                    first_T(it + 1);
+                    good = x1_wait(it + 1);
+                    if (!good) break;
                 }
-                good = mbar_wait(bar(BB_PFULL + 1), (uint32_t)it & 1u, abort_flag);
-                if (!good) break;
-                tc_fence_after();
-                if (MODE == BWD_DKV) issue_A(tmem_base + 384u, tmem_base + 128u, x0, it == 0);        // dK += dS^T Q_i
-                else issue_A(tmem_base + 256u, tmem_base + 128u, x0, it == 0);                        // dQ += dS K_j
-                tc_commit(bar(BB_XEMPTY + st));                                    // every product on this stage has been issued
-                if (more) {
-                    issue_T(tmem_base + 128u, sR1, xaddr(st ^ 1) + TILE_BYTES);                       // the next step's dP / dP^T
-                    tc_commit(bar(BB_TFULL + 1));
+                if (MODE == BWD_DKV) {
+                    good = step_wait(BB_READ + 1, it);
+                    if (!good) break;
+                    tc_fence_after();
+                    issue_A(tmem_base + 256u, tmem_base + TP, x1(it), it == 0);                           // dV += P^T dO_i
+                    good = step_wait(BB_DS, it);
+                    if (!good) break;
+                    tc_fence_after();
+                    issue_A(tmem_base + 384u, tmem_base + TDS, x0(it), it == 0);                          // dK += dS^T Q_i
+                    if (more) {
+                        tc_commit(bar(BB_X1EMPTY + it % BWD_X1_STAGES));                                 // this step's tiles are multiplied, its statistics read
+                        second_T(it + 1);
+                    }
+                } else {
+                    if (more) {
+                        good = step_wait(BB_READ + 1, it);
+                        if (!good) break;
+                        tc_fence_after();
+                        second_T(it + 1);
+                    }
+                    good = step_wait(BB_DS, it);
+                    if (!good) break;
+                    tc_fence_after();
+                    issue_A(tmem_base + 256u, tmem_base + TDS, x0(it), it == 0);                          // dQ += dS K_j
+                    if (more) tc_commit(bar(BB_DSFREE));
                 }
             }
             if (good) tc_commit(bar(BB_ACC));
@@ -322,21 +352,28 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
             load_tile(sR0, MODE == BWD_DKV ? &tmK : &tmQ, bar(BB_RES), blk * BM);
             load_tile(sR1, MODE == BWD_DKV ? &tmV : &tmdO, bar(BB_RES), blk * BM);
             bool good = true;
-            int issued = 0;
+            int issued0 = 0, issued1 = 0;
             for (int it = 0; it < n_it && good; ++it) {
-                const int st = it & 1;
-                good = mbar_wait(bar(BB_XEMPTY + st), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag);
+                const int st0 = it % BWD_X0_STAGES, st1 = it % BWD_X1_STAGES;
+                if (MODE == BWD_DQ) {
+                    good = mbar_wait(bar(BB_X0EMPTY + st0), ((uint32_t)(it / BWD_X0_STAGES) & 1u) ^ 1u, abort_flag);
+                    if (!good) break;
+                }                                                     // BWD_DKV: step it - 3 was waited for in front of the last X1 tile
+                mbar_expect_tx(bar(BB_X0FULL + st0), TILE_BYTES);
+                load_tile(sX0 + st0 * TILE_BYTES, MODE == BWD_DKV ? &tmQ : &tmK, bar(BB_X0FULL + st0), (i0 + it) * BM);
+                issued0 = it + 1;
+                good = mbar_wait(bar(BB_X1EMPTY + st1), ((uint32_t)(it / BWD_X1_STAGES) & 1u) ^ 1u, abort_flag);
                 if (!good) break;
-                issued = it + 1;
-                const uint32_t x0 = sX + st * BWD_STAGE_BYTES, x1 = x0 + TILE_BYTES;
-                mbar_expect_tx(bar(BB_XFULL + st), 2 * TILE_BYTES + (MODE == BWD_DKV ? 1024 : 0));
-                load_tile(x0, MODE == BWD_DKV ? &tmQ : &tmK, bar(BB_XFULL + st), (i0 + it) * BM);
-                load_tile(x1, MODE == BWD_DKV ? &tmdO : &tmV, bar(BB_XFULL + st), (i0 + it) * BM);
-                if (MODE == BWD_DKV) bulk_load_1d(x1 + TILE_BYTES, p.stats + (((size_t)b * p.H + h) * nqb + (i0 + it)) * 256, 1024, bar(BB_XFULL + st));
+                mbar_expect_tx(bar(BB_X1FULL + st1), TILE_BYTES + (MODE == BWD_DKV ? BWD_STATS_BYTES : 0));
+                load_tile(sX1 + st1 * TILE_BYTES, MODE == BWD_DKV ? &tmdO : &tmV, bar(BB_X1FULL + st1), (i0 + it) * BM);
+                if (MODE == BWD_DKV)
+                    bulk_load_1d(base + OFF_STATS + st1 * BWD_STATS_BYTES, p.stats + (((size_t)b * p.H + h) * nqb + (i0 + it)) * 256, BWD_STATS_BYTES, bar(BB_X1FULL + st1));
+                issued1 = it + 1;
             }
             if (!good || *abort_flag) {                               // let the copies already requested land before the memory goes away
                 drain_wait(bar(BB_RES), 0u);
-                for (int k = issued > 2 ? issued - 2 : 0; k < issued; ++k) drain_wait(bar(BB_XFULL + (k & 1)), ((uint32_t)k >> 1) & 1u);
+                for (int k = max(issued0 - BWD_X0_STAGES, 0); k < issued0; ++k) drain_wait(bar(BB_X0FULL + k % BWD_X0_STAGES), (uint32_t)(k / BWD_X0_STAGES) & 1u);
+                for (int k = max(issued1 - BWD_X1_STAGES, 0); k < issued1; ++k) drain_wait(bar(BB_X1FULL + k % BWD_X1_STAGES), (uint32_t)(k / BWD_X1_STAGES) & 1u);
             }
         }
         __syncwarp();
