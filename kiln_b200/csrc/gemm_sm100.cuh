@@ -45,12 +45,18 @@ constexpr int EPI_F32 = 0, EPI_F16 = 1, EPI_GELU16 = 2, EPI_RESID = 3, EPI_HEADS
 constexpr int GB_M = 128;                                  // accumulator rows per CTA (TMEM lanes)
 constexpr int GB_K = 64;                                   // k step: one 128-byte swizzle atom of fp16
 constexpr int G_STAGE_BYTES = (GB_M + 128) * GB_K * 2;     // 32 KiB: this CTA's A rows then its W rows, each [128][64] fp16
-constexpr int G_STAGES = 5;
+// k steps in flight: 5 next to the head epilogue, whose warps turn 32 rows x 64 fp32 through shared memory, 6 next to the others, which stage
+// one box at a time. A step takes the tensor pipe 0.2-0.3 us and its tiles come from L2 or HBM, a microsecond away. Measured on B200 with 3,
+// 4, 5 stages (8 KB of staging per warp), 6 (4 KB): N 8192, K 2048, M 3456 (fp16) 100.7, 89.3, 85.1, 84.0 us, with GELU 107.7, 97.2, 92.5, 90.4;
+// N 2048, K 8192 (residual), M 3456 114.2, 101.2, 94.2, 92.9, M 1536 -, 45.3, 40.2, 38.6; K 2048, M 1536 14.6, 14.7 with 5 and 6.
+constexpr int G_MAX_STAGES = 6;
+__host__ __device__ constexpr int g_stages(int epi) { return epi == EPI_HEADS16 ? 5 : 6; }
 constexpr int G_EPI_WARPS = 8;                             // two per TMEM lane quarter, each taking every other column chunk
 constexpr int G_THREADS = 32 * (G_EPI_WARPS + 4);          // warps 0-7 epilogue; third warpgroup: warp 8 MMA issue, warp 9 TMA loads, two idle
 constexpr int G_GROUP_M = 8;                               // row tiles per raster group (engine/src/tcgemm16.cuh:18)
-constexpr int G_STAGING = G_EPI_WARPS * 32 * 256;          // per epilogue warp 32 rows x 256 bytes of output being re-ordered
-constexpr int G_SMEM = G_STAGES * G_STAGE_BYTES + G_STAGING + 2048 + 1024;   // = 227 KiB with the alignment slack
+__host__ __device__ constexpr int g_staging_warp(int epi) { return epi == EPI_HEADS16 ? 8192 : 4096; }   // output being re-ordered, per epilogue warp
+constexpr int G_SMEM = 6 * G_STAGE_BYTES + G_EPI_WARPS * 4096 + 2048 + 1024;   // = 227 KiB with the alignment slack, the same for every epilogue:
+static_assert(g_stages(EPI_HEADS16) * G_STAGE_BYTES + G_EPI_WARPS * g_staging_warp(EPI_HEADS16) == g_stages(EPI_F32) * G_STAGE_BYTES + G_EPI_WARPS * g_staging_warp(EPI_F32), "ring and staging");
 
 struct GemmParams {
     void* C;
@@ -82,7 +88,7 @@ struct alignas(64) GemmMaps {
     CUtensorMap w2[3];             // per segment: right operand [N, K2] of the second product
 };
 
-enum { GBAR_FULL = 0, GBAR_EMPTY = G_STAGES, GBAR_ACC_FULL = 2 * G_STAGES, GBAR_ACC_EMPTY = 2 * G_STAGES + 2, GBAR_COUNT = 2 * G_STAGES + 4 };
+enum { GBAR_FULL = 0, GBAR_EMPTY = G_MAX_STAGES, GBAR_ACC_FULL = 2 * G_MAX_STAGES, GBAR_ACC_EMPTY = 2 * G_MAX_STAGES + 2, GBAR_COUNT = 2 * G_MAX_STAGES + 4 };
 
 __device__ __forceinline__ float gelu_erf(float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); }   // engine/src/tcgemm16.cuh:55
 
@@ -113,12 +119,13 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     constexpr uint32_t STAGE_TX = (GB_M + W_ROWS) * GB_K * 2;             // bytes of a stage in use
     constexpr int TILE_M = PAIR ? 256 : 128;                              // tile rows over the CTA group
     constexpr bool OUT32 = (EPI == EPI_F32 || EPI == EPI_RESID);
-    constexpr bool NARROW = BN != BUF_COLS;                               // tiles that leave in chunks of one box, 32 columns wide
-    // columns per output chunk: 256-byte rows, or 128-byte rows where a tile would be a single chunk (16-bit output of one CTA), so that
-    // both warps of a lane quarter have one: every epilogue warp has to hand its share of the accumulator back
+    constexpr bool NARROW = BN != BUF_COLS;
+    // Columns per output chunk, which leaves as one or two boxes of 32 rows: 128-byte rows, or 64-byte rows where 64 16-bit columns do not
+    // divide the tile. Every epilogue warp has a chunk: it has to hand its share of the accumulator back.
     constexpr int CW = NARROW ? 32 : OUT32 || !PAIR ? 64 : 128;
-    constexpr int NCH = BN / CW, CHUNK_BOXES = NARROW ? 1 : CW * (OUT32 ? 4 : 2) / 128;
+    constexpr int NCH = BN / CW, BOX_COLS = OUT32 || NARROW ? 32 : 64, BOXES = CW / BOX_COLS, BOX_BYTES = 32 * BOX_COLS * (OUT32 ? 4 : 2);
     static_assert(NCH >= 2, "a chunk for both warps of a lane quarter");
+    constexpr int G_STAGES = g_stages(EPI), STAGING_WARP = g_staging_warp(EPI);
     constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
 
     extern __shared__ uint8_t smem_raw[];
@@ -127,8 +134,8 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
     uint8_t* const smem = smem_raw + (base - raw);
     const uint32_t sRing = base;
     uint8_t* const stage_out = smem + G_STAGES * G_STAGE_BYTES;
-    uint8_t* const ctrl = stage_out + G_STAGING;
-    const uint32_t bars = sRing + G_STAGES * G_STAGE_BYTES + G_STAGING;
+    uint8_t* const ctrl = stage_out + G_EPI_WARPS * STAGING_WARP;
+    const uint32_t bars = sRing + G_STAGES * G_STAGE_BYTES + G_EPI_WARPS * STAGING_WARP;
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 512);
     volatile uint32_t* const abort_flag = reinterpret_cast<volatile uint32_t*>(ctrl + 516);
     auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
@@ -343,7 +350,9 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
         } else {
             const int quarter = warp & 3, chunk0 = warp >> 2;                // TMEM lanes [32 quarter, +32); chunks chunk0, chunk0 + 2, ...
             const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-            uint8_t* const my_stage = stage_out + warp * 32 * 256;           // this warp's 32 rows x 256 bytes on their way out
+            constexpr int SLOTS = STAGING_WARP / BOX_BYTES;                  // boxes on their way out at a time
+            static_assert(SLOTS == 1 || SLOTS == 2, "");
+            uint8_t* const my_stage = stage_out + warp * STAGING_WARP;
             uint32_t use[2] = {0, 0};
             int k = 0, box_use = 0;
             for (int w = group; w < n_tiles; w += n_groups, ++k) {
@@ -400,7 +409,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                         for (int c = 0; c < CW; c++) v[c] = gelu_erf(v[c]);
                     }
                     if constexpr (EPI == EPI_RESID) {
-                        if (p.gate && (!NARROW || n0 + ch * CW < p.N)) {
+                        if (p.gate && n0 + ch * CW < p.N) {
 #pragma unroll
                             for (int c = 0; c < CW; c += 4) {
                                 const float4 gt = *reinterpret_cast<const float4*>(p.gate + n0 + ch * CW + c);
@@ -408,61 +417,43 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                             }
                         }
                     }
-                    const int x = n0 + ch * CW, y = m0 + quarter * 32;
-                    if constexpr (NARROW) {
-                        // one box of 32 columns (128-byte rows of fp32, 64-byte rows of fp16, swizzled likewise) in the two halves of
-                        // this warp's stage in turn: the box before the last has been read when the last one is all that is in flight
-                        uint8_t* const box = my_stage + box_use * 4096;
-                        box_use ^= 1;
-                        if (lane == 0) tma_store_wait_read_1();
+                    // The 32 rows of the chunk go through shared memory as swizzled boxes and leave by TMA (measured: 32 row stores per
+                    // warp took 3 us, the issue rate of plain global stores from eight warps; the bulk copy takes them off the warp).
+                    // Behind the last tile the ring is free (unless other parts of a cut k range read it): a place for every box of the
+                    // warp, and nobody waits for one to be read.
+                    const bool in_ring = !SPLIT && w + n_groups >= n_tiles;
+#pragma unroll
+                    for (int b = 0; b < BOXES; b++) {
+                        uint8_t* const box = in_ring ? smem + (warp * 4 + (ch >> 1) * BOXES + b) * 4096 : my_stage + (SLOTS == 2 ? box_use * BOX_BYTES : 0);
+                        if (!in_ring) {
+                            if (lane == 0) { if (SLOTS == 2) tma_store_wait_read_1(); else tma_store_wait_read(); }   // the box that was here has been read
+                            box_use ^= 1;
+                        }
                         __syncwarp();
 #pragma unroll
-                        for (int c = 0; c < (OUT32 ? 8 : 4); c++) {
-                            if constexpr (OUT32)
-                                *reinterpret_cast<float4*>(box + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-                            else
-                                *reinterpret_cast<uint4*>(box + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
-                                    make_uint4(pack16<DT_F16>(v[8 * c], v[8 * c + 1]), pack16<DT_F16>(v[8 * c + 2], v[8 * c + 3]),
-                                               pack16<DT_F16>(v[8 * c + 4], v[8 * c + 5]), pack16<DT_F16>(v[8 * c + 6], v[8 * c + 7]));
+                        for (int c = 0; c < BOX_BYTES / 512; c++) {           // 16-byte pieces of this thread's row
+                            uint4 pk;
+                            if constexpr (OUT32) {
+                                const float* const u = v + b * 32 + 4 * c;
+                                pk = make_uint4(__float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), __float_as_uint(u[3]));
+                            } else {
+                                const float* const u = v + b * BOX_COLS + 8 * c;
+                                pk.x = pack16<DT_F16>(u[0], u[1]); pk.y = pack16<DT_F16>(u[2], u[3]);
+                                pk.z = pack16<DT_F16>(u[4], u[5]); pk.w = pack16<DT_F16>(u[6], u[7]);
+                            }
+                            if constexpr (BOX_BYTES == 4096) *reinterpret_cast<uint4*>(box + lane * 128 + ((c ^ (lane & 7)) << 4)) = pk;
+                            else *reinterpret_cast<uint4*>(box + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = pk;
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0) {                                      // an empty group where nothing is stored: the count above holds
-                            if (nrow > 0 && x < p.N) {
+                        const int x = n0 + ch * CW + b * BOX_COLS, y = m0 + quarter * 32;
+                        if (lane == 0) {                                      // an empty group where nothing is stored, so that groups count boxes
+                            if (nrow > 0 && x < p.N) {                        // a narrow last column tile stores only the boxes that begin inside it
                                 if constexpr (EPI == EPI_RESID) tma_reduce_add_3d(&maps.c[seg], smem_u32(box), x, y, 0);
                                 else tma_store_3d(&maps.c[seg], smem_u32(box), x, y, 0);
                             }
                             tma_store_commit();
                         }
-                        continue;
-                    }
-                    // the 32 rows of the chunk go through shared memory as one or two 128-byte-swizzled boxes and
-                    // leaves by TMA (measured: 32 row stores per warp took 3 us, the issue rate of plain global stores from
-                    // eight warps; the bulk copy takes them off the warp)
-                    if (lane == 0) tma_store_wait_read();                     // the boxes of the last chunk have been read
-                    __syncwarp();
-#pragma unroll
-                    for (int c = 0; c < 8 * CHUNK_BOXES; c++) {
-                        uint4 pk;
-                        if constexpr (OUT32) {
-                            pk = make_uint4(__float_as_uint(v[4 * c]), __float_as_uint(v[4 * c + 1]), __float_as_uint(v[4 * c + 2]), __float_as_uint(v[4 * c + 3]));
-                        } else {
-                            pk.x = pack16<DT_F16>(v[8 * c + 0], v[8 * c + 1]); pk.y = pack16<DT_F16>(v[8 * c + 2], v[8 * c + 3]);
-                            pk.z = pack16<DT_F16>(v[8 * c + 4], v[8 * c + 5]); pk.w = pack16<DT_F16>(v[8 * c + 6], v[8 * c + 7]);
-                        }
-                        *reinterpret_cast<uint4*>(my_stage + (c >> 3) * 4096 + lane * 128 + (((c & 7) ^ (lane & 7)) << 4)) = pk;
-                    }
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && nrow > 0 && x < p.N) {                   // a narrow last column tile stores only the boxes that begin inside it
-                        if constexpr (EPI == EPI_RESID) {
-                            tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage), x, y, 0);
-                            if (CHUNK_BOXES == 2) tma_reduce_add_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
-                        } else {
-                            tma_store_3d(&maps.c[seg], smem_u32(my_stage), x, y, 0);
-                            if (CHUNK_BOXES == 2 && x + CW / 2 < p.N) tma_store_3d(&maps.c[seg], smem_u32(my_stage) + 4096, x + CW / 2, y, 0);
-                        }
-                        tma_store_commit();
                     }
                 }
             }
