@@ -33,7 +33,7 @@
 // With P written over S (the usual layout) a stream's next S cannot be issued before its own P*V has
 // consumed P, so its cycle is  softmax + P*V + S + two hand-offs  and two streams keep the tensor core ~58 % busy.
 // Here the next S of a stream does not depend on its P: the softmax threads ask for it while they are still
-// in their exponentials (`s_req`), it runs on the tensor core under the rest of that softmax, and the
+// in their exponentials or just before them (`s_req`), it runs on the tensor core under the rest of that softmax, and the
 // threads go from one block straight into the next; P*V follows whenever P is complete.
 //
 // Balanced schedule (MODE_PAIR, `split`). Items x key blocks rarely divide by the SM count (4096 tokens:
@@ -163,10 +163,11 @@ enum { BAR_QFULL = 0, BAR_QEMPTY = 2, BAR_SFULL = 4, BAR_SREQ = 6, BAR_PFULL = 8
 static_assert(BAR_COUNT * 8 <= 256, "the shared words of the control block start at byte 256");
 // the Q tile of stream i has been prepared in place (AttnParams::q_raw); MODE_PAIR has two and does not use BAR_NORMS
 __host__ __device__ constexpr int bar_q_ready(int mode, int i) { return mode == MODE_PAIR ? BAR_NORMS + i : BAR_QREADY; }
-// when a stream asks for its next S: 0 = before its exponentials, 1 = after the first half of them, 2 = with P (no overlap)
-#ifndef KB_SREQ_AT
-#define KB_SREQ_AT 1
-#endif
+// When a stream asks for its next S: before its exponentials (MODE_PAIR, whose streams share every K/V tile and take turns at the staging
+// area: the S is there when the block ends) or after the first half of them. Measured on B200, back to back, half way -> before: self-attention
+// bf16 1536 tokens 36.84 -> 36.33 us, 4096 161.8 -> 160.0, 2 x 3456 236.4 -> 233.7; NAG 4096 69.3 -> 70.0, 1536 33.15 -> 33.26; MODE_KEYS the same
+// either way (1000 tokens fp32 22.2).
+__host__ __device__ constexpr bool s_asked_early(int mode) { return mode == MODE_PAIR; }
 
 // full-CTA barrier usable from divergent role branches (same id and count everywhere)
 __device__ __forceinline__ void cta_sync() { named_bar_sync(2, ATTN_THREADS); }
@@ -614,9 +615,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     const int valid = Tk - j_last * BN;
 #pragma unroll
                     for (int q = 0; q < 4; q++)
+                        if (MODE != MODE_NAG || valid < 32 * q + 32) {        // (one block in two or three is ragged there: 1536 x (378, 168) 29.9 -> 29.5 us)
 #pragma unroll
-                        for (int e = 0; e < 32; e++)
-                            if (q * 32 + e >= valid) s[q][e] = 0xff800000u;
+                            for (int e = 0; e < 32; e++)
+                                if (q * 32 + e >= valid) s[q][e] = 0xff800000u;
+                        }
                 }
                 // From the lowest finite value up: a block whose keys all score -inf then has weights 0 and not NaN, also as the first
                 // block of a stream (in MODE_KEYS that of stream 1 is the second of the sequence) or of a part of a cut item.
@@ -629,7 +632,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     mx3 = max3(mx3, __uint_as_float(s[3][e]), __uint_as_float(s[3][e + 1]));
                 }
                 const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                if (KB_SREQ_AT == 0 && j + 1 < je) { __syncwarp(); if (lane == 0) mbar_arrive(bar(BAR_SREQ + i)); }
+                if (s_asked_early(MODE) && j + 1 < je) { __syncwarp(); if (lane == 0) mbar_arrive(bar(BAR_SREQ + i)); }
                 // The previous P*V of this stream reads P_i and writes O_i: it must be complete before either is touched.
                 // That wait sits as late as possible: before the first store of P, or before a rescale of O.
                 bool pv_done = false;
@@ -698,7 +701,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     if (q == 0) {
                         // Ask for the next S of this stream now: it runs on the tensor core under the second half of the
                         // exponentials. The register fences keep that second half from being scheduled ahead of the request.
-                        if (KB_SREQ_AT == 1 && j + 1 < je) { __syncwarp(); if (lane == 0) mbar_arrive(bar(BAR_SREQ + i)); }
+                        if (!s_asked_early(MODE) && j + 1 < je) { __syncwarp(); if (lane == 0) mbar_arrive(bar(BAR_SREQ + i)); }
                         reg_fence32(s[2]);
                         reg_fence32(s[3]);
                     }
@@ -712,7 +715,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    if (KB_SREQ_AT == 2 && j + 1 < je) mbar_arrive(bar(BAR_SREQ + i));
                     mbar_arrive(bar(BAR_PFULL + i));
                 }
             }
