@@ -258,7 +258,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                                          MODE == BWD_DKV ? part * p.B + b : b);
                     tma_store_commit();
                 }
-                tma_store_wait_all();                                       // the stage area goes away with the thread block
+                tma_store_wait_read();                                       // the stage area goes away with the thread block
             }
         }
     } else {

@@ -284,6 +284,8 @@ struct SegIter {
             s_end = n * (blockIdx.x + 1) / gridDim.x;
         }
     }
+    // is there a segment behind the last one that next() gave?
+    __device__ __forceinline__ bool more() const { return MODE == MODE_PAIR && p.split ? s < s_end : w < p.n_items; }
     __device__ __forceinline__ bool next(Seg& o) {
         int item, jb, je;
         if (MODE == MODE_PAIR && p.split) {
@@ -334,8 +336,11 @@ struct SegIter {
 
 // K/V ring bookkeeping. The loader fills ring entries in a fixed order and every consumer counts the same way:
 //   MODE_PAIR segment: K(jb), then per key block V(j), K(j+1): K(j) is entry 2(j-jb), V(j) entry 2(j-jb)+1 of the segment;
-//   MODE_NAG and MODE_KEYS item: K0(0), K1(0), then per block j and stream i (0 first): V_i(j), K_i(j+1).
-// nag_entry returns the entry of V_i(j) within the item (K_i(j+1), when it exists, is the next one).
+//   MODE_NAG and MODE_KEYS item: K0(0), K1(0), then per block j and stream i (0 first): K_i(j+1), V_i(j). (A step of both streams takes
+//     four tiles of a ring of four or six: K first, because S_i(j+1) wants it half a step before P_i(j) wants V_i(j), and because its
+//     place is free earlier, when S_i(j) has been read. V_i(j) first: NAG 4096 x (512, 512) 61.4 us and 1536 x (378, 168) 29.9, K first 59.4
+//     and 29.0, inside a CUDA graph.)
+// nag_entry returns the first entry of (i, j) within the item: K_i(j+1) when it exists, with V_i(j) behind it, or else V_i(j).
 __device__ __forceinline__ int nag_entry(int i, int j, int L0, int L1) {
     int e = (L0 > 0) + (L1 > 0);
     const int L[2] = {L0, L1};
@@ -561,8 +566,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     if (MODE == MODE_PAIR && !two) mbar_arrive(bar(BAR_KVEMPTY + (ring0 + entry) % NST));   // stream 1 is absent: its share too
                 }
             };
-            auto k_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) : (j == 0 ? (i == 1 && it.je[0] > 0 ? 1 : 0) : nag_entry(i, j - 1, it.je[0], it.je[1]) + 1)); };
-            auto v_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) + 1 : nag_entry(i, j, it.je[0], it.je[1])); };
+            auto k_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) : (j == 0 ? (i == 1 && it.je[0] > 0 ? 1 : 0) : nag_entry(i, j - 1, it.je[0], it.je[1]))); };
+            auto v_entry = [&](int j) { return (uint32_t)(MODE == MODE_PAIR ? 2 * (j - jb) + 1 : nag_entry(i, j, it.je[0], it.je[1]) + (j + 1 < je ? 1 : 0)); };
             if (RAW_Q && p.q_raw && (MODE != MODE_PAIR || je > jb)) {
                 // MODE_PAIR: a thread takes a whole row of its stream's tile. One Q tile: a thread takes half a row, and the two
                 // halves of a row's sum of squares meet in shared memory (fbuf is free between items).
@@ -837,9 +842,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                     // 16-bit output: the tile leaves in two rounds of 64 columns through this stream's own
                                     // [128][64] staging half (128-byte rows, 128-byte swizzle: what a bulk tensor store reads);
                                     // rows past Tq are clipped by the tensor map
-                                    uint8_t* const half_stage = smem + (2 + NST) * TILE_BYTES + i * HALF_BYTES;
+                                    // and nobody waits between them behind the last segment, when no Q comes any more and both halves
+                                    // fit into the stream's Q tile (its S products are done)
+                                    const bool last = !iter.more();
 #pragma unroll
                                     for (int hh = 0; hh < 2; hh++) {
+                                        uint8_t* const half_stage = last ? smem + i * TILE_BYTES + hh * HALF_BYTES : smem + (2 + NST) * TILE_BYTES + i * HALF_BYTES;
 #pragma unroll
                                         for (int q2 = 0; q2 < 2; q2++) {
                                             float v[32];
@@ -864,9 +872,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                         if (t == 0) {
                                             tma_store_3d(&tmO, smem_u32(half_stage), it.h * HD + 64 * hh, it.q0 + i * BM, it.b);
                                             tma_store_commit();
-                                            tma_store_wait_read();               // the half may be overwritten
+                                            if (!last) tma_store_wait_read();    // the half may be overwritten
                                         }
-                                        if (hh == 0) named_bar_sync(3 + i, 128);
+                                        if (hh == 0 && !last) named_bar_sync(3 + i, 128);
                                     }
                                 } else {
                                     // head-split runs: the tile is staged in this stream's Q tile (dead: every S product of the
@@ -1206,7 +1214,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             nag_finish(true);
             if (tid == 0 && last) mbar_arrive(bar(BAR_QEMPTY + 0));
         }
-        if (lane == 0) tma_store_wait_all();                              // bulk stores issued by this thread have landed
+        if (lane == 0) tma_store_wait_read();                              // bulk stores issued by this thread have read their tiles
         tc_fence_before();
         cta_sync();
     } else {
@@ -1300,7 +1308,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         }
                         n_s += per_blk * (uint32_t)(je - jb);
                     } else {
-                        // ring order (loader): K0(0), K1(0), then per block j and stream: V_i(j), K_i(j+1). Every tile belongs to
+                        // ring order (loader): K0(0), K1(0), then per block j and stream: K_i(j+1), V_i(j). Every tile belongs to
                         // one stream. Staging-area order: S0(0), S1(0), then S_i(j+1) in the same (j, i) order.
                         good = q_wait();
                         uint32_t g = n_s;
@@ -1318,13 +1326,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                                 if (j >= it.je[ii]) continue;
                                 const bool more = j + 1 < it.je[ii];
                                 if (ii == i) {
-                                    if (more) {                               // ring: V_i(j), then K_i(j+1)
-                                        good = sreq_wait() && kv_wait(ring + 1) && issue_S(g, kv_addr(ring + 1));
+                                    const uint32_t nv = ring + (more ? 1u : 0u);   // ring: K_i(j+1), then V_i(j)
+                                    if (more) {
+                                        good = sreq_wait() && kv_wait(ring) && issue_S(g, kv_addr(ring));
                                         if (!good) break;
                                     }
-                                    good = kv_wait(ring) && (j > 0 || o_free_wait()) && p_wait();
+                                    good = kv_wait(nv) && (j > 0 || o_free_wait()) && p_wait();
                                     if (!good) break;
-                                    issue_PV(kv_addr(ring), key_block(i, j), p.Tk[MODE == MODE_NAG ? i : 0], j == 0);
+                                    issue_PV(kv_addr(nv), key_block(i, j), p.Tk[MODE == MODE_NAG ? i : 0], j == 0);
                                     if (!more) tc_commit(bar(BAR_ODONE + i));
                                 }
                                 ring += more ? 2u : 1u;
@@ -1405,8 +1414,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         for (int j = 0; j < nmax && good; ++j) {
                             for (int i = 0; i < 2 && good; i++) {
                                 if (j >= it.je[i]) continue;
-                                load_kv(MODE == MODE_NAG && i ? &tmV1 : &tmV0, key_block(i, j) * BN);
-                                if (good && j + 1 < it.je[i]) load_kv(MODE == MODE_NAG && i ? &tmK1 : &tmK0, key_block(i, j + 1) * BN);
+                                if (j + 1 < it.je[i]) load_kv(MODE == MODE_NAG && i ? &tmK1 : &tmK0, key_block(i, j + 1) * BN);
+                                if (good) load_kv(MODE == MODE_NAG && i ? &tmV1 : &tmV0, key_block(i, j) * BN);
                             }
                         }
                     }
@@ -1419,7 +1428,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         ++qe_cnt[0];
                         if (good) store_staged();
                     }
-                    tma_store_wait_all();
+                    tma_store_wait_read();
                 }
                 // on failure, let the copies already requested land before the CTA's shared memory goes away: a bounded wait on
                 // the FULL barrier of every ring slot and Q tile that still has a request outstanding

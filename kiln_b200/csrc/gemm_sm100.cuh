@@ -346,7 +346,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     }
                 }
             }
-            if (lane == 0) tma_store_wait_all();
+            if (lane == 0) tma_store_wait_read();
         } else {
             const int quarter = warp & 3, chunk0 = warp >> 2;                // TMEM lanes [32 quarter, +32); chunks chunk0, chunk0 + 2, ...
             const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
@@ -457,7 +457,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     }
                 }
             }
-            if (lane == 0) tma_store_wait_all();
+            if (lane == 0) tma_store_wait_read();
         }
     } else if (warp == G_EPI_WARPS) {
         setmaxnreg_dec<56>();

@@ -110,8 +110,9 @@ __device__ __forceinline__ void tma_reduce_add_3d(const void* tmap, uint32_t src
                  : "memory");
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }   // all but the last group
+// What a thread block owes its bulk stores before it exits is that they have read its shared memory: that they have landed is part of the
+// grid's completion, which the next kernel waits for. Without the wait for the latter NAG 1536 x (378, 168) 32.3 -> 31.8 us back to back.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // One thread of the (converged) warp, the same one for a given warp. As the condition of a role's branch it tells the compiler that
