@@ -90,7 +90,26 @@ struct alignas(64) GemmMaps {
 
 enum { GBAR_FULL = 0, GBAR_EMPTY = G_MAX_STAGES, GBAR_ACC_FULL = 2 * G_MAX_STAGES, GBAR_ACC_EMPTY = 2 * G_MAX_STAGES + 2, GBAR_COUNT = 2 * G_MAX_STAGES + 4 };
 
-__device__ __forceinline__ float gelu_erf(float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); }   // engine/src/tcgemm16.cuh:55
+// v Phi(v) (engine/src/tcgemm16.cuh:55 takes erff) without the cancellation of 1 + erf in the negative tail and at half the instructions:
+// with a = |v|, erfc(a / sqrt 2) = 2^(-a Q(a)) and v Phi(v) = (v + |v| - a 2^(-a Q(a))) / 2. Q is a polynomial fitted to
+// -log2(erfc(a / sqrt 2)) / a on [0, 7] by weighted least squares (beyond 7 the term is below 1e-11, and Q is taken at 7). Against float64 over
+// N(0,1) and [-9, 9] in fp32: rel. 2-norm 2.8e-8 and 1.3e-8, largest error 2.4e-7 (0.5 v (1 + erff): 3.8e-8, 1.8e-8, 4.5e-7); rounded to fp16 the same.
+// Up-projection of 3456 rows, N 8192, K 2048, inside a CUDA graph: 91.4 -> 87.9 us (84.8 without any GELU).
+__device__ __forceinline__ float gelu(float v) {
+    const float a = fminf(fabsf(v), 7.f);
+    float q = -2.5095840960887017e-09f;
+    q = fmaf(q, a, 9.659256505756275e-08f);
+    q = fmaf(q, a, -1.6297367437800858e-06f);
+    q = fmaf(q, a, 1.5769759556860663e-05f);
+    q = fmaf(q, a, -9.427715122001246e-05f);
+    q = fmaf(q, a, 3.198326739948243e-04f);
+    q = fmaf(q, a, -5.3875570301897824e-05f);
+    q = fmaf(q, a, -6.906468421220779e-03f);
+    q = fmaf(q, a, 5.242638662457466e-02f);
+    q = fmaf(q, a, 0.4592227637767792f);
+    q = fmaf(q, a, 1.151104211807251f);
+    return 0.5f * ((v + fabsf(v)) - a * ex2(-(q * a)));
+}
 
 // tile w -> (row tile, column tile): groups of G_GROUP_M row tiles x every column tile, column-major inside a group, so
 // the CTAs running at the same time share weight tiles in L2 (engine/src/tcgemm16.cuh:66-69)
@@ -406,7 +425,7 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     }
                     if constexpr (EPI == EPI_GELU16) {
 #pragma unroll
-                        for (int c = 0; c < CW; c++) v[c] = gelu_erf(v[c]);
+                        for (int c = 0; c < CW; c++) v[c] = gelu(v[c]);
                     }
                     if constexpr (EPI == EPI_RESID) {
                         if (p.gate && n0 + ch * CW < p.N) {

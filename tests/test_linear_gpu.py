@@ -456,6 +456,20 @@ def test_narrow_tiles(kb, M, N, K, epi):
         _close(out, ref, K + 40, f"{epi} {M}x{N}x{K} lora {lora}", epi in ("F16", "GELU16"))
 
 
+def test_gelu_over_its_whole_range(kb):
+    """Every finite fp16 value through the identity: GELU against float64, to half a unit of the fp16 result and 1e-6 of fp32 arithmetic;
+    exact limits (x far up, 0 far down)."""
+    from kiln_b200 import ops
+    x = np.arange(65536, dtype=np.uint16).view(np.float16)
+    x = x[np.isfinite(x)]
+    x = np.resize(x, (-(-x.size // 64), 64))
+    out = _run(kb, x.astype(np.float32), np.concatenate([np.eye(64, dtype=np.float32)] * 2), ops.EPI_GELU16)[:, :64].astype(np.float64)
+    v = torch.from_numpy(x.astype(np.float64))
+    ref = (v * torch.special.ndtr(v)).numpy()
+    assert np.all(np.abs(out - ref) <= np.abs(ref) * (2.0 ** -11 + 1e-6) + 2.0 ** -25 + 1e-9), np.abs(out - ref).max()
+    assert np.array_equal(out[x >= 8], x[x >= 8].astype(np.float64)) and not out[x <= -8].any()
+
+
 def test_lora_argument_errors(kb):
     import ctypes
     L = kb.lib()
