@@ -70,7 +70,7 @@ struct BwdParams {
 };
 
 // T is the first product (S or S^T) or the second (dP or dP^T) of a step. READ, DS: one arrival per softmax warp
-enum { BB_RES = 0, BB_X0FULL = 1, BB_X0EMPTY = BB_X0FULL + BWD_X0_STAGES, BB_X1FULL = BB_X0EMPTY + BWD_X0_STAGES, BB_X1EMPTY = BB_X1FULL + BWD_X1_STAGES,
+enum { BB_RES = 0, BB_X0FULL = 2, BB_X0EMPTY = BB_X0FULL + BWD_X0_STAGES, BB_X1FULL = BB_X0EMPTY + BWD_X0_STAGES, BB_X1EMPTY = BB_X1FULL + BWD_X1_STAGES,
        BB_TFULL = BB_X1EMPTY + BWD_X1_STAGES, BB_READ = BB_TFULL + 2, BB_DS = BB_READ + 2, BB_DSFREE, BB_ACC, BB_COUNT };
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -293,11 +293,11 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
             auto step_wait = [&](int which, int it) { return mbar_wait(bar(which), (uint32_t)it & 1u, abort_flag); };
             auto first_T = [&](int it) { issue_T(tmem_base + T0, sR0, x0(it)); tc_commit(bar(BB_TFULL + 0)); };    // S / S^T
             auto second_T = [&](int it) { issue_T(tmem_base + T1, sR1, x1(it)); tc_commit(bar(BB_TFULL + 1)); };   // dP / dP^T
-            bool good = mbar_wait(bar(BB_RES), 0u, abort_flag) && x0_wait(0);
+            bool good = mbar_wait(bar(BB_RES + 0), 0u, abort_flag) && x0_wait(0);
             if (good) {
                 tc_fence_after();
                 first_T(0);
-                good = x1_wait(0);
+                good = mbar_wait(bar(BB_RES + 1), 0u, abort_flag) && x1_wait(0);
                 if (good) {
                     tc_fence_after();
                     second_T(0);
@@ -348,9 +348,11 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                 tma_load_3d(dst, tm, mbar, h * HD, row0, b);
                 tma_load_3d(dst + HALF_BYTES, tm, mbar, h * HD + 64, row0, b);
             };
-            mbar_expect_tx(bar(BB_RES), 2 * TILE_BYTES);
-            load_tile(sR0, MODE == BWD_DKV ? &tmK : &tmQ, bar(BB_RES), blk * BM);
-            load_tile(sR1, MODE == BWD_DKV ? &tmV : &tmdO, bar(BB_RES), blk * BM);
+            // the resident pair, each tile in front of the first streamed one that it is multiplied with
+            auto load_res = [&](int i) {
+                mbar_expect_tx(bar(BB_RES + i), TILE_BYTES);
+                load_tile(i ? sR1 : sR0, i == 0 ? (MODE == BWD_DKV ? &tmK : &tmQ) : (MODE == BWD_DKV ? &tmV : &tmdO), bar(BB_RES + i), blk * BM);
+            };
             bool good = true;
             int issued0 = 0, issued1 = 0;
             for (int it = 0; it < n_it && good; ++it) {
@@ -359,11 +361,13 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                     good = mbar_wait(bar(BB_X0EMPTY + st0), ((uint32_t)(it / BWD_X0_STAGES) & 1u) ^ 1u, abort_flag);
                     if (!good) break;
                 }                                                     // BWD_DKV: step it - 3 was waited for in front of the last X1 tile
+                if (it == 0) load_res(0);
                 mbar_expect_tx(bar(BB_X0FULL + st0), TILE_BYTES);
                 load_tile(sX0 + st0 * TILE_BYTES, MODE == BWD_DKV ? &tmQ : &tmK, bar(BB_X0FULL + st0), (i0 + it) * BM);
                 issued0 = it + 1;
                 good = mbar_wait(bar(BB_X1EMPTY + st1), ((uint32_t)(it / BWD_X1_STAGES) & 1u) ^ 1u, abort_flag);
                 if (!good) break;
+                if (it == 0) load_res(1);
                 mbar_expect_tx(bar(BB_X1FULL + st1), TILE_BYTES + (MODE == BWD_DKV ? BWD_STATS_BYTES : 0));
                 load_tile(sX1 + st1 * TILE_BYTES, MODE == BWD_DKV ? &tmdO : &tmV, bar(BB_X1FULL + st1), (i0 + it) * BM);
                 if (MODE == BWD_DKV)
@@ -371,7 +375,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& tmQ, const CUte
                 issued1 = it + 1;
             }
             if (!good || *abort_flag) {                               // let the copies already requested land before the memory goes away
-                drain_wait(bar(BB_RES), 0u);
+                for (int i = 0; i < 2; i++) drain_wait(bar(BB_RES + i), 0u);
                 for (int k = max(issued0 - BWD_X0_STAGES, 0); k < issued0; ++k) drain_wait(bar(BB_X0FULL + k % BWD_X0_STAGES), (uint32_t)(k / BWD_X0_STAGES) & 1u);
                 for (int k = max(issued1 - BWD_X1_STAGES, 0); k < issued1; ++k) drain_wait(bar(BB_X1FULL + k % BWD_X1_STAGES), (uint32_t)(k / BWD_X1_STAGES) & 1u);
             }
