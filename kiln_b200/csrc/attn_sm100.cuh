@@ -77,10 +77,6 @@ constexpr int TILE_BYTES = BM * HD * 2; // 32 KiB: one Q, K or V tile (two 64-co
 constexpr int HALF_BYTES = TILE_BYTES / 2;
 constexpr int NSTAGE = 4;               // K/V ring depth of MODE_PAIR and MODE_NAG
 constexpr int NSTAGE_KEYS = 6;          // of MODE_KEYS, whose streams share no tile (four new ones per step of both streams)
-#ifndef KB_POLY_PAIRS
-#define KB_POLY_PAIRS 0
-#endif
-constexpr int POLY_PAIRS = KB_POLY_PAIRS; // of every 8 score pairs, this many take 2^x on the FMA pipe instead of MUFU
 constexpr int ATTN_THREADS = 384;
 // Registers per thread after the warpgroups re-divide the 384 x 168 the block starts with: 256 softmax threads x 224 + 128
 // threads of the MMA / TMA / helper warps x 56 = 64512 exactly (a larger second number would leave the softmax warps'
@@ -673,8 +669,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         }
                     }
                 }
-                // p = 2^(s*c - m*c) on packed pairs: one FFMA2 per two scores, then MUFU ex2 (and the FMA-pipe
-                // polynomial for POLY_PAIRS of every 8 pairs, when enabled).
+                // p = 2^(s*c - m*c) on packed pairs: one FFMA2 per two scores, then MUFU ex2.
                 const uint64_t c2 = pack2(c, c), nmc2 = pack2(-row_m * c, -row_m * c);
                 uint64_t sum2a = pack2(0.f, 0.f), sum2b = sum2a;
 #pragma unroll
@@ -684,14 +679,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     for (int e = 0; e < 32; e++) {                 // pair e of this half: scores 2e, 2e+1 of chunk 2q + e/16
                         const int ch = 2 * q + (e >> 4), ee = (e & 15) * 2;
                         const uint64_t x2 = fma2(pack2u(s[ch][ee], s[ch][ee + 1]), c2, nmc2);
-                        uint64_t p2;
-                        if ((e & 7) >= 8 - POLY_PAIRS) {
-                            p2 = ex2_poly2(x2);
-                        } else {
-                            float x0, x1;
-                            unpack2(x2, x0, x1);
-                            p2 = pack2(ex2(x0), ex2(x1));
-                        }
+                        float x0, x1;
+                        unpack2(x2, x0, x1);
+                        const uint64_t p2 = pack2(ex2(x0), ex2(x1));
                         if (e & 1) sum2b = add2(sum2b, p2); else sum2a = add2(sum2a, p2);
                         float p0, p1;
                         unpack2(p2, p0, p1);

@@ -8,7 +8,7 @@
 // The attention kernel's tensor-core operands are always fp16 (as in the reference, which converts to
 // fp16 while staging): bf16 and fp32 inputs are converted here, fp16 inputs that need neither norm nor
 // RoPE skip this pass entirely.
-// HBM-bound: half a warp per (row, head), 8 elements (16 bytes) per lane, one pass at full occupancy.
+// Bound by memory; a warp takes several heads of a row, see qk_prep_kernel.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

@@ -83,6 +83,24 @@ def test_many_query_tiles_and_several_key_blocks(kb, Tq, Tk, H, npad, B, kind):
             assert_close(g[sk][j0:, cs], r, f"{name} {Tq}x{Tk}x{H} image {b}", max_abs=2e-3 * max(1.0, float(np.sqrt((r * r).mean(1)).max())))
 
 
+@pytest.mark.parametrize("nq,nk", [(1, 1), (1, 4), (2, 1), (2, 3), (3, 2), (3, 7), (4, 4), (5, 1), (5, 6), (7, 2)], ids=str)
+def test_every_phase_of_the_rings(kb, nq, nk):
+    """Numbers of streamed blocks around the depths of the two rings (three and two stages), in both roles and with ragged last blocks,
+    against float64 on the rounded operands. The bound is the one of the larger cases above: 2e-3 of the largest row's rms."""
+    H, Tq, Tk = 2, 128 * nq - 37, 128 * nk - 5
+    g = torch.Generator(device="cuda").manual_seed(10 * nq + nk)
+    q, do = (torch.randn(Tq, H * 128, generator=g, device="cuda").half() for _ in range(2))
+    k, v = (torch.randn(Tk, H * 128, generator=g, device="cuda").half() for _ in range(2))
+    heads = lambda t: t.double().reshape(t.shape[0], H, 128).transpose(0, 1)
+    Q, K, V, G = map(heads, (q, k, v, do))
+    P = torch.softmax(Q @ K.transpose(1, 2) / 128 ** 0.5, -1)
+    dP = G @ V.transpose(1, 2)
+    dS = P * (dP - (dP * P).sum(-1, keepdim=True)) / 128 ** 0.5
+    refs = [x.transpose(0, 1).reshape(-1, H * 128).cpu().numpy() for x in (dS @ K, dS.transpose(1, 2) @ Q, P.transpose(1, 2) @ G)]
+    for name, out, ref in zip(("dq", "dk", "dv"), _run(kb, *(t.float().cpu().numpy() for t in (q, k, v, do)), 1, Tq, Tk, 0, H, "f16"), refs):
+        assert np.abs(out - ref).max() <= 2e-3 * max(1.0, np.sqrt((ref * ref).mean(1)).max()), f"{name}: {np.abs(out - ref).max():.2e}"
+
+
 def test_batch_equals_per_image_calls(kb):
     B, T, H = 2, 200, 2
     D = H * 128

@@ -444,6 +444,32 @@ def test_nag(kb, Tq, H, Tp, Tn, kind, s):
     (assert_close if kind == "f16" else assert_close_bf16_storage)(out16, ref, f"NAG 16-bit out Tq={Tq} H={H} Tp={Tp} Tn={Tn} {kind} s={s}")
 
 
+@pytest.mark.parametrize("Tp,Tn", [(1, 500), (128, 129), (250, 40), (300, 513), (512, 512), (640, 100), (129, 384)], ids=str)
+def test_nag_block_counts_of_both_streams(kb, Tp, Tn):
+    """One to five key blocks per stream, equal and not, over more items than SMs, so that the ring runs on from item to item; against
+    float64. 1e-2 of the largest value: fp16 weights and tiles, amplified by the guidance scale of 5."""
+    H, Tq = 16, 1290
+    g = torch.Generator(device="cuda").manual_seed(Tp + Tn)
+    q = torch.randn(Tq, H * 128, generator=g, device="cuda").half()
+    ctx = [torch.randn(n, H * 128, generator=g, device="cuda").half() for n in (Tp, Tp, Tn, Tn)]
+    out = torch.empty_like(q)
+    ws = torch.empty(kb.workspace_bytes(Tq, max(Tp, Tn), H, torch.float16, n_ctx=2), dtype=torch.uint8, device="cuda")
+    kb.attn_nag(out, q, ctx[0], ctx[1], Tp, 7, ctx[2], ctx[3], Tn, 11, 5.0, 2.5, 0.25, Tq, H, workspace=ws)
+    assert kb.check_status() == 0
+    heads = lambda t: t.double().reshape(t.shape[0], H, 128).transpose(0, 1)
+
+    def attend(k, v, npad):
+        s = torch.cat([heads(q) @ heads(k).transpose(1, 2) / 128 ** 0.5, torch.zeros(H, Tq, npad, device="cuda", dtype=torch.double)], -1)
+        return (torch.softmax(s, -1)[..., :k.shape[0]] @ heads(v)).transpose(0, 1).reshape(Tq, H * 128)
+
+    zp, zn = attend(ctx[0], ctx[1], 7), attend(ctx[2], ctx[3], 11)
+    gd = zp * 5.0 - zn * 4.0
+    ratio = gd.abs().sum(1, keepdim=True) / zp.abs().sum(1, keepdim=True)
+    ref = 0.25 * gd * torch.clamp(2.5 / ratio, max=1.0) + 0.75 * zp
+    assert (out.double() - ref).abs().max().item() <= 1e-2 * max(1.0, ref.abs().max().item())
+    assert ((out.double() - ref).norm() / ref.norm()).item() <= 2e-3
+
+
 def test_nag_identities_and_clamp(kb):
     Tq, H, L, kind = 384, 16, 512, "f16"
     q = seeded(7, Tq, H * 128, kind)
