@@ -203,32 +203,39 @@ struct PrepBatch {
         PrepSeg& sg = pp.seg[pp.nseg++];
         sg.in = in; sg.out = out; sg.w = static_cast<const __nv_bfloat16*>(w); sg.cos_t = c; sg.sin_t = s;
         sg.rows = rows; sg.ld_in = ld_in; sg.ld_out = ld_out; sg.T = T > 0 ? T : 1;
-        sg.block0 = pp.blocks;
-        pp.blocks += (unsigned)((rows + (long long)PREP_WARPS - 1) / PREP_WARPS);
     }
     long long rows() const {
         long long n = 0;
         for (int i = 0; i < pp.nseg; i++) n += pp.seg[i].rows;
         return n;
     }
+    // thread blocks of `n` rows each, over all tensors
+    unsigned lay_out(int n) {
+        pp.blocks = 0;
+        for (int i = 0; i < pp.nseg; i++) {
+            pp.seg[i].block0 = pp.blocks;
+            pp.blocks += (unsigned)((pp.seg[i].rows + (long long)n - 1) / n);
+        }
+        return pp.blocks;
+    }
 };
 
 template <typename InT, typename OutT>
-int launch_prep_t(DeviceState* st, const PrepBatch& pb, cudaStream_t stream) {
+int launch_prep_t(DeviceState* st, PrepBatch& pb, cudaStream_t stream) {
     // Pieces per lane (prep.cuh has what they measured): four of 16 bytes, two of 32; one where all of it is a few rows, as a lane with
     // less to do is done sooner
     constexpr int MANY = sizeof(InT) == 2 ? 4 : 2;
     bool rope = false;
     for (int i = 0; i < pb.pp.nseg; i++) rope = rope || pb.pp.seg[i].cos_t;
     const int np = rope || pb.rows() * pb.pp.H >= 64LL * st->sm_count ? MANY : 1;
-    const int groups = (pb.pp.H + 2 * np - 1) / (2 * np);
-    const dim3 grid(pb.pp.blocks, (unsigned)(groups < 65535 ? groups : 65535)), block(PREP_THREADS);
+    const int groups = (pb.pp.H + prep_heads(np) - 1) / prep_heads(np);
+    const dim3 grid(pb.lay_out(prep_rows(np)), (unsigned)(groups < 65535 ? groups : 65535)), block(PREP_THREADS);
     if (np == 1) return launch_dependent(qk_prep_kernel<InT, OutT, 1>, grid, block, 0, stream, nullptr, pb.pp);
     return launch_dependent(qk_prep_kernel<InT, OutT, MANY>, grid, block, 0, stream, nullptr, pb.pp);
 }
 
-int launch_prep(DeviceState* st, const PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {
-    if (pb.pp.blocks == 0) {
+int launch_prep(DeviceState* st, PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {
+    if (pb.rows() == 0) {
         // nothing to stage: the words still have to be cleared before the attention kernel starts
         if (pb.pp.zero_n > 0) return launch_dependent(zero_words_kernel, dim3(1), dim3(256), 0, stream, nullptr, pb.pp.zero_ptr, pb.pp.zero_n);
         return KB_OK;

@@ -108,14 +108,18 @@ __global__ void zero_words_kernel(unsigned int* ptr, int n) {
 // lanes there are. Measured on B200 with three sets of inputs in turn, whole attention call, one piece per lane (two with RoPE) -> this:
 // self-attention with norm and RoPE, bf16, 256 tokens 11.1 -> 10.0 us, 1000 21.6 -> 20.7, 1536 39.5 -> 38.0, 4096 144.5 -> 141.2 (NP 2: 10.2,
 // 21.1, 38.5, 142.1; NP 8: 10.9, 21.7, 38.2, 143.8); fp32, whose pieces are 32 bytes, NP 2: 1000 tokens 23.4 -> 23.4, gradients at 1024
-// 101.7 -> 100.0 (NP 4: 23.5, 100.0; 4096 tokens 151.8 -> 152.6); a context of 512 x 1024 fp32 for cross_kv 11.1 us with NP 1, 11.5 with 2.
-constexpr int PREP_WARPS = 4;                               // rows per thread block; blockIdx.y: which 2 NP heads of them
+// 101.7 -> 100.0 (NP 4: 23.5, 100.0; 4096 tokens 151.8 -> 152.6); a context of 512 x 1024 fp32 for cross_kv 11.1 us with NP 1, 11.5 with 2; NP 1
+// with the four warps of a block on one row 9.94 (fp32) and 9.95 (bf16), on four rows 10.37 and 9.90, half a warp per head (before) 10.18 and 10.05.
+constexpr int PREP_WARPS = 4;
+// A thread block takes four rows and 2 NP heads of them, or (NP = 1) 8 heads of one row; blockIdx.y: which heads
+__host__ __device__ constexpr int prep_rows(int np) { return np == 1 ? 1 : PREP_WARPS; }
+__host__ __device__ constexpr int prep_heads(int np) { return np == 1 ? 2 * PREP_WARPS : 2 * np; }
 constexpr int PREP_THREADS = 32 * PREP_WARPS;
 
 template <typename InT, typename OutT, int NP>
 __global__ void __launch_bounds__(PREP_THREADS)
 qk_prep_kernel(const __grid_constant__ PrepParams pp) {
-    constexpr int HEADS = 2 * NP, NI = NP > 1 ? NP / 2 : 1;
+    constexpr int ROWS = prep_rows(NP), HEADS = prep_heads(NP), NI = NP > 1 ? NP / 2 : 1;
     pdl_launch();
     pdl_wait();
     if (blockIdx.x == 0 && blockIdx.y == 0)
@@ -126,12 +130,12 @@ qk_prep_kernel(const __grid_constant__ PrepParams pp) {
         if (i < pp.nseg && blockIdx.x >= pp.seg[i].block0) si = i;
     const PrepSeg& sg = pp.seg[si];
     const int lane = threadIdx.x & 31;
-    const unsigned row = PREP_WARPS * (blockIdx.x - sg.block0) + (threadIdx.x >> 5);
+    const unsigned row = ROWS * (blockIdx.x - sg.block0) + (ROWS > 1 ? threadIdx.x >> 5 : 0u);
     if (row >= (unsigned)sg.rows) return;
     const int r = (int)row;
     const InT* const src = static_cast<const InT*>(sg.in) + (size_t)r * sg.ld_in;
     OutT* const dst = static_cast<OutT*>(sg.out) + (size_t)r * sg.ld_out;
-    for (int h0 = (int)blockIdx.y * HEADS; h0 < pp.H; h0 += (int)gridDim.y * HEADS) {   // one round up to 65535 groups of heads
+    for (int h0 = (int)blockIdx.y * HEADS + (ROWS > 1 ? 0 : 2 * (int)(threadIdx.x >> 5)); h0 < pp.H; h0 += (int)gridDim.y * HEADS) {   // one round up to 65535 groups of heads
         if (NP > 1 && sg.cos_t) {
             const int sub = lane & 7, hl = h0 + (lane >> 3);     // heads hl, hl + 4, ...
             Raw8<InT> ra[NI], rb[NI];
