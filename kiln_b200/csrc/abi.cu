@@ -222,16 +222,15 @@ struct PrepBatch {
 
 template <typename InT, typename OutT>
 int launch_prep_t(DeviceState* st, PrepBatch& pb, cudaStream_t stream) {
-    // Pieces per lane (prep.cuh has what they measured): four of 16 bytes, two of 32; one where all of it is a few rows, as a lane with
-    // less to do is done sooner
     constexpr int MANY = sizeof(InT) == 2 ? 4 : 2;
     bool rope = false;
     for (int i = 0; i < pb.pp.nseg; i++) rope = rope || pb.pp.seg[i].cos_t;
-    const int np = rope || pb.rows() * pb.pp.H >= 64LL * st->sm_count ? MANY : 1;
-    const int groups = (pb.pp.H + prep_heads(np) - 1) / prep_heads(np);
-    const dim3 grid(pb.lay_out(prep_rows(np)), (unsigned)(groups < 65535 ? groups : 65535)), block(PREP_THREADS);
-    if (np == 1) return launch_dependent(qk_prep_kernel<InT, OutT, 1>, grid, block, 0, stream, nullptr, pb.pp);
-    return launch_dependent(qk_prep_kernel<InT, OutT, MANY>, grid, block, 0, stream, nullptr, pb.pp);
+    const PrepLayout l = prep_layout(pb.rows() * pb.pp.H, pb.pp.H, sizeof(InT) == 4, rope, st->sm_count);
+    for (pb.pp.heads_log2 = 0; 1 << pb.pp.heads_log2 < l.heads; ++pb.pp.heads_log2) {}
+    const dim3 grid(pb.lay_out(l.rows), (unsigned)(l.groups < 65535 ? l.groups : 65535)), block(PREP_THREADS);
+    return launch_dependent(l.np == 1 ? (l.few ? qk_prep_few_kernel<InT, OutT, 1> : qk_prep_kernel<InT, OutT, 1>)
+                                      : (l.few ? qk_prep_few_kernel<InT, OutT, MANY> : qk_prep_kernel<InT, OutT, MANY>),
+                            grid, block, 0, stream, nullptr, pb.pp);
 }
 
 int launch_prep(DeviceState* st, PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "ptx.cuh"
+#include "routes.h"
 
 namespace kb {
 
@@ -87,6 +88,7 @@ struct PrepSeg {
 struct PrepParams {
     PrepSeg seg[5];
     int nseg, H;
+    int heads_log2;              // qk_prep_few_kernel: log2 of PrepLayout::heads
     float eps;
     unsigned blocks;             // total thread blocks
     unsigned int* zero_ptr;      // optional: zero_n words the first thread block clears (counters and flags that the
@@ -110,16 +112,12 @@ __global__ void zero_words_kernel(unsigned int* ptr, int n) {
 // 21.1, 38.5, 142.1; NP 8: 10.9, 21.7, 38.2, 143.8); fp32, whose pieces are 32 bytes, NP 2: 1000 tokens 23.4 -> 23.4, gradients at 1024
 // 101.7 -> 100.0 (NP 4: 23.5, 100.0; 4096 tokens 151.8 -> 152.6); a context of 512 x 1024 fp32 for cross_kv 11.1 us with NP 1, 11.5 with 2; NP 1
 // with the four warps of a block on one row 9.94 (fp32) and 9.95 (bf16), on four rows 10.37 and 9.90, half a warp per head (before) 10.18 and 10.05.
-constexpr int PREP_WARPS = 4;
-// A thread block takes four rows and 2 NP heads of them, or (NP = 1) 8 heads of one row; blockIdx.y: which heads
-__host__ __device__ constexpr int prep_rows(int np) { return np == 1 ? 1 : PREP_WARPS; }
-__host__ __device__ constexpr int prep_heads(int np) { return np == 1 ? 2 * PREP_WARPS : 2 * np; }
-constexpr int PREP_THREADS = 32 * PREP_WARPS;
+constexpr int PREP_THREADS = 32 * PREP_WARPS;   // routes.h (PrepLayout) says what a thread block takes
 
 template <typename InT, typename OutT, int NP>
 __global__ void __launch_bounds__(PREP_THREADS)
 qk_prep_kernel(const __grid_constant__ PrepParams pp) {
-    constexpr int ROWS = prep_rows(NP), HEADS = prep_heads(NP), NI = NP > 1 ? NP / 2 : 1;
+    constexpr int ROWS = prep_units(NP), HEADS = prep_heads(NP), NI = NP > 1 ? NP / 2 : 1;
     pdl_launch();
     pdl_wait();
     if (blockIdx.x == 0 && blockIdx.y == 0)
@@ -197,6 +195,105 @@ qk_prep_kernel(const __grid_constant__ PrepParams pp) {
                 for (int e = 0; e < 8; e++) x.v[e] = x.v[e] * rs * fw.v[e];
             }
             if (hl + 2 * i < pp.H) Io<OutT>::st8(dst + (hl + 2 * i) * 128 + 8 * sub, x);
+        }
+    }
+}
+
+// The same with few heads, which would leave lanes of a unit (PrepLayout, which has both sides measured) idle: a unit takes 2^heads_log2 heads,
+// a divisor of H, of each of several rows. A kernel of its own: written as one with the above, its places cost that one 3 % of cross_kv
+// (fp32, 512 rows 9.85 -> 10.15 us).
+template <typename InT, typename OutT, int NP>
+__global__ void __launch_bounds__(PREP_THREADS)
+qk_prep_few_kernel(const __grid_constant__ PrepParams pp) {
+    constexpr int UNITS = prep_units(NP), HEADS = prep_heads(NP), NI = NP > 1 ? NP / 2 : 1;
+    pdl_launch();
+    pdl_wait();
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < pp.zero_n; i += PREP_THREADS) pp.zero_ptr[i] = 0u;
+    int si = 0;
+#pragma unroll
+    for (int i = 1; i < 5; i++)
+        if (i < pp.nseg && blockIdx.x >= pp.seg[i].block0) si = i;
+    const PrepSeg& sg = pp.seg[si];
+    const int lane = threadIdx.x & 31;
+    const int hs = pp.heads_log2, step = 1 << hs;
+    const unsigned row0 = (UNITS * (blockIdx.x - sg.block0) + (NP > 1 ? threadIdx.x >> 5 : 0u)) * (unsigned)(HEADS >> hs);
+    if (row0 >= (unsigned)sg.rows) return;
+    const int last = sg.rows - 1 - (int)row0;                    // last row, from the unit's first on
+    const InT* const src = static_cast<const InT*>(sg.in) + (size_t)row0 * sg.ld_in;
+    OutT* const dst = static_cast<OutT*>(sg.out) + (size_t)row0 * sg.ld_out;
+    const int k_warp = NP > 1 ? 0 : 2 * (int)(threadIdx.x >> 5);  // a warp's first pair of the unit
+    for (int h0 = (int)blockIdx.y * step; h0 < pp.H; h0 += (int)gridDim.y * step) {   // one round up to 65535 groups of heads
+        // pair k of the unit: its row, its place in the tensor, and is it one (past the last row or head: read again, not stored)
+        auto row_of = [&](int k) { return min(k >> hs, last); };
+        auto at = [&](int k, int ld) { return (size_t)row_of(k) * ld + (h0 + (k & (step - 1))) * 128; };
+        auto live = [&](int k) { return (k >> hs) <= last; };
+        if (NP > 1 && sg.cos_t) {
+            const int sub = lane & 7, k0 = lane >> 3;            // pairs k0, k0 + 4, ...
+            Raw8<InT> ra[NI], rb[NI];
+#pragma unroll
+            for (int i = 0; i < NI; i++) {
+                ra[i] = Io<InT>::raw8(src + at(k0 + 4 * i, sg.ld_in) + 8 * sub);
+                rb[i] = Io<InT>::raw8(src + at(k0 + 4 * i, sg.ld_in) + 64 + 8 * sub);
+            }
+            F8 c, s;
+            auto table = [&](int k) {
+                const size_t tr = (size_t)((row0 + (unsigned)row_of(k)) % (unsigned)sg.T) * 64 + 8 * sub;
+                c = Io<float>::ld8(sg.cos_t + tr);
+                s = Io<float>::ld8(sg.sin_t + tr);
+            };
+            table(k0);
+            Raw8<__nv_bfloat16> wa, wb;
+            if (sg.w) { wa = Io<__nv_bfloat16>::raw8(sg.w + 8 * sub); wb = Io<__nv_bfloat16>::raw8(sg.w + 64 + 8 * sub); }
+#pragma unroll
+            for (int i = 0; i < NI; i++) {
+                if (i > 0) table(k0 + 4 * i);
+                F8 a = Io<InT>::f8(ra[i]), b = Io<InT>::f8(rb[i]);
+                if (sg.w) {
+                    float ss = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) ss += a.v[e] * a.v[e] + b.v[e] * b.v[e];
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                    const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
+                    const F8 fa = Io<__nv_bfloat16>::f8(wa), fb = Io<__nv_bfloat16>::f8(wb);
+#pragma unroll
+                    for (int e = 0; e < 8; e++) { a.v[e] = a.v[e] * rs * fa.v[e]; b.v[e] = b.v[e] * rs * fb.v[e]; }
+                }
+                F8 x, y;
+#pragma unroll
+                for (int e = 0; e < 8; e++) {                    // engine/src/kernels.cu:769-771
+                    x.v[e] = a.v[e] * c.v[e] - b.v[e] * s.v[e];
+                    y.v[e] = b.v[e] * c.v[e] + a.v[e] * s.v[e];
+                }
+                if (live(k0 + 4 * i)) {
+                    Io<OutT>::st8(dst + at(k0 + 4 * i, sg.ld_out) + 8 * sub, x);
+                    Io<OutT>::st8(dst + at(k0 + 4 * i, sg.ld_out) + 64 + 8 * sub, y);
+                }
+            }
+            continue;
+        }
+        const int sub = lane & 15, k0 = (lane >> 4) + k_warp;   // pairs k0, k0 + 2, ...
+        Raw8<InT> rx[NP];
+#pragma unroll
+        for (int i = 0; i < NP; i++) rx[i] = Io<InT>::raw8(src + at(k0 + 2 * i, sg.ld_in) + 8 * sub);
+        Raw8<__nv_bfloat16> w;
+        if (sg.w) w = Io<__nv_bfloat16>::raw8(sg.w + 8 * sub);
+#pragma unroll
+        for (int i = 0; i < NP; i++) {
+            F8 x = Io<InT>::f8(rx[i]);
+            if (sg.w) {                                           // block-uniform
+                float ss = 0.f;
+#pragma unroll
+                for (int e = 0; e < 8; e++) ss += x.v[e] * x.v[e];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float rs = rsqrtf(ss * (1.f / 128.f) + pp.eps);
+                const F8 fw = Io<__nv_bfloat16>::f8(w);
+#pragma unroll
+                for (int e = 0; e < 8; e++) x.v[e] = x.v[e] * rs * fw.v[e];
+            }
+            if (live(k0 + 2 * i)) Io<OutT>::st8(dst + at(k0 + 2 * i, sg.ld_out) + 8 * sub, x);
         }
     }
 }

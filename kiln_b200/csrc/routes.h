@@ -4,6 +4,12 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#ifdef __CUDACC__
+#define KB_HOST_DEVICE __host__ __device__   // what the kernels are built from as well
+#else
+#define KB_HOST_DEVICE
+#endif
+
 namespace kb {
 
 #ifndef KB_SPLIT_MARGIN
@@ -71,6 +77,39 @@ inline bool share_bytes(const MatBytes& x, const MatBytes& y) {
 // head) of the output lies exactly on its own Q, which only the item itself reads.
 inline bool q_survives_output(const MatBytes& q, const MatBytes& out) {
     return !share_bytes(q, out) || (q.p == out.p && q.stride == out.stride && q.width == out.width);
+}
+
+// Pre-pass: what a thread block takes. A unit is a warp, or with np = 1 the thread block; it takes prep_heads(np) (row, head) pairs of one row,
+// or with few heads those of several rows. np: pieces of eight elements per lane, four of 16 bytes or two of 32; one where all of it is a few
+// rows, as a lane with less to do is done sooner (never with RoPE, whose lanes hold two pieces).
+// The line between few rows and many, 64 pairs per SM (9472), lies where neither is the better one for long. Measured on B200, back to back,
+// many -> one: cross_kv, whose context has 8 heads, 512 rows fp32 10.2 -> 9.9 us, bf16 10.3 -> 9.9, 1024 rows 16.0 -> 15.6, 15.7 -> 15.4, 1184 (here)
+// 21.2 -> 20.9, 20.8 -> 20.4, 2368 29.9 -> 30.6, 29.0 -> 28.6, 3000 34.0 -> 33.9, 32.5 -> 33.3; self-attention, 16 heads, three tensors, plain:
+// 256 tokens 11.5 -> 11.4, 9.5 -> 9.6, 500 (24000 pairs) 14.4 -> 15.4, 12.3 -> 12.3, 1000 22.9 -> 23.5, 17.3 -> 18.9, 1536 40.7 -> 41.7, 32.7 -> 34.8.
+constexpr int PREP_WARPS = 4;
+KB_HOST_DEVICE constexpr int prep_units(int np) { return np == 1 ? 1 : PREP_WARPS; }
+KB_HOST_DEVICE constexpr int prep_heads(int np) { return np == 1 ? 2 * PREP_WARPS : 2 * np; }
+struct PrepLayout {
+    int np;
+    bool few;          // few heads (qk_prep_few_kernel)
+    int heads;         // of a row, in a unit; few: the largest power of two that divides H, so that no lane is idle
+    int rows, groups;  // rows of a thread block; thread blocks side by side that take a row's heads
+};
+// Few: where more than 3/8 of a unit's lanes would be idle, with RoPE 1/2 (there a row's table values serve two of its heads), of a unit of four
+// heads 1/4. Measured on B200, back to back, a row to a unit -> few (half a warp per pair, which knows no rows), pre-pass alone, plain: 4096
+// rows, 1 head fp32 4.7 -> 1.8 us (2.0), bf16 4.7 -> 1.5 (1.9), 2 heads fp32 4.7 -> 2.0 (2.2), 2048 rows, 4 heads bf16 2.5 -> 1.8 (2.1); RoPE,
+// 8192 rows, 2 heads fp32 4.1 -> 3.1 (3.9), bf16 4.9 -> 3.2 (4.0), 5 heads fp32 7.9 -> 6.5 (6.3); the other way RoPE bf16, 4 heads, 512 rows
+// 1.8 -> 2.1 (2.1), 4096 rows 3.0 -> 3.2 (3.9). Self-attention, plain, 1 head, 1536 tokens fp32 24.0 -> 20.3 (20.2), 4096 tokens bf16 44.9 -> 38.1
+// (38.2), 2 heads, 1000 tokens fp32 18.8 -> 16.6 (16.8).
+inline PrepLayout prep_layout(long long pairs, int H, bool in32, bool rope, int sm_count) {
+    const int np = rope || pairs >= 64LL * sm_count ? (in32 ? 2 : 4) : 1, all = prep_heads(np), lanes = (H + all - 1) / all * all;
+    PrepLayout l = {np, 8 * (lanes - H) > (all == 4 ? 2 : rope ? 4 : 3) * lanes, all, prep_units(np), lanes / all};
+    if (l.few) {
+        while (H % l.heads) l.heads /= 2;
+        l.rows *= all / l.heads;
+        l.groups = H / l.heads;
+    }
+    return l;
 }
 
 // GEMM: CTA pairs on 256x256 tiles when that fills the device better. Measured on B200 a CTA of a pair spends about 11/8 of the

@@ -323,12 +323,9 @@ def test_qk_prep_vs_reference_kernels_golden(kb, golden):
     assert kb.check_status() == 0
 
 
-@pytest.mark.parametrize("H", [1, 3, 8, 9, 17])
-@pytest.mark.parametrize("rows", [1, 6, 333, 3001])
-def test_qk_prep_head_and_row_remainders(kb, H, rows):
-    """Heads that no group of 2, 4 or 8 divides, a last thread block with fewer rows, tables shorter than the rows, every form of the
-    kernel, padding left alone. Reference in float64; bounds: one rounding of the result, and fp32 arithmetic in front of it (norm: a
-    sum of 128 squares, then three products and a sum: below 2^-19 of the largest value of a row)."""
+def _check_qk_prep(kb, H, rows):
+    """Every form of the kernel on rows x H heads, padding left alone. Reference in float64; bounds: one rounding of the result, and fp32
+    arithmetic in front of it (norm: a sum of 128 squares, then three products and a sum: below 2^-19 of the largest value of a row)."""
     g = torch.Generator(device="cuda").manual_seed(rows * 31 + H)
     T = max(1, rows - 2)
     w = (1 + 0.1 * torch.randn(128, generator=g, device="cuda")).bfloat16()
@@ -353,6 +350,19 @@ def test_qk_prep_head_and_row_remainders(kb, H, rows):
                 ulp = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}[ot]
                 bound = y.abs() * ulp + y.abs().amax(1, keepdim=True) * 2.0 ** -19 + 2.0 ** -24
                 assert ((full[:, :H * 128].double() - y).abs() <= bound).all(), (it, ot, norm, rope)
+
+
+@pytest.mark.parametrize("H", [1, 3, 8, 9, 17])
+@pytest.mark.parametrize("rows", [1, 6, 333, 3001])
+def test_qk_prep_head_and_row_remainders(kb, H, rows):
+    """Heads that no group of 2, 4 or 8 divides, a last thread block with fewer rows, tables shorter than the rows."""
+    _check_qk_prep(kb, H, rows)
+
+
+@pytest.mark.parametrize("H,rows", [(1, 9473), (2, 4737), (4, 2369), (3, 3200), (9, 1053), (5, 1895), (2, 4735), (4, 7)], ids=str)
+def test_qk_prep_few_heads(kb, H, rows):
+    """Units of several rows of few heads, with many pieces per lane (from 9472 pairs on) and with one; a last unit of fewer rows."""
+    _check_qk_prep(kb, H, rows)
 
 
 def test_self_config4_full_size(kb):

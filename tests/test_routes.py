@@ -32,6 +32,9 @@ def rules(tmp_path_factory):
                    '    const int mc[3] = {0, mc2, mc4}; const kb::GemmShape g = kb::gemm_shape(M, N, ksteps, n_seg, any, 148, mc); return g.pair * 8 + g.split; }\n'
                    'extern "C" int width(int M, int N, int ksteps, int any) {\n'
                    '    const int mc[3] = {0, 74, 37}; return kb::gemm_shape(M, N, ksteps, 1, false, 148, mc, any).width; }\n'
+                   'extern "C" void prep(int rows, int H, int in32, int rope, int* out) {\n'
+                   '    const kb::PrepLayout l = kb::prep_layout((long long)rows * H, H, in32, rope, 148);\n'
+                   '    out[0] = l.np; out[1] = l.few; out[2] = l.heads; out[3] = l.rows; out[4] = l.groups; }\n'
                    'extern "C" int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {\n'
                    '    return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth}); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
@@ -104,3 +107,19 @@ def test_narrow_gemm_tiles_where_they_measured_faster(rules):
         assert rules.width(M, N, ksteps, 1) == (256, 224, 192)[times.index(min(times))], (M, N, ksteps)
         assert rules.width(M, N, ksteps, 0) in (128, 256)            # the head epilogue has no narrow tiles
     assert rules.width(128, 8192, 32, 1) == 128
+
+
+def test_the_pre_pass_leaves_few_lanes_idle(rules):
+    """However few heads there are: a thread block's 2 np pairs per warp are (row, head) pairs of the tensor, up to 3/8 of them (RoPE 1/2)
+    and up to the rows that a last thread block lacks; of few heads all of them."""
+    for H in range(1, 70):
+        for rows in (1, 100, 3000, 40000):
+            for in32 in (0, 1):
+                for rope in (0, 1):
+                    out = (ctypes.c_int * 5)()
+                    rules.prep(rows, H, in32, rope, out)
+                    np_, few, heads, block_rows, groups = out
+                    assert np_ == ((2 if in32 else 4) if rope or rows * H >= 64 * SMS else 1)
+                    assert block_rows * heads == 4 * 2 * np_                       # what its four warps can take
+                    assert groups * heads >= H and (groups - 1) * heads < H
+                    assert 8 * (groups * heads - H) <= (4 if rope else 3) * groups * heads and (not few or groups * heads == H)
