@@ -438,12 +438,17 @@ gemm16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ G
                     }
                     // The 32 rows of the chunk go through shared memory as swizzled boxes and leave by TMA (measured: 32 row stores per
                     // warp took 3 us, the issue rate of plain global stores from eight warps; the bulk copy takes them off the warp).
-                    // Behind the last tile the ring is free (unless other parts of a cut k range read it): a place for every box of the
-                    // warp, and nobody waits for one to be read.
-                    const bool in_ring = !SPLIT && w + n_groups >= n_tiles;
+                    // Behind the last tile the ring is free, of a cut k range (one tile per CTA) beyond what the other parts read there: a place
+                    // for every box of the warp, and nobody waits for one to be read. Of a pair with a cut range half of the warps finish rows.
+                    // (The cut ranges through the staging area, residual, N 2048, back to back: K 2048, M 128 9.2 us, here 9.0, M 300 9.9 -> 9.6,
+                    // M 384 9.9 -> 9.6; K 8192, M 1024, pairs, 37.0 -> 36.6.)
+                    const bool in_ring = SPLIT || w + n_groups >= n_tiles;
+                    constexpr int READ_BY_PARTS = SPLIT ? BN / 4 * GB_M * 16 : 0;
+                    static_assert(READ_BY_PARTS + (SPLIT && PAIR ? 4 : 8) * 4 * 4096 <= G_STAGES * G_STAGE_BYTES, "four places per warp");
+                    const uint32_t place = READ_BY_PARTS + (SPLIT && PAIR ? (warp >> 2) * 2 + (warp & 1) : warp) * 4 * 4096;
 #pragma unroll
                     for (int b = 0; b < BOXES; b++) {
-                        uint8_t* const box = in_ring ? smem + (warp * 4 + (ch >> 1) * BOXES + b) * 4096 : my_stage + (SLOTS == 2 ? box_use * BOX_BYTES : 0);
+                        uint8_t* const box = in_ring ? smem + place + ((ch >> 1) * BOXES + b) * 4096 : my_stage + (SLOTS == 2 ? box_use * BOX_BYTES : 0);
                         if (!in_ring) {
                             if (lane == 0) { if (SLOTS == 2) tma_store_wait_read_1(); else tma_store_wait_read(); }   // the box that was here has been read
                             box_use ^= 1;
