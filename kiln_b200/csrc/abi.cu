@@ -737,7 +737,7 @@ int linear16_segments(void* const* C, int ldc, const void* A, int lda, const voi
     if ((rc = get_state(&st))) return rc;
     // F16, HEADS16: the epilogues that a launch of several projections and a call per projection both have
     const bool any_n_seg = (epi == KB_EPI_HEADS16 || epi == KB_EPI_F16) && N % 128 == 0;
-    const GemmShape g = gemm_shape(M, N, K / GB_K, n_seg, any_n_seg, st->sm_count, st->max_clusters, epi != KB_EPI_HEADS16);
+    const GemmShape g = gemm_shape(M, N, K / GB_K, n_seg, any_n_seg, st->sm_count, st->max_clusters, epi != KB_EPI_HEADS16, epi == KB_EPI_GELU16);
     const bool narrow = g.pair && g.width != 256;
     const int w_rows = narrow ? g.width / 2 : 128;               // W rows per load
     CUtensorMap ta;

@@ -6,11 +6,11 @@
 // loads its own 128 rows of A and 128 of the 256 W rows per 64-wide k step (32 KiB) and keeps its 128x256 half of the
 // accumulator, so a CTA moves half the shared-memory bytes per flop of the single-CTA shape. That matters because
 // measured on B200 a 128x128 single-CTA tile is bound by shared-memory bandwidth (TMA writes plus operand reads,
-// about 100 B/clk/SM), not by the tensor pipe. Single: one CTA per 128x128 tile, for N not a multiple of 256, M <= 128,
-// or when the pair shape would fill the device worse (the host decides).
+// about 100 B/clk/SM), not by the tensor pipe. Single: one CTA per 128x128 tile, for M <= 128 or when the pair shapes would
+// fill the device worse, and where N is no multiple of 256 and the k range is short (the host decides).
 //
-// NARROW: the same pair on 224 or 192 columns, where that fills a round of tiles better (gemm_shape in routes.h has the rule and both sides
-// measured). Each CTA then loads 112 or 96 W rows per k step, and a tile leaves in chunks of 32 columns: one fp32 box of 128-byte rows,
+// NARROW: the same pair on 224 or 192 columns, of any N, where that fills the rounds of tiles better (gemm_shape in routes.h has the rule and
+// both sides measured). Each CTA then loads 112 or 96 W rows per k step, and a tile leaves in chunks of 32 columns: one fp32 box of 128-byte rows,
 // or one fp16 box of 64-byte rows. Not for the head epilogue, whose tiles are whole heads.
 //
 // Split K (p.split_k = 2 or 4): with fewer tiles than half of the SMs the k steps of a tile are cut into split_k ranges, one CTA (or

@@ -119,46 +119,66 @@ inline PrepLayout prep_layout(long long pairs, int H, bool in32, bool rope, int 
 // the epilogue of twice the columns). Measured on B200 inside a CUDA graph, whole k range -> split (* without dependent launches,
 // which save 1.5 us): N 2048, K 8192: M 128 40.2* -> 16.3 us, 512 40.8* -> 25.3, 1024 41.6* -> 29.1; N 2048, K 2048: M 128 14.4* -> 9.2,
 // 512 15.0* -> 11.0; with M 1024 (pairs, head epilogue) 14.7 -> 17.1, so not taken there. N 96 (a stacked LoRA), K 2048, M 1536: 13.4* -> 10.1.
-//
-// Narrow tiles: a CTA pair takes 224 or 192 columns where whole rounds of 256 would leave SMs without a tile. A k step takes in proportion
-// to the width (330, 285, 240 ns in a round that is not full), so the rounds decide. Measured on B200 inside a CUDA graph, 256 columns ->
-// the width taken: N 2048, K 2048 (residual): M 1536 18.8 -> 15.1 us (192: 66 tiles on 74 pairs, not 48), 1792 18.5 -> 16.6 (224), 2560 29.0 ->
-// 22.9 (192), 3456 29.3 -> 26.5 (224); K 8192: M 1536 48.4 -> 40.9, 3456 96.7 -> 95.0; N 8192, K 2048 (GELU): M 512 21.1 -> 18.4, 1024 31.3 ->
-// 28.0, 1536 42.8 -> 40.4, 3456 94.9 -> 92.8; the other way N 2048, K 2048, M 2048 18.8 (256) against 22.8 (224) and 22.4 (192).
-constexpr int SPLIT_K_COST = 560, SPLIT_K_COST_PAIR = 760;
+constexpr int SPLIT_K_COST = 70, SPLIT_K_COST_PAIR = 95;
 struct GemmShape {
     bool pair;
     int split;
     int width;   // columns of a tile
 };
-// The cheapest shape among those with `split` parts (0: any). max_clusters[1], [2]: resident clusters of 2 and 4 CTAs. any_width: the
-// epilogue has the narrow tiles (of a single matrix). unit: time of a k step, in eighths of the unit above.
-inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int split, int sm_count, const int* max_clusters, bool any_width = false) {
-    static constexpr struct { bool pair; int width, unit, max_split; } kinds[] = {{true, 256, 88, 2}, {true, 224, 78, 1}, {true, 192, 67, 1}, {false, 128, 64, 4}};
+// The cheapest shape among those with `split` parts (0: any). max_clusters[1], [2]: resident clusters of 2 and 4 CTAs.
+inline GemmShape gemm_cheapest(int M, int N, long long ksteps, int n_seg, int split, int sm_count, const int* max_clusters) {
     long long best = -1;
     GemmShape shape = {false, 1, 128};
-    for (const auto& kind : kinds) {
-        const bool narrow = kind.pair && kind.width != 256;
-        if (kind.pair && (M <= 128 || (narrow ? !any_width || n_seg > 1 : N % 256 != 0))) continue;
-        const int height = kind.pair ? 256 : 128;
-        const long long tiles = (long long)((M + height - 1) / height) * ((N + kind.width - 1) / kind.width) * n_seg;
-        const long long groups = kind.pair ? sm_count / 2 : sm_count;
-        for (int s = 1; s <= kind.max_split; s *= 2) {
-            if ((split && s != split) || (s > 1 && (ksteps < 2 * s || tiles > max_clusters[kind.pair ? s : s / 2]))) continue;
-            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + s - 1) / s) * kind.unit + (s == 1 ? 0 : kind.pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
-            if (best < 0 || cost < best) { best = cost; shape = {kind.pair, s, kind.width}; }
+    for (int pair = 1; pair >= 0; pair--) {
+        if (pair && (N % 256 || M <= 128)) continue;
+        const int tile = pair ? 256 : 128;
+        const long long tiles = (long long)((M + tile - 1) / tile) * ((N + tile - 1) / tile) * n_seg;
+        const long long unit = pair ? 11 : 8, groups = pair ? sm_count / 2 : sm_count;
+        for (int s = 1; s <= (pair ? 2 : 4); s *= 2) {
+            if ((split && s != split) || (s > 1 && (ksteps < 2 * s || tiles > max_clusters[pair ? s : s / 2]))) continue;
+            const long long cost = ((tiles + groups - 1) / groups) * ((ksteps + s - 1) / s) * unit + (s == 1 ? 0 : pair ? SPLIT_K_COST_PAIR : SPLIT_K_COST);
+            if (best < 0 || cost < best) { best = cost; shape = {pair != 0, s, tile}; }
         }
     }
     return shape;
+}
+
+// Narrow tiles: a CTA pair takes 224 or 192 columns where that is faster than the shape above. The cost of a launch whose k range is not cut, in
+// units of ~3.9 ns: k steps x time of one x rounds of tiles, a last round that is not full charged six tenths and four tenths of its part (in
+// long launches the thread blocks drift apart, and under the power cap time follows the work), and what a pair needs once more than a single
+// CTA for twice the rows (1.2 us: filling, a longer epilogue). GELU keeps the epilogue warps of the wide chunks (tiles of 256 and 128 columns)
+// busy longer than a k step's share of them, so those steps cost a tenth more. Measured on B200 with all widths forced, inside a CUDA graph, in
+// single calls with pauses; sustained the differences grow (GELU, M 4096: 123, 108, 122 us):
+//                          N 2048, residual                              N 8192, GELU (K 2048)
+//   M       1536  1792  2048  2560  3456  4096   K 8192: 1536  3456     512  1024  2304  3456  3840  4096  8192   F16: 1536  3456  3840  F32: 3456
+//   256     19.8  19.8  20.1  30.7  31.7  33.1           52.6  96.9    21.2  33.8  61.8  98.0 103.1 107.2 213.3        40.3  87.7  92.5       95.6
+//   224     18.1  18.4  24.6  28.3  29.7  37.2           46.8  94.9    19.1  29.4  61.4  89.1  98.0 102.4 202.9        38.6  85.7  94.9       93.2
+//   192     16.4  23.2  24.9  26.3  34.1  36.2           42.3 107.2    25.9  35.2  64.5  96.3 101.4 109.6 214.4        42.0  90.5  95.2       99.3
+// and M 1100, K 1024, F16, 128 columns 21.9, 192 20.8; where N is no multiple of 256 (M 1537, N 2056, F16), 128, 224 columns: K 64 5.1, 6.8 us, 512 8.5, 8.9, 1024 11.3, 11.3, 2048 17.8, 16.7.
+// The rule is within 3 % of the best width in each of 95 such measurements, 5.5 % sustained (tests/test_routes.py).
+constexpr int GEMM_PAIR_FIXED = 300;
+inline long long gemm_tile_cost(int M, int N, long long ksteps, int width, bool gelu, int sm_count) {
+    const bool pair = width != 128;
+    const int height = pair ? 256 : 128, unit = width == 256 ? (gelu ? 98 : 88) : width == 224 ? 80 : width == 192 ? 71 : gelu ? 64 : 59;
+    const long long tiles = (long long)((M + height - 1) / height) * ((N + width - 1) / width), groups = pair ? sm_count / 2 : sm_count;
+    return ksteps * unit * (6 * ((tiles + groups - 1) / groups) * groups + 4 * tiles) / groups + (pair ? 10 * GEMM_PAIR_FIXED : 0);
 }
 // n_seg weight matrices in one launch. any_n_seg: the outputs have to be the same to the bit whether the projections of an activation
 // share a launch or not. The number of parts is the order of the sums (the tile shape is not), so it is then the one that suits three
 // segments, for one and two as well: a split that would pay for a single projection only is left out (N 2048, K 2048: four parts up to
 // M 256, two up to M 512; up to M 128 two parts are left). What that costs the single call, head epilogue, device time: M 128
 // 9.1 us either way, M 256 10.2 -> 10.7, M 512 10.3 -> 11.1.
-inline GemmShape gemm_shape(int M, int N, long long ksteps, int n_seg, bool any_n_seg, int sm_count, const int* max_clusters, bool any_width = false) {
+inline GemmShape gemm_shape(int M, int N, long long ksteps, int n_seg, bool any_n_seg, int sm_count, const int* max_clusters, bool any_width = false,
+                            bool gelu = false) {
     const int split = any_n_seg ? gemm_cheapest(M, N, ksteps, 3, 0, sm_count, max_clusters).split : 0;
-    return gemm_cheapest(M, N, ksteps, n_seg, split, sm_count, max_clusters, any_width);
+    GemmShape g = gemm_cheapest(M, N, ksteps, n_seg, split, sm_count, max_clusters);
+    if (!any_width || n_seg > 1 || g.split > 1 || M <= 128) return g;
+    long long best = gemm_tile_cost(M, N, ksteps, g.width, gelu, sm_count);
+    for (int width = 224; width >= 192; width -= 32) {
+        const long long cost = gemm_tile_cost(M, N, ksteps, width, gelu, sm_count);
+        if (cost < best) { best = cost; g = {true, 1, width}; }
+    }
+    return g;
 }
 
 }  // namespace kb
