@@ -13,6 +13,7 @@ import torch
 
 import oracle
 from util_gpu import assert_close, dev, sample_rows, seeded
+from util_routes import SMS, linear16_width
 
 pytestmark = pytest.mark.gpu
 
@@ -224,12 +225,15 @@ def test_edge_shapes_every_epilogue(kb, M, N, K):
     assert np.all(np.abs(out - ref) <= 2.0 ** -10 * np.abs(ref) + 1e-4), f"{M}x{N}x{K} heads16: {np.abs(out - ref).max():.3e}"
 
 
-@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (4096, 16, 2048), (100, 2, 2048), (128, 16, 2048), (300, 16, 2048), (512, 16, 2048), (200, 16, 8192)],
-                         ids=["pair_tiles", "single_tiles", "dit_size", "four_parts", "two_parts", "split_for_one_only", "split_for_one_only_512", "long_k"])
+@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (4096, 16, 2048), (100, 2, 2048), (128, 16, 2048), (300, 16, 2048), (512, 16, 2048), (200, 16, 8192), (1536, 16, 2048),
+                                   (1792, 16, 2048)],
+                         ids=["pair_tiles", "single_tiles", "dit_size", "four_parts", "two_parts", "split_for_one_only", "split_for_one_only_512", "long_k",
+                              "one_call_on_192_columns", "one_call_on_224_columns"])
 def test_qkv_one_launch_equals_three_calls(kb, M, H, K):
     """kb_linear16_qkv: q and k with their own norm weights and RoPE, v plain — bit-identical to three kb_linear16 calls."""
     from kiln_b200 import ops
     N = H * 128
+    assert M not in (1536, 1792) or linear16_width(M, N, K, "F16") == {1536: 192, 1792: 224}[M]
     side = int(np.sqrt(M))
     dx = dev(seeded(300, M, K, "f16"), "f16")
     ws = [dev(seeded(301 + i, N, K, "f16", 1.0 / np.sqrt(K)), "f16") for i in range(3)]
@@ -372,7 +376,8 @@ def test_second_product_shapes(kb, M, N, K, K2):
     _close(c[torch.as_tensor(rows, device="cuda")].cpu().numpy(), ref, K + K2, f"{M}x{N}x{K}+{K2}", False)
 
 
-@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (128, 16, 2048), (300, 16, 2048)], ids=["pair_tiles", "single_tiles", "two_parts", "split_for_one_only"])
+@pytest.mark.parametrize("M,H,K", [(300, 2, 128), (333, 3, 192), (128, 16, 2048), (300, 16, 2048), (1536, 16, 2048), (1792, 16, 2048)],
+                         ids=["pair_tiles", "single_tiles", "two_parts", "split_for_one_only", "one_call_on_192_columns", "one_call_on_224_columns"])
 def test_qkv_lora_one_launch_equals_three_calls(kb, M, H, K):
     """kb_linear16_qkv_lora with a different rank per projection (none on v) — bit-identical to three kb_linear16_lora /
     kb_linear16 calls, and the head epilogue sees the LoRA-adjusted value (checked against the oracle on q)."""
@@ -423,8 +428,8 @@ def test_narrow_outputs_of_the_store_epilogues(kb, N):
 
 @pytest.mark.parametrize("M,N", [(128, 38400), (2561, 1920), (19001, 200)], ids=lambda v: str(v))
 def test_more_than_two_tiles_per_thread_block(kb, M, N):
-    """Beyond two tiles a thread block comes back to its first accumulator, which every epilogue warp has to have handed back: 300 tiles
-    of 128 x 128, and two or three rounds of narrow tiles of CTA pairs. Fp64 reference of the same product, bounds as elsewhere."""
+    """Beyond two tiles a thread block comes back to its first accumulator, which every epilogue warp has to have handed back: 300, 315 and
+    298 tiles of 128 x 128. (Narrow tiles: the test below.) Fp64 reference of the same product, bounds as elsewhere."""
     from kiln_b200 import ops
     K = 64
     x, w = seeded(700, M, K, "f16"), seeded(701, N, K, "f16", 1.0 / np.sqrt(K))
@@ -434,11 +439,36 @@ def test_more_than_two_tiles_per_thread_block(kb, M, N):
         _close(_run(kb, x, w, epi), r, K, f"M={M} N={N} epi {epi}", epi != ops.EPI_F32)
 
 
+@pytest.mark.parametrize("epi", ["F32", "F16", "GELU16", "RESID"])
+@pytest.mark.parametrize("M,width", [(1500, 224), (1270, 192)], ids=["224", "192"])
+def test_three_rounds_of_narrow_tiles(kb, epi, M, width):
+    """Three tiles per CTA pair, the third in the first one's accumulator; last row and column tiles that are cut (the residual takes whole
+    128 columns only); nothing written outside the matrix. Fp64 reference of the same product, bounds as elsewhere."""
+    from kiln_b200 import ops
+    N, K = (8192 if epi == "RESID" else 8104), 1024
+    assert linear16_width(M, N, K, epi) == width and -(-M // 256) * -(-N // width) > 2 * (SMS // 2)
+    assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
+    x, w = seeded(720, M, K, "f16"), seeded(721, N, K, "f16", 1.0 / np.sqrt(K))
+    ref = (dev(x).double() @ dev(w).double().T)
+    g = torch.Generator(device="cuda").manual_seed(722)
+    kw = {}
+    if epi == "GELU16":
+        ref = torch.nn.functional.gelu(ref)
+    if epi == "RESID":
+        gate, resid = torch.randn(N, generator=g, device="cuda"), torch.randn(M, N, generator=g, device="cuda")
+        ref = resid.double() + gate.double() * ref
+        kw = {"gate": gate.cpu().numpy(), "resid": resid.cpu().numpy()}
+    _close(_run(kb, x, w, getattr(ops, "EPI_" + epi), ldc_pad=64, **kw), ref.cpu().numpy(), K, f"{epi} {M}x{N}x{K}", epi in ("F16", "GELU16"))
+
+
 @pytest.mark.parametrize("M,N,K,epi", [(1281, 2048, 128, "RESID"), (1792, 2048, 192, "RESID"), (1300, 2048, 64, "F32"), (700, 1928, 64, "F16"), (400, 8192, 64, "GELU16"),
-                                       (257, 8000, 128, "GELU16"), (1537, 2056, 64, "F32")], ids=str)
+                                       (257, 8000, 128, "GELU16"), (1537, 2056, 64, "F32"), (1537, 2056, 1024, "F16"), (1537, 2056, 1024, "F32"),
+                                       (1500, 1928, 1024, "F16"), (257, 8000, 2048, "GELU16")], ids=str)
 def test_narrow_tiles(kb, M, N, K, epi):
-    """Tiles of 224 and 192 columns: last row and column tiles that are cut, every epilogue that has them, a second product; nothing
-    written outside the matrix. Fp64 reference of the same products, bounds as elsewhere."""
+    """Tiles of 224 and 192 columns: last row and column tiles that are cut, every epilogue that has them, a second product (and three short k
+    ranges whose N is no multiple of 256, which stay on single CTAs); nothing written outside the matrix. Fp64 reference of the same products,
+    bounds as elsewhere."""
+    assert (linear16_width(M, N, K, epi) in (192, 224)) == (N % 256 == 0 or K >= 1024)
     from kiln_b200 import ops
     e = getattr(ops, "EPI_" + epi)
     x, w = seeded(710, M, K, "f16"), seeded(711, N, K, "f16", 1.0 / np.sqrt(K))
@@ -468,6 +498,18 @@ def test_gelu_over_its_whole_range(kb):
     ref = (v * torch.special.ndtr(v)).numpy()
     assert np.all(np.abs(out - ref) <= np.abs(ref) * (2.0 ** -11 + 1e-6) + 2.0 ** -25 + 1e-9), np.abs(out - ref).max()
     assert np.array_equal(out[x >= 8], x[x >= 8].astype(np.float64)) and not out[x <= -8].any()
+
+
+def test_gelu_of_infinities_and_nan(kb):
+    """What the reference's expression gives: inf of inf, NaN of -inf and NaN; of sums that fp16 does not hold inf above and 0 below."""
+    from kiln_b200 import ops
+    x = np.zeros((128, 64), np.float32)
+    x[:5, 0] = [np.inf, -np.inf, np.nan, 65504.0, -65504.0]
+    for top, want in ((1.0, [np.inf, np.nan, np.nan, 65504.0, 0.0]), (65504.0, [np.inf, np.nan, np.nan, np.inf, 0.0])):
+        w = np.zeros((128, 64), np.float32)
+        w[:, 0] = top
+        out = _run(kb, x, w, ops.EPI_GELU16)
+        assert np.array_equal(out[:5], np.repeat(np.float32(want)[:, None], 128, 1), equal_nan=True), out[:5, 0]
 
 
 def test_lora_argument_errors(kb):

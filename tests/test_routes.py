@@ -1,11 +1,11 @@
-"""CPU tests of the rules that pick an attention call's schedule and a GEMM's tile shape (kiln_b200/csrc/routes.h, plain C++)."""
+"""CPU tests of the rules that pick an attention call's schedule, a GEMM's tile shape and what a thread block of the pre-pass takes
+(kiln_b200/csrc/routes.h, plain C++)."""
 import ctypes
-import os
-import subprocess
 
 import pytest
 
-CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "kiln_b200", "csrc")
+import util_routes
+
 WHOLE, BALANCED, KEYS = 0, 1, 2
 SMS = 148
 
@@ -75,24 +75,8 @@ WIDTHS = [  # epilogue, M, N, K, single calls, sustained
     ('F16', 1100, 8168, 1024, (22.4, 22.2, 21.2), (23.9, 24.0, 23.1)), ('GELU16', 1100, 8168, 1024, (27.0, 25.3, 24.2), (28.6, 26.4, 25.4))]
 
 @pytest.fixture(scope="module")
-def rules(tmp_path_factory):
-    d = tmp_path_factory.mktemp("routes")
-    src = d / "routes.cpp"
-    src.write_text('#include "routes.h"\n'
-                   'extern "C" int route(int B, int Tq, int Tk, int H, int sms, int keys, int room) { return kb::attn_route(B, Tq, Tk, H, sms, keys, room); }\n'
-                   'extern "C" int gemm(int M, int N, int ksteps, int n_seg, int any, int mc2, int mc4) {\n'
-                   '    const int mc[3] = {0, mc2, mc4}; const kb::GemmShape g = kb::gemm_shape(M, N, ksteps, n_seg, any, 148, mc); return g.pair * 8 + g.split; }\n'
-                   'extern "C" int width(int M, int N, int ksteps, int any_n_seg, int any, int gelu) {\n'
-                   '    const int mc[3] = {0, 74, 37}; return kb::gemm_shape(M, N, ksteps, 1, any_n_seg, 148, mc, any, gelu).width; }\n'
-                   'extern "C" void prep(int rows, int H, int in32, int rope, int* out) {\n'
-                   '    const kb::PrepLayout l = kb::prep_layout((long long)rows * H, H, in32, rope, 148);\n'
-                   '    out[0] = l.np; out[1] = l.few; out[2] = l.heads; out[3] = l.rows; out[4] = l.groups; }\n'
-                   'extern "C" int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {\n'
-                   '    return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth}); }\n')
-    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, "-o", str(d / "routes.so"), str(src)], check=True)
-    lib = ctypes.CDLL(str(d / "routes.so"))
-    lib.survives.argtypes = [ctypes.c_size_t] * 7
-    return lib
+def rules():
+    return util_routes.rules()
 
 
 @pytest.fixture(scope="module")
@@ -149,11 +133,11 @@ def test_raw_q_needs_an_output_that_leaves_it_alone(rules):
 
 
 @pytest.mark.parametrize("case", WIDTHS, ids=lambda c: "x".join(map(str, c[:4])))
-def test_narrow_gemm_tiles_where_they_measured_faster(rules, case):
+def test_narrow_gemm_tiles_where_they_measured_faster(case):
     """The width taken is the fastest of the three, within 3 % in single calls and 5.5 % sustained."""
     epi, M, N, K, single, sustained = case
     widths = (256, 224, 192) if N % 256 == 0 else (128, 224, 192)
-    w = widths.index(rules.width(M, N, K // 64, epi == "F16" and N % 128 == 0, 1, epi == "GELU16"))
+    w = widths.index(util_routes.linear16_width(M, N, K, epi))
     assert single[w] <= 1.03 * min(single) and sustained[w] <= 1.055 * min(sustained)
 
 
