@@ -228,9 +228,12 @@ int launch_prep_t(DeviceState* st, PrepBatch& pb, cudaStream_t stream) {
     const PrepLayout l = prep_layout(pb.rows() * pb.pp.H, pb.pp.H, sizeof(InT) == 4, rope, st->sm_count);
     for (pb.pp.heads_log2 = 0; 1 << pb.pp.heads_log2 < l.heads; ++pb.pp.heads_log2) {}
     const dim3 grid(pb.lay_out(l.rows), (unsigned)(l.groups < 65535 ? l.groups : 65535)), block(PREP_THREADS);
-    return launch_dependent(l.np == 1 ? (l.few ? qk_prep_few_kernel<InT, OutT, 1> : qk_prep_kernel<InT, OutT, 1>)
-                                      : (l.few ? qk_prep_few_kernel<InT, OutT, MANY> : qk_prep_kernel<InT, OutT, MANY>),
-                            grid, block, 0, stream, nullptr, pb.pp);
+    if (l.few) {
+        if (l.np == 1) return launch_dependent(qk_prep_few_kernel<InT, OutT, 1>, grid, block, 0, stream, nullptr, pb.pp);
+        return launch_dependent(qk_prep_few_kernel<InT, OutT, MANY>, grid, block, 0, stream, nullptr, pb.pp);
+    }
+    if (l.np == 1) return launch_dependent(qk_prep_kernel<InT, OutT, 1>, grid, block, 0, stream, nullptr, pb.pp);
+    return launch_dependent(qk_prep_kernel<InT, OutT, MANY>, grid, block, 0, stream, nullptr, pb.pp);
 }
 
 int launch_prep(DeviceState* st, PrepBatch& pb, int in_dtype, int out_dtype, cudaStream_t stream) {
