@@ -825,17 +825,6 @@ int kb_linear16_qkv_lora(void* const* C3, int ldc, const void* A, int lda, const
 // ------------------------------------------------------------------------------------------- attention backward
 namespace {
 size_t bwd_stats_bytes(int B, int Tq, int H) { return align256((size_t)B * H * ((Tq + 127) / 128) * 256 * sizeof(float)); }
-// How the dK/dV role cuts its query blocks when there are too few (key block, head, image) triples to fill the GPU
-// (cross-attention to a short context): parts of q_per query blocks each; 1 part = no cut.
-void bwd_qsplit(int B, int Tq, int Tk, int H, int sm_count, int* qsplit, int* q_per) {
-    const long long triples = (long long)B * H * ((Tk + 127) / 128);
-    const int nqb = (Tq + 127) / 128;
-    int want = (int)(sm_count / (triples > 0 ? triples : 1));
-    if (want > nqb) want = nqb;
-    if (want < 2) { *qsplit = 1; *q_per = nqb; return; }
-    *q_per = (nqb + want - 1) / want;
-    *qsplit = (nqb + *q_per - 1) / *q_per;
-}
 size_t bwd_partial_bytes(int B, int Tk, int H, int qsplit) { return qsplit > 1 ? 2 * align256((size_t)qsplit * B * Tk * H * 128 * sizeof(float)) : 0; }
 size_t bwd_fixed_bytes(int B, int Tq, int Tk, int H, int dtype) {
     // statistics; the room of an fp16 O. The forward pass leaves D itself and stores no O, so nothing reads or writes that room, but a

@@ -1,5 +1,5 @@
-// Which schedule an attention call takes and which tile shape a GEMM: rules on sizes only, plain host code (no CUDA headers), so that
-// they can be tested without a device.
+// Which schedule an attention call takes, how its backward cuts query ranges, which tile shape a GEMM takes and what a thread block of the
+// pre-pass: rules on sizes only, plain host code (no CUDA headers), so that they can be tested without a device.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -77,6 +77,18 @@ inline bool share_bytes(const MatBytes& x, const MatBytes& y) {
 // head) of the output lies exactly on its own Q, which only the item itself reads.
 inline bool q_survives_output(const MatBytes& q, const MatBytes& out) {
     return !share_bytes(q, out) || (q.p == out.p && q.stride == out.stride && q.width == out.width);
+}
+
+// Backward: how the dK/dV role cuts its query blocks when there are too few (key block, head, image) triples to fill the GPU
+// (cross-attention to a short context): parts of q_per query blocks each; 1 part = no cut.
+inline void bwd_qsplit(int B, int Tq, int Tk, int H, int sm_count, int* qsplit, int* q_per) {
+    const long long triples = (long long)B * H * ((Tk + 127) / 128);
+    const int nqb = (Tq + 127) / 128;
+    int want = (int)(sm_count / (triples > 0 ? triples : 1));
+    if (want > nqb) want = nqb;
+    if (want < 2) { *qsplit = 1; *q_per = nqb; return; }
+    *q_per = (nqb + want - 1) / want;
+    *qsplit = (nqb + *q_per - 1) / *q_per;
 }
 
 // Pre-pass: what a thread block takes. A unit is a warp, or with np = 1 the thread block; it takes prep_heads(np) (row, head) pairs of one row,

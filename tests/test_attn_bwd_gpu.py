@@ -16,6 +16,7 @@ import torch
 
 import oracle
 from util_gpu import assert_close, dev, sample_rows, seeded
+from util_routes import SMS, bwd_q_per
 
 pytestmark = pytest.mark.gpu
 
@@ -83,22 +84,37 @@ def test_many_query_tiles_and_several_key_blocks(kb, Tq, Tk, H, npad, B, kind):
             assert_close(g[sk][j0:, cs], r, f"{name} {Tq}x{Tk}x{H} image {b}", max_abs=2e-3 * max(1.0, float(np.sqrt((r * r).mean(1)).max())))
 
 
+def _check_against_float64(kb, B, Tq, Tk, H, seed):
+    """All of dq, dk and dv against float64 on the rounded operands. The bound is the one of the larger cases above: 2e-3 of the largest
+    row's rms."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, do = (torch.randn(B * Tq, H * 128, generator=g, device="cuda").half() for _ in range(2))
+    k, v = (torch.randn(B * Tk, H * 128, generator=g, device="cuda").half() for _ in range(2))
+    heads = lambda t: t.double().reshape(B, -1, H, 128).transpose(1, 2)
+    Q, K, V, G = map(heads, (q, k, v, do))
+    P = torch.softmax(Q @ K.transpose(2, 3) / 128 ** 0.5, -1)
+    dP = G @ V.transpose(2, 3)
+    dS = P * (dP - (dP * P).sum(-1, keepdim=True)) / 128 ** 0.5
+    refs = [x.transpose(1, 2).reshape(-1, H * 128).cpu().numpy() for x in (dS @ K, dS.transpose(2, 3) @ Q, P.transpose(2, 3) @ G)]
+    for name, out, ref in zip(("dq", "dk", "dv"), _run(kb, *(t.float().cpu().numpy() for t in (q, k, v, do)), B, Tq, Tk, 0, H, "f16"), refs):
+        assert np.abs(out - ref).max() <= 2e-3 * max(1.0, np.sqrt((ref * ref).mean(1)).max()), f"{name}: {np.abs(out - ref).max():.2e}"
+
+
 @pytest.mark.parametrize("nq,nk", [(1, 1), (1, 4), (2, 1), (2, 3), (3, 2), (3, 7), (4, 4), (5, 1), (5, 6), (7, 2)], ids=str)
 def test_every_phase_of_the_rings(kb, nq, nk):
-    """Numbers of streamed blocks around the depths of the two rings (three and two stages), in both roles and with ragged last blocks,
-    against float64 on the rounded operands. The bound is the one of the larger cases above: 2e-3 of the largest row's rms."""
-    H, Tq, Tk = 2, 128 * nq - 37, 128 * nk - 5
-    g = torch.Generator(device="cuda").manual_seed(10 * nq + nk)
-    q, do = (torch.randn(Tq, H * 128, generator=g, device="cuda").half() for _ in range(2))
-    k, v = (torch.randn(Tk, H * 128, generator=g, device="cuda").half() for _ in range(2))
-    heads = lambda t: t.double().reshape(t.shape[0], H, 128).transpose(0, 1)
-    Q, K, V, G = map(heads, (q, k, v, do))
-    P = torch.softmax(Q @ K.transpose(1, 2) / 128 ** 0.5, -1)
-    dP = G @ V.transpose(1, 2)
-    dS = P * (dP - (dP * P).sum(-1, keepdim=True)) / 128 ** 0.5
-    refs = [x.transpose(0, 1).reshape(-1, H * 128).cpu().numpy() for x in (dS @ K, dS.transpose(1, 2) @ Q, P.transpose(1, 2) @ G)]
-    for name, out, ref in zip(("dq", "dk", "dv"), _run(kb, *(t.float().cpu().numpy() for t in (q, k, v, do)), 1, Tq, Tk, 0, H, "f16"), refs):
-        assert np.abs(out - ref).max() <= 2e-3 * max(1.0, np.sqrt((ref * ref).mean(1)).max()), f"{name}: {np.abs(out - ref).max():.2e}"
+    """Numbers of streamed key blocks around the depths of the two rings (three and two stages) in the dQ role, with ragged last blocks; the
+    dK/dV role has so few key blocks here that each of its thread blocks streams one query block, the parts are summed behind it."""
+    assert bwd_q_per(1, 128 * nq - 37, 128 * nk - 5, 2) == 1
+    _check_against_float64(kb, 1, 128 * nq - 37, 128 * nk - 5, 2, 10 * nq + nk)
+
+
+@pytest.mark.parametrize("B,H,nq,nk,per", [(5, 16, n, 1, n) for n in range(1, 8)] + [(1, 16, 7, 2, 2), (1, 16, 10, 2, 3), (1, 16, 15, 2, 4), (1, 16, 18, 2, 5)], ids=str)
+def test_every_phase_of_the_rings_of_the_dkv_role(kb, B, H, nq, nk, per):
+    """The same in the dK/dV role, whose Q ring has no wait of its own but leans on the one of the dO ring a step before: one to seven query
+    blocks streamed by a thread block, with whole query ranges and with cut ones, the last of which is shorter. Every head's dk and dv."""
+    Tq, Tk = 128 * nq - 37, 128 * nk - 5
+    assert bwd_q_per(B, Tq, Tk, H) == per and torch.cuda.get_device_properties(0).multi_processor_count == SMS
+    _check_against_float64(kb, B, Tq, Tk, H, 100 * nq + per)
 
 
 def test_batch_equals_per_image_calls(kb):

@@ -25,6 +25,11 @@ void prep(int rows, int H, int in32, int rope, int* out) {
     const kb::PrepLayout l = kb::prep_layout((long long)rows * H, H, in32, rope, 148);
     out[0] = l.np; out[1] = l.few; out[2] = l.heads; out[3] = l.rows; out[4] = l.groups;
 }
+int q_per(int B, int Tq, int Tk, int H) {
+    int qsplit, q_per;
+    kb::bwd_qsplit(B, Tq, Tk, H, 148, &qsplit, &q_per);
+    return q_per;
+}
 int survives(size_t q, size_t rows, size_t stride, size_t width, size_t o, size_t ostride, size_t owidth) {
     return kb::q_survives_output({(void*)q, rows, stride, width}, {(void*)o, rows, ostride, owidth});
 }
@@ -47,3 +52,8 @@ def rules():
 def linear16_width(M, N, K, epi):
     """Columns of a tile of one linear16 call with epilogue "F32", "F16", "GELU16" or "RESID"."""
     return rules().width(M, N, K // 64, epi == "F16" and N % 128 == 0, 1, epi == "GELU16")
+
+
+def bwd_q_per(B, Tq, Tk, H):
+    """Query blocks that a thread block of the dK/dV role streams at most."""
+    return rules().q_per(B, Tq, Tk, H)
