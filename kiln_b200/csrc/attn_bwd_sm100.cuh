@@ -51,7 +51,7 @@ namespace kb {
 
 constexpr int BWD_DKV = 0, BWD_DQ = 1;
 constexpr int BWD_THREADS = 384;                              // warps 0-7 softmax / epilogue, 8 MMA issue, 9 TMA loads, 10-11 idle
-constexpr int BWD_SOFTMAX_REGS = 224, BWD_OTHER_REGS = 56;    // 384 x 168 = 256 x 224 + 128 x 56
+constexpr int BWD_SOFTMAX_REGS = 224, BWD_OTHER_REGS = 56;    // 384 x 168 = 256 x 224 + 128 x 56 (-Xptxas -v: 12 bytes of spill stores, 24 of loads)
 constexpr int BWD_X0_STAGES = 3, BWD_X1_STAGES = 2;           // of the streamed tiles: X0 (Q_i or K_j), X1 (dO_i or V_j, with the statistics)
 constexpr int BWD_STATS_BYTES = 1024;                         // the statistics of a query block
 constexpr int BWD_SMEM = (2 + BWD_X0_STAGES + BWD_X1_STAGES) * TILE_BYTES + BWD_X1_STAGES * BWD_STATS_BYTES + 1024;   // resident pair, rings, control block

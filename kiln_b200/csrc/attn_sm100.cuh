@@ -82,7 +82,7 @@ constexpr int ATTN_THREADS = 384;
 // threads of the MMA / TMA / helper warps x 56 = 64512 exactly (a larger second number would leave the softmax warps'
 // increase waiting forever). Spills matter more than usual here: with 227 KB of the SM's 256 KB configured as shared memory there is
 // almost no L1 left, so every spill access is an L2 round trip. At 224 -Xptxas -v reports none for MODE_KEYS and for MODE_PAIR with
-// stored outputs, 28 bytes of stores and 24 of loads for MODE_PAIR with RowStats, 52 and 44 for MODE_NAG with a 16-bit output.
+// stored outputs, 24 bytes of stores and 20 of loads for MODE_PAIR with RowStats, 52 and 44 for MODE_NAG with a 16-bit output.
 #ifndef KB_SOFTMAX_REGS
 #define KB_SOFTMAX_REGS 224
 #endif
